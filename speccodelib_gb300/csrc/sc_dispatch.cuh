@@ -213,6 +213,18 @@ cudaError_t launch_xwarp(const FieldList<T>& fin, const FieldList<T>& fout, cons
   return cudaGetLastError();
 }
 
+template <typename T, int LOGM>
+cudaError_t launch_xumax(const FieldList<T>& fin, const Geom& g, const C2<T>* twM, const C2<T>* twN, const XArgs<T>& xa,
+                         unsigned long long* out, cudaStream_t s) {
+  using Cfg = XuCfg<T, LOGM>;
+  auto k = xpass_umax_kernel<T, LOGM>;
+  static cudaError_t attr = smem_attr(k, Cfg::SMEM);
+  if (attr != cudaSuccess) return attr;
+  const long long nb = (xa.rows + Cfg::WARPS - 1) / Cfg::WARPS;
+  k<<<(unsigned)nb, Cfg::NT, Cfg::SMEM, s>>>(fin, g, twM, twN, xa, out);
+  return cudaGetLastError();
+}
+
 template <typename T, int LOGN>
 cudaError_t launch_zfwd_adj(const FieldList<T>& fin, const AdjArgs<T>& aa, const Geom& g, const C2<T>* tw,
                             cudaStream_t s) {
@@ -282,7 +294,16 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
     return cudaGetLastError();                                                                   \
   }
 
-#define SC_DEFINE_XWARP(T, CASES)                                                                \
+#define SC_DEFINE_XWARP(T, CASES, UCASES)                                                        \
+  template <>                                                                                    \
+  cudaError_t sc::Launch<T>::xpass_umax(int logm, const FieldList<T>& fin, const Geom& g,        \
+                                        const C2<T>* twM, const C2<T>* twN, const XArgs<T>& xa,  \
+                                        unsigned long long* out, cudaStream_t s) {               \
+    switch (logm) {                                                                              \
+      UCASES                                                                                     \
+      default: return cudaErrorNotSupported;                                                     \
+    }                                                                                            \
+  }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::xpass_warp(int logm, int mode, const FieldList<T>& fin,             \
                                         const FieldList<T>& fout, const Geom& g,                 \
@@ -293,6 +314,9 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
       default: return cudaErrorNotSupported;                                                     \
     }                                                                                            \
   }
+
+#define SC_XUMAX_CASE(T, L) \
+  case L: return sc::launch_xumax<T, L>(fin, g, twM, twN, xa, out, s);
 
 #define SC_XWARP_CASE(T, L)                                                                      \
   case L:                                                                                        \
@@ -420,13 +444,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
 #define SC_DEFINE_OPS(T)                                                                         \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::diag(const DiagArgs<T>& da, const Geom& g, cudaStream_t s) {        \
-    size_t sm = sizeof(double) * (size_t)da.nshell;                                              \
-    sc::diag_partial_kernel<T><<<da.nblocks, 256, sm, s>>>(da, g);                               \
-    cudaError_t e = cudaGetLastError();                                                          \
-    if (e != cudaSuccess) return e;                                                              \
-    sc::diag_final_kernel<<<1, 256, 0, s>>>(da.partial, da.nblocks, sc::DQ_N + da.nshell,        \
-                                            da.out);                                             \
-    return cudaGetLastError();                                                                   \
+    return sc::diag_launch<T>(da, g, s);                                                         \
   }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::specop(const SpecOpArgs<T>& oa, const Geom& g, cudaStream_t s) {    \
@@ -466,7 +484,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
     sc::moments_kernel<T><<<nb, 256, 0, s>>>(d, g, rpb, partial);                                \
     cudaError_t e = cudaGetLastError();                                                          \
     if (e != cudaSuccess) return e;                                                              \
-    sc::moments_final_kernel<<<1, 32, 0, s>>>(partial, nb, out);                                 \
+    sc::moments_final_kernel<<<1, 256, 0, s>>>(partial, nb, out);                                \
     return cudaGetLastError();                                                                   \
   }                                                                                              \
   template <>                                                                                    \
@@ -492,7 +510,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
     sc::phys_kernel<T><<<nblocks, 256, 0, s>>>(pa, g);                                           \
     cudaError_t e = cudaGetLastError();                                                          \
     if (e != cudaSuccess || pa.op != sc::PH_DYN2) return e;                                      \
-    sc::dyn_final_kernel<<<1, 32, 0, s>>>(pa.partial, nblocks, c1_out, lm_mm);                   \
+    sc::dyn_final_kernel<<<1, 256, 0, s>>>(pa.partial, nblocks, c1_out, lm_mm);                  \
     return cudaGetLastError();                                                                   \
   }
 

@@ -148,6 +148,11 @@ template <typename T> struct Launch {
   static cudaError_t xpass_warp(int logm, int mode, const FieldList<T>& fin, const FieldList<T>& fout,
                                 const Geom& g, const C2<T>* twM, const C2<T>* twN, const XArgs<T>& xa,
                                 cudaStream_t s);
+  // c2r of three velocity rows at a time, kept in registers: max |u|^2 over the
+  // grid and the count of non-finite points, added to out[0] (the bits of a
+  // non-negative double) and out[1]; lengths as xpass_warp
+  static cudaError_t xpass_umax(int logm, const FieldList<T>& fin, const Geom& g, const C2<T>* twM, const C2<T>* twN,
+                                const XArgs<T>& xa, unsigned long long* out, cudaStream_t s);
 };
 
 }  // namespace sc

@@ -110,10 +110,7 @@ int run(const void* vx, const void* vy, const void* vz, int nx, int ny, int nz, 
   if (rc != SC_OK) return rc;
   da.partial = scratch;
   da.out = out;
-  sc::diag_partial_kernel<T><<<da.nblocks, 256, sizeof(double) * da.nshell, s>>>(da, g);
-  sc::diag_final_kernel<<<1, 256, 0, s>>>(scratch, da.nblocks, sc::DQ_N + da.nshell, out);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return err(SC_ERR_CUDA, "sc_diagnostics_noalloc: launch failed");
+  if (sc::diag_launch<T>(da, g, s) != cudaSuccess) return err(SC_ERR_CUDA, "sc_diagnostics_noalloc: launch failed");
   return SC_OK;
 }
 

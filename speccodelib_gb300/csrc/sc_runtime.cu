@@ -309,13 +309,14 @@ template <typename T> struct Impl {
   static int pencil_tile(int logz) { return (sizeof(T) == 4 && logz < 9) ? 16 : 8; }
 
   // ---- TMA-fed plain strided pass over nf equally spaced fields ----
-  static int plain_tma(sc_handle* h, const char* name, int axis, bool inv, C* base, int nf) {
+  // (src: the fields it reads, when they are not the ones it writes)
+  static int plain_tma(sc_handle* h, const char* name, int axis, bool inv, C* base, int nf, const C* src = nullptr) {
     auto* g = &h->g;
     const int logn = axis == 1 ? h->logy : h->logz;
     const int N = axis == 1 ? g->ny : g->nz;
     const int P = L::tma_tile(logn);
     CUtensorMap map;
-    SC_TRY(encode_fields(h, base, nf, axis, P, N, &map));
+    SC_TRY(encode_fields(h, src ? src : base, nf, axis, P, N, &map));
     sc::TmaPass<T> tp{};
     tp.base = base;
     tp.field = g->field;
@@ -425,6 +426,10 @@ template <typename T> struct Impl {
       SC_TRY(launch(h, "zpass_inv", [&] { return L::plain(h->logz, true, fl, zpass_args(h, nf), *g, g->ny, tw(h, g->nz), h->stream); }));
       SC_TRY(launch(h, "ypass_inv", [&] { return L::plain(h->logy, true, fl, ypass_args(h, nf), *g, g->nz, tw(h, g->ny), h->stream); }));
     }
+    return inverse_x(h, fl, nf);
+  }
+  static int inverse_x(sc_handle* h, const sc::FieldList<T>& fl, int nf) {
+    auto* g = &h->g;
     for (int i = 0; i < nf; i += 3) {
       sc::FieldList<T> sub{};
       for (int c = 0; c < 3; ++c) sub.f[c] = fl.f[i + c];
@@ -1401,7 +1406,8 @@ template <typename T> struct Impl {
   }
 
   // ---- reductions ----
-  static int diag_run(sc_handle* h, const C* const v[3], int physical, double kmax2, int nshell, double* host_out) {
+  static int diag_run(sc_handle* h, const C* const v[3], int physical, double kmax2, int nshell, double* host_out,
+                      double* dev_out = nullptr) {
     auto* g = &h->g;
     sc::DiagArgs<T> da{};
     for (int c = 0; c < 3; ++c) da.v[c] = v[c];
@@ -1414,7 +1420,7 @@ template <typename T> struct Impl {
     if ((size_t)da.nblocks * (sc::DQ_N + nshell) > h->dpart_len)
       return fail(SC_ERR_INVALID, "reduction scratch too small");
     da.partial = h->dpart;
-    da.out = h->dout;
+    da.out = dev_out ? dev_out : h->dout;
     SC_TRY(launch(h, "diag", [&] { return L::diag(da, *g, h->stream); }));
     if (host_out) {
       SC_CUDA(cudaMemcpyAsync(host_out, h->dout, sizeof(double) * (sc::DQ_N + nshell), cudaMemcpyDeviceToHost, h->stream));
@@ -1439,18 +1445,50 @@ template <typename T> struct Impl {
   }
 
   static int diagnostics(sc_handle* h, sc_diag* d, double* eks) {
-    const int ns = h->g.nx / 2;
-    std::vector<double> out(sc::DQ_N + ns), outp(sc::DQ_N);
+    auto* g = &h->g;
+    const int ns = g->nx / 2;
+    // one read-back for everything: [spectral sums and shells | physical sums]
+    std::vector<double> out(2 * sc::DQ_N + ns);
+    double* const outp = out.data() + sc::DQ_N + ns;
+    double* const dphys = h->dout + sc::DQ_N + ns;
     const C* v[3] = {F(h, S_V), F(h, S_V + 1), F(h, S_V + 2)};
-    SC_TRY(diag_run(h, v, 0, -1.0, ns, out.data()));
-    // max |u| from the physical field (copy, inverse transform, reduce)
-    for (int c = 0; c < 3; ++c)
-      SC_CUDA(cudaMemcpyAsync(F(h, S_W + c), F(h, S_V + c), h->csize * h->g.field, cudaMemcpyDeviceToDevice, h->stream));
-    SC_TRY(inverse(h, range(h, S_W, 3), 3));
-    const C* u[3] = {F(h, S_W), F(h, S_W + 1), F(h, S_W + 2)};
-    SC_TRY(diag_run(h, u, 1, -1.0, 0, outp.data()));
+    SC_TRY(diag_run(h, v, 0, -1.0, ns, nullptr));
+    // max |u| from the physical field: z- and y-inverse into the work slots,
+    // then the c2r rows reduced in registers where the warp kernel has the
+    // length, else stored and reduced
+    auto w3 = range(h, S_W, 3);
+    bool reduced = false;
+    if (h->tma && h->xwarp) {
+      SC_TRY(plain_tma(h, "zpass_inv", 2, true, w3.f[0], 3, v[0]));
+      SC_TRY(plain_tma(h, "ypass_inv", 1, true, w3.f[0], 3));
+      SC_CUDA(cudaMemsetAsync(dphys, 0, 2 * sizeof(double), h->stream));
+      SC_TRY(launch(h, "xpass_umax", [&] {
+        cudaError_t e = L::xpass_umax(h->logx - 1, w3, *g, tw(h, g->nx / 2), tw(h, g->nx), xargs(h),
+                                      reinterpret_cast<unsigned long long*>(dphys), h->stream);
+        reduced = e != cudaErrorNotSupported;
+        return reduced ? e : cudaSuccess;
+      }));
+      if (!reduced) SC_TRY(inverse_x(h, w3, 3));
+    } else {
+      for (int c = 0; c < 3; ++c)
+        SC_CUDA(cudaMemcpyAsync(w3.f[c], v[c], h->csize * g->field, cudaMemcpyDeviceToDevice, h->stream));
+      SC_TRY(inverse(h, w3, 3));
+    }
+    if (!reduced) {
+      const C* u[3] = {w3.f[0], w3.f[1], w3.f[2]};
+      SC_TRY(diag_run(h, u, 1, -1.0, 0, nullptr, dphys));
+    }
     double sc3[3];
-    SC_CUDA(cudaMemcpy(sc3, h->dscal, sizeof sc3, cudaMemcpyDeviceToHost));
+    SC_CUDA(cudaMemcpyAsync(out.data(), h->dout, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, h->stream));
+    SC_CUDA(cudaMemcpyAsync(sc3, h->dscal, sizeof sc3, cudaMemcpyDeviceToHost, h->stream));
+    SC_TRY(check_derr(h));
+    if (reduced) {
+      unsigned long long n;
+      std::memcpy(&n, &outp[1], sizeof n);
+      const double mu2 = outp[0];
+      outp[sc::DQ_MAXU2] = mu2;
+      outp[sc::DQ_NONFINITE] = (double)n;
+    }
     if (d) {
       d->energy = out[sc::DQ_ENERGY];
       d->enstrophy = out[sc::DQ_K2Q];
@@ -1772,7 +1810,7 @@ int sc_create(const sc_params* pin, sc_handle** out) {
   SC_CUDA(cudaMemset(h->derr, 0, sizeof(int)));
   h->dpart_len = (size_t)1024 * (sc::DQ_N + g.nx / 2) + 2 * 4096;
   SC_CUDA(cudaMalloc(&h->dpart, sizeof(double) * h->dpart_len));
-  SC_CUDA(cudaMalloc(&h->dout, sizeof(double) * (sc::DQ_N + g.nx / 2)));
+  SC_CUDA(cudaMalloc(&h->dout, sizeof(double) * (2 * sc::DQ_N + g.nx / 2)));
   double c0[8] = {p.c1, 0, 0, 0, 0, 0, 0, 0};
   SC_CUDA(cudaMemcpy(h->dscal, c0, sizeof c0, cudaMemcpyHostToDevice));
   if (p.precision == SC_FP32) SC_TRY(Impl<float>::setup_tables(h.get()));

@@ -749,4 +749,88 @@ xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __re
   }
 }
 
+// Maximum of |u|^2 over the physical grid and the non-finite count, from the
+// three velocity fields after the z- and y-inverse: a warp per row transforms
+// the three rows and combines them in registers, so physical space is never
+// written (the c2r pass with stores and the reduction re-reading them took 102
+// + 70 us at 256^3 FP32, this 73).  Bound by the shared-memory pipe as the
+// x-pass is.
+template <typename T, int LOGM> struct XuCfg {
+  static constexpr int STG = XwCfg<T, LOGM>::STG;
+  static constexpr int PER_WARP = WarpFFT<T, LOGM>::SMEM + 2 * STG;
+  static_assert((PER_WARP * sizeof(C2<T>)) % 16 == 0 && (WarpFFT<T, LOGM>::SMEM * sizeof(C2<T>)) % 16 == 0,
+                "staging buffers must start on 16-byte boundaries");
+  static constexpr int WARPS = 8, NT = 32 * WARPS;
+  static constexpr size_t SMEM = sizeof(C2<T>) * PER_WARP * WARPS;
+};
+
+template <typename T, int LOGM>
+__global__ void __launch_bounds__(XuCfg<T, LOGM>::NT, 2)
+xpass_umax_kernel(FieldList<T> fin, Geom g, const C2<T>* __restrict__ twM, const C2<T>* __restrict__ twN, XArgs<T> xa,
+                  unsigned long long* out) {
+  using C = C2<T>;
+  using Cfg = XuCfg<T, LOGM>;
+  using Row = XwRow<T, LOGM>;
+  constexpr int E = Row::E;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ __align__(8) uint64_t sbar[2 * Cfg::WARPS];
+  __shared__ double wmax[Cfg::WARPS];
+  __shared__ int wnf[Cfg::WARPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * Cfg::WARPS + warp;
+  T m = T(0);
+  int nf = 0;
+  if (row < xa.rows) {
+    Row R;
+    R.sm = reinterpret_cast<C*>(smraw) + warp * Cfg::PER_WARP;
+    R.twM = twM;
+    R.twN = twN;
+    if constexpr (Row::TX) R.tx = xa.twx + WarpTw::offset(LOGM);
+    R.off = row * g.nxp;
+    R.lane = lane;
+    const C* seq[3] = {fin.f[0], fin.f[1], fin.f[2]};
+    R.stg = R.sm + WarpFFT<T, LOGM>::SMEM;
+    R.stg_elems = Cfg::STG;
+    R.seq = seq;
+    R.nseq = 3;
+    R.sbar = sbar + 2 * warp;
+    R.err = xa.err;
+    R.stage_start();
+    C u2[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) u2[i] = czero<C>();
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      C x[E];
+      R.load_z(seq[c], x);
+      Row::WF::template nat_to_scr<true, Row::TX>(x, R.sm, twM, lane, R.tx);
+#pragma unroll
+      for (int i = 0; i < E; ++i) u2[i] = mk<C>(x[i].x * x[i].x + u2[i].x, x[i].y * x[i].y + u2[i].y);
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      m = fmax(m, fmax(u2[i].x, u2[i].y));
+      nf += (!isfinite(u2[i].x) || !isfinite(u2[i].y)) ? 1 : 0;
+    }
+  }
+  const double wm = warp_max((double)m);
+  nf = __reduce_add_sync(0xffffffffu, nf);
+  if (lane == 0) {
+    wmax[warp] = wm;
+    wnf[warp] = nf;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double b = 0.0;
+    int n = 0;
+    for (int w = 0; w < Cfg::WARPS; ++w) {
+      b = fmax(b, wmax[w]);
+      n += wnf[w];
+    }
+    // non-negative doubles order as their bit patterns do
+    atomicMax(&out[0], (unsigned long long)__double_as_longlong(b));
+    if (n) atomicAdd(&out[1], (unsigned long long)n);
+  }
+}
+
 }  // namespace sc
