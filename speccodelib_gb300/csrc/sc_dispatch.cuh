@@ -4,6 +4,7 @@
 #include "sc_launch.h"
 #include "sc_ops.cuh"
 #include "sc_tma_passes.cuh"
+#include "sc_xgroup.cuh"
 #include "sc_xwarp.cuh"
 #include "sc_adjoint.cuh"
 #include "sc_fused.cuh"
@@ -213,6 +214,30 @@ cudaError_t launch_xwarp(const FieldList<T>& fin, const FieldList<T>& fout, cons
   return cudaGetLastError();
 }
 
+template <typename T, int LOGM, int MODE>
+cudaError_t launch_xgroup(const FieldList<T>& fin, const FieldList<T>& fout, const Geom& g, const C2<T>* twM,
+                          const C2<T>* twN, const XArgs<T>& xa, cudaStream_t s) {
+  using Cfg = XgCfg<T, LOGM, MODE>;
+  auto k = xpass_group_kernel<T, LOGM, MODE>;
+  static cudaError_t attr = smem_attr(k, Cfg::SMEM);
+  if (attr != cudaSuccess) return attr;
+  const int per = Cfg::WARPS * GroupFFT<T, LOGM>::RW;
+  k<<<(unsigned)((xa.rows + per - 1) / per), Cfg::NT, Cfg::SMEM, s>>>(fin, fout, g, twM, twN, xa);
+  return cudaGetLastError();
+}
+
+template <typename T, int LOGM>
+cudaError_t launch_xgumax(const FieldList<T>& fin, const Geom& g, const C2<T>* twM, const C2<T>* twN,
+                          const XArgs<T>& xa, unsigned long long* out, cudaStream_t s) {
+  using Cfg = XgUmaxCfg<T, LOGM>;
+  auto k = xgroup_umax_kernel<T, LOGM>;
+  static cudaError_t attr = smem_attr(k, Cfg::SMEM);
+  if (attr != cudaSuccess) return attr;
+  const int per = Cfg::WARPS * GroupFFT<T, LOGM>::RW;
+  k<<<(unsigned)((xa.rows + per - 1) / per), Cfg::NT, Cfg::SMEM, s>>>(fin, g, twM, twN, xa, out);
+  return cudaGetLastError();
+}
+
 template <typename T, int LOGM>
 cudaError_t launch_xumax(const FieldList<T>& fin, const Geom& g, const C2<T>* twM, const C2<T>* twN, const XArgs<T>& xa,
                          unsigned long long* out, cudaStream_t s) {
@@ -314,6 +339,15 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
       default: return cudaErrorNotSupported;                                                     \
     }                                                                                            \
   }
+
+#define SC_XGUMAX_CASE(T, L) \
+  case L: return sc::launch_xgumax<T, L>(fin, g, twM, twN, xa, out, s);
+
+#define SC_XGROUP_CASE(T, L)                                                                     \
+  case L:                                                                                        \
+    return mode == sc::XW_ADJ    ? sc::launch_xgroup<T, L, sc::XW_ADJ>(fin, fout, g, twM, twN, xa, s)  \
+           : mode == sc::XW_SMAG ? sc::launch_xgroup<T, L, sc::XW_SMAG>(fin, fout, g, twM, twN, xa, s) \
+                                 : sc::launch_xgroup<T, L, sc::XW_DNS>(fin, fout, g, twM, twN, xa, s);
 
 #define SC_XUMAX_CASE(T, L) \
   case L: return sc::launch_xumax<T, L>(fin, g, twM, twN, xa, out, s);

@@ -114,12 +114,15 @@ template <bool INV, typename C> __device__ __forceinline__ void dft16(C* v) {
 #pragma unroll
     for (int k2 = 1; k2 < 4; ++k2) {
       const int e = n1 * k2;
+      if (e == 4) {   // -+ i: no arithmetic
+        v[n1 + 4 * k2] = INV ? cmuli(v[n1 + 4 * k2]) : cmulmi(v[n1 + 4 * k2]);
+        continue;
+      }
       R c, sn;   // W16^e = cos(2 pi e/16) - i sin(2 pi e/16) (forward)
       switch (e) {
         case 1: c = W16<R>::c1; sn = W16<R>::s1; break;
         case 2: c = W16<R>::h; sn = W16<R>::h; break;
         case 3: c = W16<R>::s1; sn = W16<R>::c1; break;
-        case 4: c = 0; sn = 1; break;
         case 6: c = -W16<R>::h; sn = W16<R>::h; break;
         default: c = -W16<R>::c1; sn = -W16<R>::s1; break;   // e = 9
       }

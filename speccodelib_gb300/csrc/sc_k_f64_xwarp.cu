@@ -1,4 +1,7 @@
-// Compiled instances: warp-per-row x-pass, double arithmetic (M = 64, 128).
+// Compiled instances: lane-group x-pass, double arithmetic (M = 16 .. 256).
 #include "sc_dispatch.cuh"
-SC_DEFINE_XWARP(double, SC_XWARP_CASE(double, 6) SC_XWARP_CASE(double, 7),
-                SC_XUMAX_CASE(double, 6) SC_XUMAX_CASE(double, 7))
+SC_DEFINE_XWARP(double,
+                SC_XGROUP_CASE(double, 4) SC_XGROUP_CASE(double, 5) SC_XGROUP_CASE(double, 6)
+                SC_XGROUP_CASE(double, 7) SC_XGROUP_CASE(double, 8),
+                SC_XGUMAX_CASE(double, 4) SC_XGUMAX_CASE(double, 5) SC_XGUMAX_CASE(double, 6)
+                SC_XGUMAX_CASE(double, 7) SC_XGUMAX_CASE(double, 8))

@@ -749,6 +749,31 @@ xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __re
   }
 }
 
+// A block's maximum m (non-negative) and count nf into out[0] and out[1];
+// every thread of the block's WARPS warps calls it.
+template <int WARPS> __device__ __forceinline__ void umax_block_out(double m, int nf, unsigned long long* out) {
+  __shared__ double wmax[WARPS];
+  __shared__ int wnf[WARPS];
+  const int warp = threadIdx.x >> 5;
+  m = warp_max(m);
+  nf = __reduce_add_sync(0xffffffffu, nf);
+  if ((threadIdx.x & 31) == 0) {
+    wmax[warp] = m;
+    wnf[warp] = nf;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double b = 0.0;
+  int n = 0;
+  for (int w = 0; w < WARPS; ++w) {
+    b = fmax(b, wmax[w]);
+    n += wnf[w];
+  }
+  // non-negative doubles order as their bit patterns do
+  atomicMax(&out[0], (unsigned long long)__double_as_longlong(b));
+  if (n) atomicAdd(&out[1], (unsigned long long)n);
+}
+
 // Maximum of |u|^2 over the physical grid and the non-finite count, from the
 // three velocity fields after the z- and y-inverse: a warp per row transforms
 // the three rows and combines them in registers, so physical space is never
@@ -774,8 +799,6 @@ xpass_umax_kernel(FieldList<T> fin, Geom g, const C2<T>* __restrict__ twM, const
   constexpr int E = Row::E;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(8) uint64_t sbar[2 * Cfg::WARPS];
-  __shared__ double wmax[Cfg::WARPS];
-  __shared__ int wnf[Cfg::WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * Cfg::WARPS + warp;
   T m = T(0);
@@ -813,24 +836,7 @@ xpass_umax_kernel(FieldList<T> fin, Geom g, const C2<T>* __restrict__ twM, const
       nf += (!isfinite(u2[i].x) || !isfinite(u2[i].y)) ? 1 : 0;
     }
   }
-  const double wm = warp_max((double)m);
-  nf = __reduce_add_sync(0xffffffffu, nf);
-  if (lane == 0) {
-    wmax[warp] = wm;
-    wnf[warp] = nf;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = 0.0;
-    int n = 0;
-    for (int w = 0; w < Cfg::WARPS; ++w) {
-      b = fmax(b, wmax[w]);
-      n += wnf[w];
-    }
-    // non-negative doubles order as their bit patterns do
-    atomicMax(&out[0], (unsigned long long)__double_as_longlong(b));
-    if (n) atomicAdd(&out[1], (unsigned long long)n);
-  }
+  umax_block_out<Cfg::WARPS>((double)m, nf, out);
 }
 
 }  // namespace sc

@@ -47,3 +47,39 @@ def test_diagnostics_nonfinite(specns_lib, shape):
         with pytest.raises(S.SpecNSError) as e:
             h.diagnostics()
     assert e.value.code == 3
+
+
+TOL = {S.SC_FP64: 1e-12, S.SC_FP32: 1e-5}   # the library's bounds against the oracle
+X_SHAPES = [(16, 8, 8), (32, 8, 16), (64, 16, 8), (128, 8, 8), (256, 8, 16), (512, 8, 8), (1024, 8, 8)]
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", X_SHAPES)
+@pytest.mark.parametrize("sgs", ["none", "smag"])
+def test_rhs_x_lengths(specns_lib, shape, prec, sgs):
+    """The x-pass of the right-hand side (Lamb product; Lamb product and
+    Smagorinsky stress) at every row length, on grids of few rows."""
+    nx, ny, nz = shape
+    kw = dict(forced=0) if sgs == "none" else dict(forced=0, sgs=S.SC_SGS_SMAG, c1=0.03)
+    v = [fresh(a, DT[prec]) for a in hermitian_fields(shape, 41, kcut=0.4 * max(shape))]
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, forced=False, sgs=sgs, c1=0.03))
+    ref = R.ratesdudt([a.astype(np.complex128) for a in v], g)
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, **kw)) as h:
+        h.set_state(*v)
+        w = h.rhs()
+    assert rel_l2(w, ref) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", X_SHAPES[1:6])
+def test_vjp_x_lengths(specns_lib, shape, prec):
+    """The adjoint's x-pass at the same lengths, over one RK4 step."""
+    nx, ny, nz = shape
+    v = [fresh(a, DT[prec]) for a in hermitian_fields(shape, 43, kcut=6.0)]
+    lam = [fresh(a, DT[prec]) for a in hermitian_fields(shape, 44)]
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, nu=0.02, dt=1e-3))
+    ref = R.rk4_step_adj([a.astype(np.complex128) for a in v], [a.astype(np.complex128) for a in lam], g)
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, nu=0.02, dt=1e-3)) as h:
+        h.set_state(*v)
+        out = h.adjoint_vjp(1, lam, 1)
+    assert rel_l2(out, ref) < (1e-11 if prec == S.SC_FP64 else 1e-4)   # the bounds of the adjoint's other tests
