@@ -546,14 +546,23 @@ __device__ __forceinline__ void finish_point(const StageArgs<T>& st, const Geom&
 
 // K_f of force.f90:16-22 from the zinv partial sums, fixed order.
 // Visits exactly the (tile, ky) blocks that zinv wrote: (t*P)^2 + ky^2 < fkmax2.
+// One thread walks the band's few rows, in index order; testing every row of
+// the axis instead put ny double-precision compares (5 us at ny = 64) in front
+// of the band's tiles.
 __device__ __forceinline__ double forcing_energy(const double* partial, int tiles, int P, int ny,
                                                  double fkmax2) {
   double s = 0.0;
-  for (int t = 0; t < tiles; ++t)
-    for (int iy = 0; iy < ny; ++iy) {
-      const double ky = wavenum(iy, ny), kx0 = (double)t * P;
-      if (kx0 * kx0 + ky * ky < fkmax2) s += partial[(long long)t * ny + iy];
+  const int fk_b = k2_lt(fkmax2);
+  for (int t = 0; t < tiles; ++t) {
+    const double* row = partial + (long long)t * ny;
+    const int kx2 = t * P * t * P;
+    int k = 0;   // |ky| < k lies in the band
+    while (k <= ny / 2 && kx2 + k * k < fk_b) {
+      if (k < ny / 2) s += row[k];
+      ++k;
     }
+    for (int iy = max(ny / 2, ny - k + 1); iy < ny; ++iy) s += row[iy];
+  }
   return s;
 }
 
