@@ -144,14 +144,13 @@ class Clocks:
 # accumulator, which stage 3 left holding E^2 v + its partial sum, and
 # writes the state).  With stages 1-3 fused into zfwd_zinv (15, 18, 18 F:
 # the RHS, v, acc read; acc and the next u, w written) zfwd runs stage 4
-# only (9 F); zinv runs once per step and zinv_kx0 covers one kx tile (not
-# counted).
-KERNELS = ["zinv", "ypass_inv", "xpass", "ypass_fwd", "zfwd", "zfwd_zinv", "zinv_kx0", "fixup"]
+# only (9 F); zinv runs once per step.
+KERNELS = ["zinv", "ypass_inv", "xpass", "ypass_fwd", "zfwd", "zfwd_zinv"]
 
 
 def kernel_fields(fused):
     return {"zinv": 9.0, "ypass_inv": 12.0, "xpass": 9.0, "ypass_fwd": 6.0,
-            "zfwd": 9.0 if fused else 12.75, "zfwd_zinv": 17.0, "zinv_kx0": 0.0, "fixup": 0.0}
+            "zfwd": 9.0 if fused else 12.75, "zfwd_zinv": 17.0}
 
 
 def traffic_from_profiles(kernel):

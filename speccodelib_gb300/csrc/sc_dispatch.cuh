@@ -40,7 +40,6 @@ cudaError_t launch_zinv(const ZvArgs<T>& za, const FieldList<T>& out, const Geom
   static cudaError_t attr = smem_attr(k, Cfg::SMEM);
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Cfg::P - 1) / Cfg::P, g.ny);
-  if (za.tiles_x > 0 && (unsigned)za.tiles_x < grid.x) grid.x = za.tiles_x;
   k<<<grid, Cfg::NT, Cfg::SMEM, s>>>(za, out, g, tw);
   return cudaGetLastError();
 }
@@ -196,8 +195,7 @@ cudaError_t launch_zinv5(const CUtensorMap& vmap, const CUtensorMap& umap, const
     static cudaError_t attr = smem_attr(k, Z::SMEM);
     if (attr != cudaSuccess) return attr;
     dim3 grid((g.nxh + Z::P - 1) / Z::P, g.ny);
-    if (za.tiles_x > 0 && (unsigned)za.tiles_x < grid.x) grid.x = za.tiles_x;
-    k<<<grid, Z::NT, Z::SMEM, s>>>(vmap, umap, za, out, g, tw, err);
+      k<<<grid, Z::NT, Z::SMEM, s>>>(vmap, umap, za, out, g, tw, err);
     return cudaGetLastError();
   }
 }
@@ -459,8 +457,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
     long long n = (long long)g.ny * g.nz;                                                        \
     int nb = (int)((n + 255) / 256);                                                             \
     if (nb > 4096) nb = 4096;                                                                    \
-    if (st.mode == sc::SM_AB2V) sc::fixup_kx0_kernel<T, sc::SM_AB2V><<<nb, 256, 0, s>>>(st, g);   \
-    else sc::fixup_kx0_kernel<T><<<nb, 256, 0, s>>>(st, g);                                      \
+    sc::fixup_kx0_kernel<T><<<nb, 256, 0, s>>>(st, g);                                           \
     return cudaGetLastError();                                                                   \
   }
 

@@ -8,12 +8,10 @@
 // and s never goes through HBM: 6 field passes fewer per right-hand side
 // (write s, read s) and one launch fewer.
 //
-// The exception is the kx = 0 column: symmetrize copies conj(s(-ky, -kz))
-// into its targets, values that belong to another tile.  Tiles with kx0 = 0
-// therefore store s as the unfused kernel does; after the kx = 0 fix-up a
-// one-tile zinv (grid.x = 1) produces their outputs.  Tiles inside the
-// forcing band (kx0^2 + ky^2 < fkmax^2) also store s, which the next stage's
-// forcing reads.
+// The kx = 0 column, whose symmetrize copy needs another pencil's values, is
+// exchanged between the two CTAs of a cluster (hermitian_column).  Tiles inside
+// the forcing band (kx0^2 + ky^2 < fkmax^2) also store s, which the next
+// stage's forcing reads.
 //
 // Five transforms instead of six: kx and ky are constant along a z pencil, so
 // w_z = i kx u_y - i ky u_x is formed pointwise from the transformed u; only
@@ -317,7 +315,7 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
 
 // Standalone z-inverse (MODE ZV_DNS, or ZV_SMAG for the LES operands): the
 // stage input tile by TMA, K_f partial sums, then zinv_from_tiles.
-// grid = (kx tiles or za.tiles_x, ny).
+// grid = (kx tiles, ny).
 template <typename T, int LOGN, int MODE>
 __global__ void __launch_bounds__(ZiCfg<T, LOGN>::NT, ZiCfg<T, LOGN>::MINB)
 zinv5_tma_kernel(const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap umap, ZvArgs<T> za,
@@ -478,7 +476,7 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
 // MODE the stage's update mode (SM_RK1..3; -1: st.mode at run time).
 // grid = (kx tiles, ny).
 template <typename T, int LOGN, int MODE>
-__global__ void __launch_bounds__(ZiCfg<T, LOGN>::NT, ZiCfg<T, LOGN>::MINB)
+__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(ZiCfg<T, LOGN>::NT, ZiCfg<T, LOGN>::MINB)
 zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap fmap,
                      StageArgs<T> st, FusedArgs<T> fa, Geom g, const C2<T>* __restrict__ tw, int* err) {
   using Z = ZiCfg<T, LOGN>;
@@ -497,15 +495,15 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
   __shared__ double s_coef;
   __shared__ double red[NT / 32 + 1];
   const int kx0 = blockIdx.x * P;
-  const int iy = blockIdx.y;
+  const int iy = paired_row(blockIdx.y, g.ny);
   const int nvalid = min(P, g.nxh - kx0);
   const long long zstride = (long long)g.ny * g.nxp;
   const long long base = (long long)iy * g.nxp + kx0;
   const T ky = (T)wavenum(iy, g.ny);
-  const bool tile0 = kx0 == 0;
+  const bool paired = kx0 == 0;   // meets its partner: both CTAs stay until then
   const bool band = st.forced && ((double)kx0 * kx0 + (double)ky * ky < st.fkmax2);
   const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(st.fkmax2), kc_b = k2_lt(st.kcut2);
-  if (launch_failed(err)) return;
+  if (!paired && launch_failed(err)) return;
   if (threadIdx.x == 0) {
     for (int c = 0; c < 3; ++c) mbar_init(&bars[c], 1);
     fence_mbar_init();
@@ -522,12 +520,18 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
     }
   }
   __syncthreads();
+  bool ok = true;
   for (int c = 0; c < 3; ++c) {
-    if (!mbar_wait_bounded(&bars[c], 0, err)) return;
+    ok = mbar_wait_bounded(&bars[c], 0, err) && ok;
+    if (!ok && !paired) return;
     // the update's operands into L2 once the Lamb tiles are in (issued with
     // them, the prefetch delays them)
     if (c == 2 && threadIdx.x == 0) prefetch_update_tile<Cfg>(&fmap, st, kx0, iy);
     EF::template run_inplace<false>(rt[c], tw);
+  }
+  if (paired) {
+    hermitian_column<T, P, N, NT>(rt, st, g, iy, base, zstride, band, band ? s_coef : 0.0, 0, fk_b);
+    if (!ok) return;
   }
   // spectral update; the next stage input goes back into the tiles
   double q = 0.0;
@@ -556,36 +560,29 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
       C* wp = wv[i];
       const int kz = wavenum(iz, g.nz);
       const int k2 = ix * ix + kyi * kyi + kz * kz;
-      if (band && k2 < fk_b) {
+      if (band && k2 < fk_b && ix > 0) {
         const T ac = (T)s_coef;
 #pragma unroll
         for (int c = 0; c < 3; ++c) wp[c] = cadd(wp[c], cscale(st.sin[c][idx], ac));
-      }
-      if (ix == 0) {
-        const long long sd = ((long long)iz * g.ny + iy) * 3;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) st.side[sd + c] = wp[c];
-        if (iz > g.nz / 2 || (iz == 0 && iy > g.ny / 2)) continue;
       }
       if (iy == g.ny / 2 || iz == g.nz / 2 || ix == g.nxh - 1 || (ix == 0 && iy == 0 && iz == 0))
         wp[0] = wp[1] = wp[2] = czero<C>();
       C sn[3];
       finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, vv[i], av[i], sn);
-      if (tile0 || band || fa.store_all) {
+      if (band || fa.store_all) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) st.sout[c][idx] = sn[c];
       }
-      if (!tile0) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) rt[c][e] = sn[c];
-        if (band && k2 < fk_b) {
+      for (int c = 0; c < 3; ++c) rt[c][e] = sn[c];
+      if (band && k2 < fk_b) {
+        double es = 0.0;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) q += (double)sn[c].x * sn[c].x + (double)sn[c].y * sn[c].y;
-        }
+        for (int c = 0; c < 3; ++c) es += (double)sn[c].x * sn[c].x + (double)sn[c].y * sn[c].y;
+        q += ix == 0 ? 0.5 * es : es;
       }
     }
   }
-  if (tile0) return;
   __syncthreads();
   // forcing band energy of the next stage input (force.f90:16-22), FP64
   if (band && fa.kf_next) {

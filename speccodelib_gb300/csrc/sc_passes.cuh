@@ -148,7 +148,6 @@ template <typename T> struct ZvArgs {
   int mask_rhs;
   double kcut2;
   double inv_n3;
-  int tiles_x;       // > 0: only the first tiles_x kx tiles (grid.x)
   int ustore;        // TMA z-inverse: u stored from its tiles by bulk tensor stores
 };
 

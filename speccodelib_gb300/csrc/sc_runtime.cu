@@ -581,23 +581,14 @@ template <typename T> struct Impl {
         fa.store_all = store_all;
         CUtensorMap fmap5;
         SC_TRY(prefetch_slots(h, st, P5, &fmap5));
-        SC_TRY(launch(h, "zfwd_zinv", [&] { return L::zfwd_zinv_tma(h->logz, lmap5, fmap5, st, fa, *g, tw(h, g->nz), h->derr, h->stream); }));
-        SC_TRY(launch(h, "fixup", [&] { return L::fixup(st, *g, h->stream); }));
-        // the kx = 0 tile of the next stage's zinv, after the fix-up
-        CUtensorMap smap;
-        SC_TRY(encode_fields(h, st.sout[0], 3, 2, P5, g->nz, &smap));
-        sc::ZvArgs<T> z0 = za;
-        for (int c = 0; c < 3; ++c) z0.v[c] = st.sout[c];
-        z0.fs.partial = kf_next;
-        z0.tiles_x = 1;
-        z0.ustore = 1;
-        return launch(h, "zinv_kx0", [&] { return L::zinv5_tma(h->logz, smap, lmap5, z0, wl, *g, tw(h, g->nz), h->derr, h->stream); });
+        return launch(h, "zfwd_zinv", [&] { return L::zfwd_zinv_tma(h->logz, lmap5, fmap5, st, fa, *g, tw(h, g->nz), h->derr, h->stream); });
       }
       CUtensorMap vmap_out = lmap;
       const bool vstore = st.mode == sc::SM_RK4 && st.vout[1] == st.vout[0] + g->field &&
                           st.vout[2] == st.vout[0] + 2 * g->field;
       if (vstore) SC_TRY(encode_fields(h, st.vout[0], 3, 2, P, g->nz, &vmap_out));
-      SC_TRY(launch(h, "zfwd", [&] { return L::zfwd_tma(h->logz, lmap, vmap_out, vstore ? 1 : 0, st, *g, tw(h, g->nz), h->derr, h->stream); }));
+      // symmetrize included, its kx = 0 copy exchanged inside the kernel
+      return launch(h, "zfwd", [&] { return L::zfwd_tma(h->logz, lmap, vmap_out, vstore ? 1 : 0, st, *g, tw(h, g->nz), h->derr, h->stream); });
     } else {
       if (les && h->tma && h->zinv5 && sin_spaced && L::zinv5_supported(h->logz)) {
         // LES operands u, w, S_ij: TMA-fed, eight transforms (not 12), u by bulk stores

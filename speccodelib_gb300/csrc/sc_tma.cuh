@@ -123,6 +123,31 @@ __device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int c0, 
                : "memory");
 }
 
+// Barrier over the CTAs of a cluster (release / acquire, every thread).
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// The value at the address of `p` (own shared memory) in cluster CTA `rank`.
+__device__ __forceinline__ float2 cluster_load(const float2* p, uint32_t rank) {
+  uint32_t a;
+  float2 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ double2 cluster_load(const double2* p, uint32_t rank) {
+  uint32_t a;
+  double2 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+  return v;
+}
+
 // Tensor view of `nf` equally spaced fields for the strided-axis passes:
 // dims (x: nxh complex in 8-byte units, y: ny, z: nz, field), rows of pitch
 // nxp.  Columns beyond nxh are outside the tensor and load as zero.

@@ -83,3 +83,30 @@ def test_vjp_x_lengths(specns_lib, shape, prec):
         h.set_state(*v)
         out = h.adjoint_vjp(1, lam, 1)
     assert rel_l2(out, ref) < (1e-11 if prec == S.SC_FP64 else 1e-4)   # the bounds of the adjoint's other tests
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", [(16, 8, 8), (32, 64, 16), (64, 16, 256), (128, 8, 512), (32, 32, 1024)])
+def test_kx0_copy(specns_lib, shape, prec):
+    """symmetrize's kx = 0 copies between the pencils ky and -ky, with the
+    forcing band on them, from a field without that symmetry: the right-hand
+    side and two RK4 steps (fused stages and the last one)."""
+    nx, ny, nz = shape
+    v = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 51, kcut=5.0)]
+    skew = [0.3 * a[:, :, 0] for a in hermitian_fields(shape, 52, kcut=4.0)]
+    for a, s in zip(v, skew):
+        a[:, :, 0] += (1j * s).astype(a.dtype)
+    kw = dict(nu=0.02, dt=1e-3, fkmax=3.1, eps=0.2)
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, **kw))
+    vd = [a.astype(np.complex128) for a in v]
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, **kw)) as h:
+        h.set_state(*v)
+        w = h.rhs()
+        h.rk4_steps(2)
+        out = h.get_state()
+    ref = R.ratesdudt(vd, g)
+    assert rel_l2(w, ref) < TOL[prec]
+    assert rel_l2([a[:, :, 0] for a in w], [a[:, :, 0] for a in ref]) < TOL[prec]
+    ref = R.rk4_run(vd, g, 2)
+    assert rel_l2(out, ref) < TOL[prec]
+    assert rel_l2([a[:, :, 0] for a in out], [a[:, :, 0] for a in ref]) < TOL[prec]
