@@ -89,6 +89,7 @@ struct sc_handle {
   double* kf_partial = nullptr;
   int kf_ntiles_max = 0;          // capacity of kf_partial in tiles
   int* derr = nullptr;            // device error word (bounded waits)
+  int device = 0;                 // the device it was created on
   int nsm = 152;                  // SM count of the device
   bool tma = true;                // TMA-fed strided passes
   bool tma_zinv = false;          // TMA-fed zinv (the register-fed one is faster at 512^3)
@@ -1506,35 +1507,88 @@ template <typename T> struct Impl {
 // A strided copy of 2 KB rows from host memory runs far below the host
 // link's bandwidth (12.1 end-to-end steps/s at 512^3 against 23.4).  Pinned
 // host memory is read or written by the repack kernel itself, through its
-// mapped address; other host memory (or SPECNS_COPY=staged) moves as one
-// contiguous copy to or from a device field in the reference layout,
-// repacked on the device.  Device pointers, copies inside a graph capture
-// and SPECNS_COPY=strided keep the strided copy.
+// mapped address, and so is memory of the handle's device (a strided
+// device-to-device copy ran at 3.3 TB/s); other host memory (or
+// SPECNS_COPY=staged) moves as one contiguous copy to or from a device field
+// in the reference layout, repacked on the device.  Other pointers, copies
+// inside a graph capture and SPECNS_COPY=strided keep the strided copy.
+constexpr int kRepackMax = 3;
+template <typename E> struct RepackArgs {
+  E* dst[kRepackMax];
+  const E* src[kRepackMax];
+};
+// blockIdx.y = field.  Four elements per thread and turn, loads before stores:
+// rows of nx/2+1 elements start on no common alignment, so an access moves one
+// element, and the bytes in flight come from the unrolling.  512^3 FP32, three
+// fields: 0.99 ms as strided copies, 0.78 here.
 template <typename E>
-__global__ void __launch_bounds__(256) repack_rows_kernel(E* __restrict__ dst, long long dpitch,
-                                                          const E* __restrict__ src, long long spitch, int w,
+__global__ void __launch_bounds__(256) repack_rows_kernel(RepackArgs<E> ra, long long dpitch, long long spitch, int w,
                                                           long long rows) {
+  E* __restrict__ dst = ra.dst[blockIdx.y];
+  const E* __restrict__ src = ra.src[blockIdx.y];
+  constexpr int U = 4;
   for (sc::Walk3 it(blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x, rows * w, w,
                     1 << 30);
-       it.ok(); it.next())
-    dst[it.row() * dpitch + it.ix] = src[it.row() * spitch + it.ix];
+       it.ok();) {
+    E v[U];
+    long long d[U];
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (it.ok()) {
+        v[j] = src[it.row() * spitch + it.ix];
+        d[j] = it.row() * dpitch + it.ix;
+        n = j + 1;
+        it.next();
+      }
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (j < n) dst[d[j]] = v[j];
+  }
 }
 
-static int repack(sc_handle* h, void* dst, long long dpitch, const void* src, long long spitch) {
-  const long long rows = (long long)h->g.ny * h->g.nz;
-  const int grid = h->nsm * 8;
-  if (h->csize == 8)
-    repack_rows_kernel<uint2><<<grid, 256, 0, h->stream>>>(static_cast<uint2*>(dst), dpitch,
-                                                         static_cast<const uint2*>(src), spitch, h->g.nxh, rows);
-  else
-    repack_rows_kernel<uint4><<<grid, 256, 0, h->stream>>>(static_cast<uint4*>(dst), dpitch,
-                                                         static_cast<const uint4*>(src), spitch, h->g.nxh, rows);
+template <typename E>
+static void repack_launch(sc_handle* h, void* const* dst, long long dpitch, const void* const* src, long long spitch,
+                          int n) {
+  RepackArgs<E> ra{};
+  for (int i = 0; i < n; ++i) {
+    ra.dst[i] = static_cast<E*>(dst[i]);
+    ra.src[i] = static_cast<const E*>(src[i]);
+  }
+  const long long rows = (long long)h->g.ny * h->g.nz, need = (rows * h->g.nxh + 255) / 256;
+  const long long most = (long long)h->nsm * 8;
+  repack_rows_kernel<E><<<dim3((unsigned)(need < most ? need : most), n), 256, 0, h->stream>>>(ra, dpitch, spitch,
+                                                                                                h->g.nxh, rows);
+}
+// n <= kRepackMax fields
+static int repack(sc_handle* h, void* const* dst, long long dpitch, const void* const* src, long long spitch, int n) {
+  if (h->csize == 8) repack_launch<uint2>(h, dst, dpitch, src, spitch, n);
+  else repack_launch<uint4>(h, dst, dpitch, src, spitch, n);
   SC_CUDA(cudaGetLastError());
   return SC_OK;
 }
 
-// How host pointer p is reached: 0 not host memory (or capturing: strided
-// copy), 1 staged, 2 directly (pinned, mapped: *dp its device address).
+// Whether `bytes` from device pointer p lie inside one allocation; a buffer
+// that is too short goes to the strided copy, which reports it.
+static bool in_allocation(const void* p, size_t bytes) {
+  static PFN_cuMemGetAddressRange_v3020 range = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      range = reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
+  });
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
+  return range && range(&base, &size, q) == CUDA_SUCCESS && q - base + bytes <= size;
+}
+
+// How user pointer p is reached: 0 neither of the below (or capturing: strided
+// copy), 1 staged, 2 directly (pinned and mapped, or this device's memory:
+// *dp its device address).
 static int host_route(sc_handle* h, const void* p, void** dp) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 0;
@@ -1545,10 +1599,15 @@ static int host_route(sc_handle* h, const void* p, void** dp) {
     return 0;
   }
   // the repack kernel moves whole elements (8 or 16 bytes): a buffer not
-  // aligned to that goes through the staged copy
+  // aligned to that goes through the staged (host) or strided (device) copy
   const bool aligned = reinterpret_cast<uintptr_t>(p) % h->csize == 0;
   if (a.type == cudaMemoryTypeHost && h->copy_mode == 1 && a.devicePointer && aligned) {
     *dp = a.devicePointer;
+    return 2;
+  }
+  if (a.type == cudaMemoryTypeDevice && a.device == h->device && aligned &&
+      in_allocation(p, h->csize * h->g.nxh * (size_t)h->g.ny * h->g.nz)) {
+    *dp = const_cast<void*>(p);
     return 2;
   }
   if (a.type != cudaMemoryTypeHost && a.type != cudaMemoryTypeUnregistered) return 0;
@@ -1563,35 +1622,60 @@ static int host_route(sc_handle* h, const void* p, void** dp) {
   return 1;
 }
 
-int copy_in(sc_handle* h, void* dst, const void* src) {
+// user memory (reference layout) -> n padded device fields; those reached
+// directly share one launch
+int copy_in(sc_handle* h, void* const* dst, const void* const* src, int n) {
   const size_t w = h->csize * h->g.nxh, rows = (size_t)h->g.ny * h->g.nz;
-  void* dp = nullptr;
-  switch (host_route(h, src, &dp)) {
-    case 1:
-      SC_CUDA(cudaMemcpyAsync(h->stage, src, w * rows, cudaMemcpyHostToDevice, h->stream));
-      return repack(h, dst, h->g.nxp, h->stage, h->g.nxh);
-    case 2:
-      return repack(h, dst, h->g.nxp, dp, h->g.nxh);
-    default:
-      SC_CUDA(cudaMemcpy2DAsync(dst, h->csize * h->g.nxp, src, w, w, rows, cudaMemcpyDefault, h->stream));
-      return SC_OK;
+  void* kd[kRepackMax];
+  const void* ks[kRepackMax];
+  int nk = 0;
+  for (int i = 0; i < n; ++i) {
+    void* dp = nullptr;
+    switch (host_route(h, src[i], &dp)) {
+      case 1: {
+        SC_CUDA(cudaMemcpyAsync(h->stage, src[i], w * rows, cudaMemcpyHostToDevice, h->stream));
+        const void* st[1] = {h->stage};
+        SC_TRY(repack(h, dst + i, h->g.nxp, st, h->g.nxh, 1));
+        break;
+      }
+      case 2:
+        kd[nk] = dst[i];
+        ks[nk++] = dp;
+        break;
+      default:
+        SC_CUDA(cudaMemcpy2DAsync(dst[i], h->csize * h->g.nxp, src[i], w, w, rows, cudaMemcpyDefault, h->stream));
+    }
   }
+  return nk ? repack(h, kd, h->g.nxp, ks, h->g.nxh, nk) : SC_OK;
 }
-int copy_out(sc_handle* h, void* dst, const void* src) {
+int copy_in(sc_handle* h, void* dst, const void* src) { return copy_in(h, &dst, &src, 1); }
+
+// n padded device fields -> user memory
+int copy_out(sc_handle* h, void* const* dst, const void* const* src, int n) {
   const size_t w = h->csize * h->g.nxh, rows = (size_t)h->g.ny * h->g.nz;
-  void* dp = nullptr;
-  switch (host_route(h, dst, &dp)) {
-    case 1:
-      SC_TRY(repack(h, h->stage, h->g.nxh, src, h->g.nxp));
-      SC_CUDA(cudaMemcpyAsync(dst, h->stage, w * rows, cudaMemcpyDeviceToHost, h->stream));
-      return SC_OK;
-    case 2:
-      return repack(h, dp, h->g.nxh, src, h->g.nxp);
-    default:
-      SC_CUDA(cudaMemcpy2DAsync(dst, w, src, h->csize * h->g.nxp, w, rows, cudaMemcpyDefault, h->stream));
-      return SC_OK;
+  void* kd[kRepackMax];
+  const void* ks[kRepackMax];
+  int nk = 0;
+  for (int i = 0; i < n; ++i) {
+    void* dp = nullptr;
+    switch (host_route(h, dst[i], &dp)) {
+      case 1: {
+        void* st[1] = {h->stage};
+        SC_TRY(repack(h, st, h->g.nxh, src + i, h->g.nxp, 1));
+        SC_CUDA(cudaMemcpyAsync(dst[i], h->stage, w * rows, cudaMemcpyDeviceToHost, h->stream));
+        break;
+      }
+      case 2:
+        kd[nk] = dp;
+        ks[nk++] = src[i];
+        break;
+      default:
+        SC_CUDA(cudaMemcpy2DAsync(dst[i], w, src[i], h->csize * h->g.nxp, w, rows, cudaMemcpyDefault, h->stream));
+    }
   }
+  return nk ? repack(h, kd, h->g.nxh, ks, h->g.nxp, nk) : SC_OK;
 }
+int copy_out(sc_handle* h, void* dst, const void* src) { return copy_out(h, &dst, &src, 1); }
 void* slot(sc_handle* h, int i) {
   return static_cast<char*>(h->fields) + (size_t)i * h->g.field * h->csize;
 }
@@ -1781,6 +1865,7 @@ int sc_create(const sc_params* pin, sc_handle** out) {
   {
     int dev = 0;
     SC_CUDA(cudaGetDevice(&dev));
+    h->device = dev;
     SC_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev));
   }
   SC_CUDA(cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking));
@@ -1864,7 +1949,8 @@ int sc_set_dt(sc_handle* h, double dt) {
 int sc_set_state(sc_handle* h, const void* vx, const void* vy, const void* vz) {
   if (!h || !vx || !vy || !vz) return fail(SC_ERR_INVALID, "null argument");
   const void* v[3] = {vx, vy, vz};
-  for (int c = 0; c < 3; ++c) SC_TRY(copy_in(h, slot(h, S_V + c), v[c]));
+  void* f[3] = {slot(h, S_V), slot(h, S_V + 1), slot(h, S_V + 2)};
+  SC_TRY(copy_in(h, f, v, 3));
   SC_CUDA(cudaStreamSynchronize(h->stream));
   h->step = 0;
   h->ab2_pass = 0;
@@ -1876,13 +1962,14 @@ int sc_set_state(sc_handle* h, const void* vx, const void* vy, const void* vz) {
 int sc_get_state(sc_handle* h, void* vx, void* vy, void* vz) {
   if (!h || !vx || !vy || !vz) return fail(SC_ERR_INVALID, "null argument");
   void* v[3] = {vx, vy, vz};
-  for (int c = 0; c < 3; ++c) SC_TRY(copy_out(h, v[c], slot(h, S_V + c)));
+  const void* f[3] = {slot(h, S_V), slot(h, S_V + 1), slot(h, S_V + 2)};
+  SC_TRY(copy_out(h, v, f, 3));
   SC_CUDA(cudaStreamSynchronize(h->stream));
   return SC_OK;
 }
 
 int sc_set_state_device(sc_handle* h, const void* vx, const void* vy, const void* vz) {
-  return sc_set_state(h, vx, vy, vz);   // cudaMemcpyDefault resolves device pointers
+  return sc_set_state(h, vx, vy, vz);   // host_route tells device pointers
 }
 int sc_get_state_device(sc_handle* h, void* vx, void* vy, void* vz) {
   return sc_get_state(h, vx, vy, vz);

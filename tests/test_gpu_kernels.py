@@ -110,3 +110,28 @@ def test_kx0_copy(specns_lib, shape, prec):
     ref = R.rk4_run(vd, g, 2)
     assert rel_l2(out, ref) < TOL[prec]
     assert rel_l2([a[:, :, 0] for a in out], [a[:, :, 0] for a in ref]) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", [(8, 8, 8), (32, 16, 64), (512, 8, 32)])
+@pytest.mark.parametrize("shift", [0, 4])
+def test_device_state_round_trip(specns_lib, shape, prec, shift):
+    """States in device memory, on the element's alignment and off it."""
+    torch = pytest.importorskip("torch")
+    nx, ny, nz = shape
+    n = nz * ny * (nx // 2 + 1)
+    cs = 8 if prec == S.SC_FP32 else 16
+    bufs = [torch.zeros(n * cs + 16, dtype=torch.uint8, device="cuda") for _ in range(6)]
+    rng = np.random.default_rng(3)
+    v = [(rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(DT[prec]) for _ in range(3)]
+    for b, a in zip(bufs, v):
+        b[shift:shift + n * cs] = torch.from_numpy(a.view(np.uint8)).cuda()
+    torch.cuda.synchronize()
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz)) as h:
+        h.set_state_device(*(b.data_ptr() + shift for b in bufs[:3]))
+        host = h.get_state()
+        h.get_state_device(*(b.data_ptr() + shift for b in bufs[3:]))
+    for a, b, c in zip(v, host, bufs[3:]):
+        assert np.array_equal(b.reshape(-1), a)
+        assert np.array_equal(c[shift:shift + n * cs].cpu().numpy().view(DT[prec]), a)
+        assert int(c[:shift].sum()) == 0 and int(c[shift + n * cs:].sum()) == 0
