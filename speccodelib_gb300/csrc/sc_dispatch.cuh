@@ -68,6 +68,14 @@ cudaError_t launch_xpass(const FieldList<T>& fin, const FieldList<T>& fout, cons
   return cudaGetLastError();
 }
 
+// XP_SCALAR: the lengths that neither the warp nor the lane-group x-pass has
+template <typename T, int LOGM>
+cudaError_t launch_xpass_scalar(const FieldList<T>& fin, const FieldList<T>& fout, const Geom& g, const C2<T>* twM,
+                                const C2<T>* twN, const XArgs<T>& xa, cudaStream_t s) {
+  if constexpr (LOGM <= 3 || LOGM >= 9) return launch_xpass<T, LOGM, XP_SCALAR>(fin, fout, g, twM, twN, xa, s);
+  else return cudaErrorNotSupported;
+}
+
 template <typename T, int LOGN, bool INV>
 cudaError_t launch_plain_tma(const CUtensorMap& map, const TmaPass<T>& tp, const Geom& g, const C2<T>* tw,
                              int nsm, cudaStream_t s) {
@@ -106,6 +114,19 @@ cudaError_t launch_zfwd_fields_tma(const CUtensorMap& fmap, const StageArgs<T>& 
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Cfg::P - 1) / Cfg::P, g.ny);
   k<<<grid, Cfg::NT, sm, s>>>(fmap, st, g, tw, err);
+  return cudaGetLastError();
+}
+
+template <typename T, int LOGN>
+cudaError_t launch_zfwd_div(const CUtensorMap& fmap, const CUtensorMap& omap, const DivArgs<T>& da, const Geom& g,
+                            const C2<T>* tw, int* err, cudaStream_t s) {
+  using Cfg = TmaCfg<T, LOGN>;
+  auto k = zfwd_div_tma_kernel<T, LOGN>;
+  constexpr size_t sm = 3 * Cfg::TILE_BYTES + kSmemAlignPad;
+  static cudaError_t attr = smem_attr(k, sm);
+  if (attr != cudaSuccess) return attr;
+  dim3 grid((g.nxh + Cfg::P - 1) / Cfg::P, g.ny);
+  k<<<grid, ZfCfg<T, LOGN>::NT, sm, s>>>(fmap, omap, da, g, tw, err);
   return cudaGetLastError();
 }
 
@@ -343,7 +364,8 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
 
 #define SC_XGROUP_CASE(T, L)                                                                     \
   case L:                                                                                        \
-    return mode == sc::XW_ADJ    ? sc::launch_xgroup<T, L, sc::XW_ADJ>(fin, fout, g, twM, twN, xa, s)  \
+    return mode == sc::XW_ADJ      ? sc::launch_xgroup<T, L, sc::XW_ADJ>(fin, fout, g, twM, twN, xa, s)  \
+           : mode == sc::XW_SCALAR ? sc::launch_xgroup<T, L, sc::XW_SCALAR>(fin, fout, g, twM, twN, xa, s) \
            : mode == sc::XW_SMAG ? sc::launch_xgroup<T, L, sc::XW_SMAG>(fin, fout, g, twM, twN, xa, s) \
                                  : sc::launch_xgroup<T, L, sc::XW_DNS>(fin, fout, g, twM, twN, xa, s);
 
@@ -352,7 +374,8 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
 
 #define SC_XWARP_CASE(T, L)                                                                      \
   case L:                                                                                        \
-    return mode == sc::XW_ADJ    ? sc::launch_xwarp<T, L, sc::XW_ADJ>(fin, fout, g, twM, twN, xa, s)  \
+    return mode == sc::XW_ADJ      ? sc::launch_xwarp<T, L, sc::XW_ADJ>(fin, fout, g, twM, twN, xa, s)  \
+           : mode == sc::XW_SCALAR ? sc::launch_xwarp<T, L, sc::XW_SCALAR>(fin, fout, g, twM, twN, xa, s) \
            : mode == sc::XW_SMAG ? sc::launch_xwarp<T, L, sc::XW_SMAG>(fin, fout, g, twM, twN, xa, s) \
                                  : sc::launch_xwarp<T, L, sc::XW_DNS>(fin, fout, g, twM, twN, xa, s);
 
@@ -395,6 +418,15 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
     }                                                                                            \
   }                                                                                              \
   template <>                                                                                    \
+  cudaError_t sc::Launch<T>::zfwd_div_tma(int logn, const CUtensorMap& fmap, const CUtensorMap& omap, \
+                                          const DivArgs<T>& da, const Geom& g, const C2<T>* tw,  \
+                                          int* err, cudaStream_t s) {                            \
+    switch (logn) {                                                                              \
+      SC_LOGN_CASES(SC_ZFWDDIV_CASE_##T)                                                         \
+      default: return cudaErrorInvalidValue;                                                     \
+    }                                                                                            \
+  }                                                                                              \
+  template <>                                                                                    \
   cudaError_t sc::Launch<T>::zfwd_tma(int logn, const CUtensorMap& lmap, const CUtensorMap& vmap,  \
                                       int vstore, const StageArgs<T>& st, const Geom& g,         \
                                       const C2<T>* tw, int* err, cudaStream_t s) {               \
@@ -414,6 +446,8 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
 #define SC_ZINVTMA_CASE_double(L) case L: return sc::launch_zinv_tma<double, L>(vmap, za, out, g, tw, err, s);
 #define SC_ZFWDFIELDS_CASE_float(L) case L: return sc::launch_zfwd_fields_tma<float, L, 9>(fmap, st, g, tw, err, s);
 #define SC_ZFWDFIELDS_CASE_double(L) case L: return sc::launch_zfwd_fields_tma<double, L, 9>(fmap, st, g, tw, err, s);
+#define SC_ZFWDDIV_CASE_float(L) case L: return sc::launch_zfwd_div<float, L>(fmap, omap, da, g, tw, err, s);
+#define SC_ZFWDDIV_CASE_double(L) case L: return sc::launch_zfwd_div<double, L>(fmap, omap, da, g, tw, err, s);
 #define SC_ZFWDTMA_CASE_float(L) case L: return sc::launch_zfwd_tma<float, L>(lmap, vmap, vstore, st, g, tw, err, s);
 #define SC_ZFWDTMA_CASE_double(L) case L: return sc::launch_zfwd_tma<double, L>(lmap, vmap, vstore, st, g, tw, err, s);
 
@@ -577,6 +611,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
       case sc::XP_C2R3: return sc::launch_xpass<T, L, sc::XP_C2R3>(fin, fout, g, twM, twN, xa, s); \
       case sc::XP_R2C3: return sc::launch_xpass<T, L, sc::XP_R2C3>(fin, fout, g, twM, twN, xa, s); \
       case sc::XP_ADJ: return sc::launch_xpass<T, L, sc::XP_ADJ>(fin, fout, g, twM, twN, xa, s);   \
+      case sc::XP_SCALAR: return sc::launch_xpass_scalar<T, L>(fin, fout, g, twM, twN, xa, s);     \
       default: return cudaErrorInvalidValue;                                          \
     }
 #define SC_XPASS_CASE_float(L) SC_XPASS_BODY(float, L)

@@ -57,6 +57,7 @@ template <typename T> struct AdjArgs;
 template <typename T> struct AdjOpArgs;
 template <typename T> struct FusedArgs;
 template <typename T> struct BandArgs;
+template <typename T> struct DivArgs;
 
 template <typename T> struct Launch {
   static int tile();                                   // pencil tile width P
@@ -103,6 +104,10 @@ template <typename T> struct Launch {
   // through vmap (st.vout[0..2], tiles as lmap)
   static cudaError_t zfwd_tma(int logn, const CUtensorMap& lmap, const CUtensorMap& vmap, int vstore,
                               const StageArgs<T>& st, const Geom& g, const C2<T>* tw, int* err, cudaStream_t s);
+  // z-forward of a scalar's three flux fields (fmap) with the divergence,
+  // forcing, symmetrize and mask, into the field of omap (tiles tma_tile wide)
+  static cudaError_t zfwd_div_tma(int logn, const CUtensorMap& fmap, const CUtensorMap& omap, const DivArgs<T>& da,
+                                  const Geom& g, const C2<T>* tw, int* err, cudaStream_t s);
   // z-forward of nin fields (9: the LES Lamb vector and tau_ij) through a
   // TMA ring, fmap tiled tma_tile wide; cudaErrorNotSupported otherwise
   static cudaError_t zfwd_fields_tma(int logn, int nin, const CUtensorMap& fmap, const StageArgs<T>& st,

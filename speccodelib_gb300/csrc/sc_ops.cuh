@@ -370,13 +370,14 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
 // ---------------------------------------------------------------------------
 // force_rot.f90's coefficient on the device: a = eps / (2 kinet + tiny), kinet
 // the 1/2-weighted (kx = 0) energy of v on lo2 <= k2 < hi2 (force_rot.f90:
-// 16-27).  One block walks the band's bounding box |k_i| <= floor(sqrt(hi2))
+// 16-27); with nf = 1 and tiny = 0 forcephi_rot.f90's, of one field.  One block walks the band's bounding box |k_i| <= floor(sqrt(hi2))
 // in a fixed order and sums in FP64, so the result is deterministic and no
 // host synchronisation is needed (the rotating pass reads *out in its
 // z-forward epilogue).
 // ---------------------------------------------------------------------------
 template <typename T> struct BandArgs {
   const C2<T>* v[3];
+  int nf;                 // fields summed (1 or 3)
   double lo2, hi2, eps, tiny;
   double* out;
 };
@@ -402,8 +403,7 @@ __global__ void __launch_bounds__(256) band_coef_kernel(BandArgs<T> ba, Geom g) 
     const int iy = ky < 0 ? ky + g.ny : ky, iz = kz < 0 ? kz + g.nz : kz;
     const long long idx = ((long long)iz * g.ny + iy) * g.nxp + ix;
     double e = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
+    for (int c = 0; c < ba.nf; ++c) {
       const C2<T> a = ba.v[c][idx];
       e += (double)a.x * a.x + (double)a.y * a.y;
     }

@@ -733,15 +733,17 @@ __global__ void fixup_kx0_kernel(StageArgs<T> st, Geom g) {
 // ---------------------------------------------------------------------------
 // xpass: per-row c2r, physical-space product, r2c
 // ---------------------------------------------------------------------------
-enum XpMode { XP_DNS = 0, XP_SMAG = 1, XP_C2R3 = 2, XP_R2C3 = 3, XP_ADJ = 4 };
-// modes of the warp-per-row x-pass (sc_xwarp.cuh)
-enum XwMode { XW_DNS = 0, XW_ADJ = 1, XW_SMAG = 2 };
+enum XpMode { XP_DNS = 0, XP_SMAG = 1, XP_C2R3 = 2, XP_R2C3 = 3, XP_ADJ = 4, XP_SCALAR = 5 };
+// modes of the warp-per-row and lane-group x-passes (sc_xwarp.cuh, sc_xgroup.cuh)
+enum XwMode { XW_DNS = 0, XW_ADJ = 1, XW_SMAG = 2, XW_SCALAR = 3 };
 template <int MODE> struct XpIO;
 template <> struct XpIO<XP_DNS> { static constexpr int fin = 6, fout = 3; };
 template <> struct XpIO<XP_SMAG> { static constexpr int fin = 12, fout = 9; };
 template <> struct XpIO<XP_C2R3> { static constexpr int fin = 3, fout = 3; };
 template <> struct XpIO<XP_R2C3> { static constexpr int fin = 3, fout = 3; };
 template <> struct XpIO<XP_ADJ> { static constexpr int fin = 9, fout = 6; };   // (u, w, phi) -> (w x phi, phi x u)
+
+template <> struct XpIO<XP_SCALAR> { static constexpr int fin = 7, fout = 6; };   // (u, w, phi) -> (u x w, u phi)
 
 template <typename T> struct XArgs {
   const C2<T>* twx;        // the twiddle table base (WarpTw blocks after entry 4096)
@@ -857,6 +859,10 @@ xpass_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __restric
             const int c1 = (gq + 1) % 3, c2 = (gq + 2) % 3;
             const C ua = U(c1), ub = U(c2), wa = U(3 + c1), wb = U(3 + c2);
             res = mk<C>((ua.x * wb.x - ub.x * wa.x) * sc, (ua.y * wb.y - ub.y * wa.y) * sc);
+          } else if (MODE == XP_SCALAR) {
+            // convecphi_dns.f90:20-23: u_i phi
+            const C ui = U(gq - 3), ph = U(6);
+            res = mk<C>(ui.x * ph.x * sc, ui.y * ph.y * sc);
           } else {
             // smag.f90:41-64: tau_ij = -2 c1 D^2 |S| S_ij / N^3
             const C s11 = U(6), s12 = U(7), s13 = U(8), s22 = U(9), s23 = U(10), s33 = U(11);

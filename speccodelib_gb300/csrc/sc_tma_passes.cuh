@@ -460,4 +460,106 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
   }
 }
 
+// z-forward pass of a passive scalar's flux u phi (three fields, scaled by
+// 1/N^3 in the x-pass): w_phi = i k . (u phi)^ (convecphi_dns.f90:25-47), plus
+// the scalar's forcing, symmetrize and the dealiasing mask, leaving by bulk
+// tensor stores.  Three forward passes, a divergence pass, up to two forcing
+// passes, two symmetrize passes and the mask over whole fields become the
+// flux read once and w_phi written once (4 F); latency-bound at 2 CTAs per SM
+// as the other z-forward passes (86 us at 256^3 FP32, 3.1 TB/s).
+template <typename T> struct DivArgs {
+  const C2<T>* phi;       // band forcing: += (*fcoef) phi on flo2 <= k2 < fhi2 (fcoef may be null)
+  const double* fcoef;
+  double flo2, fhi2;
+  const C2<T>* vz;        // mean gradient: -= meangrad vz (vz may be null)
+  T meangrad;
+  int mask;               // zero k2 >= kcut2 (k2 > 0)
+  double kcut2;
+};
+
+template <typename T, int LOGN>
+__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(ZfCfg<T, LOGN>::NT, 2)
+zfwd_div_tma_kernel(const __grid_constant__ CUtensorMap fmap, const __grid_constant__ CUtensorMap omap, DivArgs<T> da,
+                    Geom g, const C2<T>* __restrict__ tw, int* err) {
+  using Cfg = TmaCfg<T, LOGN>;
+  using E = typename ZfCfg<T, LOGN>::Engine;
+  using C = C2<T>;
+  constexpr int P = Cfg::P;
+  constexpr int N = Cfg::N;
+  constexpr int NT = ZfCfg<T, LOGN>::NT;
+  extern __shared__ __align__(128) unsigned char smdyn[];
+  unsigned char* smraw = align128(smdyn);
+  C* w[3];
+  for (int c = 0; c < 3; ++c) w[c] = reinterpret_cast<C*>(smraw + c * Cfg::TILE_BYTES);
+  __shared__ __align__(8) uint64_t bars[3];
+  const int kx0 = blockIdx.x * P;
+  const int iy = paired_row(blockIdx.y, g.ny);
+  const int nvalid = min(P, g.nxh - kx0);
+  const long long zstride = (long long)g.ny * g.nxp;
+  const long long base = (long long)iy * g.nxp + kx0;
+  const bool paired = kx0 == 0;   // meets its partner: both CTAs stay until then
+  if (!paired && launch_failed(err)) return;
+  if (threadIdx.x == 0) {
+    for (int c = 0; c < 3; ++c) mbar_init(&bars[c], 1);
+    fence_mbar_init();
+    fence_proxy_async();
+    for (int c = 0; c < 3; ++c)
+      tma_issue_tile<Cfg>(w[c], &fmap, &bars[c], 2, kx0, iy, c, P, Cfg::TILE_BYTES);
+  }
+  __syncthreads();
+  bool ok = true;
+  for (int c = 0; c < 3; ++c) {
+    ok = mbar_wait_bounded(&bars[c], 0, err) && ok;
+    if (!ok && !paired) return;
+    E::template run_inplace<false>(w[c], tw);
+  }
+  const int kyi = wavenum(iy, g.ny);
+  const int lo_b = k2_lt(da.flo2), hi_b = k2_lt(da.fhi2), kc_b = k2_lt(da.kcut2);
+  const bool fblock = da.fcoef && kx0 * kx0 + kyi * kyi < hi_b;
+  const T fc = fblock ? (T)*da.fcoef : T(0);
+  constexpr int EB = NT >= 512 ? 2 : 4;
+  for (int e0 = threadIdx.x; e0 < P * N; e0 += NT * EB) {
+    C vz[EB];
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      const int e = e0 + i * NT;
+      const int p = e % P, iz = e / P;
+      vz[i] = czero<C>();
+      if (da.vz && e < P * N && p < nvalid) vz[i] = da.vz[base + iz * zstride + p];
+    }
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      const int e = e0 + i * NT;
+      if (e >= P * N) continue;
+      const int p = e % P, iz = e / P, ix = kx0 + p;
+      const int kzi = wavenum(iz, g.nz), k2 = ix * ix + kyi * kyi + kzi * kzi;
+      C d = cadd(cadd(cscale(w[0][e], (T)ix), cscale(w[1][e], (T)kyi)), cscale(w[2][e], (T)kzi));
+      d = cmuli(d);
+      if (fblock && k2 >= lo_b && k2 < hi_b && p < nvalid) d = cadd(d, cscale(da.phi[base + iz * zstride + p], fc));
+      if (da.vz) d = csub(d, cscale(vz[i], da.meangrad));
+      if (iy == g.ny / 2 || iz == g.nz / 2 || ix == g.nxh - 1 || k2 == 0 || (da.mask && k2 >= kc_b)) d = czero<C>();
+      w[0][e] = d;
+    }
+  }
+  if (paired) {
+    // the kx = 0 copy, as hermitian_column: zeroing and mask are the same at k and -k
+    cluster_sync();
+    const uint32_t from = iy == 0 ? cluster_rank() : (cluster_rank() ^ 1u);
+    for (int n = threadIdx.x; n < N; n += NT)
+      if (n > N / 2 || (n == 0 && iy > g.ny / 2))
+        w[0][n * P] = iy == g.ny / 2 ? czero<C>() : cconj(cluster_load(&w[0][((N - n) % N) * P], from));
+    cluster_sync();
+    if (!ok) return;
+  }
+  fence_proxy_async();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int h = 0; h < Cfg::NBOX; ++h)
+      tma_store_4d(&omap, reinterpret_cast<char*>(w[0]) + (size_t)h * Cfg::BOX * P * sizeof(C), kx0 * Cfg::U, iy,
+                   h * Cfg::BOX, 0);
+    tma_store_commit();
+    tma_store_wait_read<0>();
+  }
+}
+
 }  // namespace sc

@@ -195,6 +195,22 @@ template <typename T, int LOGM> struct XgRow {
     store_r2c(x, of[1], sc);
   }
 
+  // of[c] = r2c(sc a_c phi) (convecphi_dns.f90:20-23)
+  __device__ __forceinline__ void flux_store(const C* pf, C* const of[3], T sc) const {
+    C b[E];
+    load_phys(pf, b);
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      C x[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const C a = kept(c, i);
+        x[i] = mk<C>(a.x * b[i].x, a.y * b[i].y);
+      }
+      store_r2c(x, of[c], sc);
+    }
+  }
+
   // tau_ij = tcoef |S| S_ij (smag.f90:41-64) of the S_ij rows sf (order 11 12
   // 13 22 23 33), kept in rows 0..5
   __device__ __forceinline__ void tau_store(const C* const sf[6], C* const of[6], T tcoef) const {
@@ -272,9 +288,13 @@ xpass_group_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __r
   const C* u[3] = {fin.f[0], fin.f[1], fin.f[2]};
   const C* w[3] = {fin.f[3], fin.f[4], fin.f[5]};
   C* o[3] = {fout.f[0], fout.f[1], fout.f[2]};
-  if constexpr (MODE == XW_DNS) {
+  if constexpr (MODE == XW_DNS || MODE == XW_SCALAR) {
     R.load_a(u);
     R.cross_store(w, o, xa.scale);
+    if constexpr (MODE == XW_SCALAR) {
+      C* of[3] = {fout.f[3], fout.f[4], fout.f[5]};
+      R.flux_store(fin.f[6], of, xa.scale);
+    }
   } else if constexpr (MODE == XW_SMAG) {
     const C* s[6] = {fin.f[6], fin.f[7], fin.f[8], fin.f[9], fin.f[10], fin.f[11]};
     C* ot[6] = {fout.f[3], fout.f[4], fout.f[5], fout.f[6], fout.f[7], fout.f[8]};

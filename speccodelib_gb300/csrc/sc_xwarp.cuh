@@ -484,19 +484,22 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
     }
   }
 
+  // a_c at points i0 .. i0 + G - 1 (G = min(E, 4))
+  __device__ __forceinline__ void a_group(int c, int i0, C (&a)[4]) const {
+    static_assert(E % 4 == 0 || !TM, "a rows are read four points at a time");
+    if constexpr (TM) a4(c, i0, a);
+    else {
+#pragma unroll
+      for (int i = 0; i < (E < 4 ? E : 4); ++i) a[i] = as[(c * E + i0 + i) * 32 + lane];
+    }
+  }
+
   // out = r2c(sc * (a x b)), b = c2r of rows bf[0..2]; the cross product is
   // accumulated as the b components arrive (convec_dns.f90:30-38: even
   // points in .x, odd points in .y)
   __device__ __forceinline__ void cross_store(const C* const bf[3], C* const of[3], T sc) {
-    static_assert(E % 4 == 0 || !TM, "a rows are read four points at a time");
     constexpr int G = E < 4 ? E : 4;   // points per group of a reads
-    auto A = [&](int c, int i0, C (&a)[4]) {
-      if constexpr (TM) a4(c, i0, a);
-      else {
-#pragma unroll
-        for (int i = 0; i < G; ++i) a[i] = as[(c * E + i0 + i) * 32 + lane];
-      }
-    };
+    auto A = [&](int c, int i0, C (&a)[4]) { a_group(c, i0, a); };
     // L_z is complete after b_y and leaves before b_z is transformed, so
     // only L_x and L_y stay in registers through the last transform
     auto out = [&](C (&l)[E], int c) {
@@ -556,6 +559,29 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
     }
     out(l0, 0);
     out(l1, 1);
+  }
+
+  // of[c] = r2c(sc * a_c phi), phi = c2r of row pf (convecphi_dns.f90:20-23)
+  __device__ __forceinline__ void flux_store(const C* pf, C* const of[3], T sc) {
+    constexpr int G = E < 4 ? E : 4;
+    C b[E];
+    load_z(pf, b);
+    WF::template nat_to_scr<true, TX>(b, sm, twM, lane, tx);
+#pragma unroll
+    for (int i = 0; i < E; ++i) b[i] = cscale(b[i], sc);
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      C x[E];
+#pragma unroll
+      for (int i0 = 0; i0 < E; i0 += G) {
+        C a[4];
+        a_group(c, i0, a);
+#pragma unroll
+        for (int ii = 0; ii < G; ++ii) x[i0 + ii] = mk<C>(a[ii].x * b[i0 + ii].x, a[ii].y * b[i0 + ii].y);
+      }
+      WF::template scr_to_nat<false, TX>(x, sm, twM, lane, tx);
+      r2c_store(x, of[c] + off);
+    }
   }
 
   // S_ij rows sf[0..5] (order 11 12 13 22 23 33) -> c2r, kept in shared
@@ -655,6 +681,8 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
 //   w x phi = -(phi x w) into fout[0..2], then phi x u into fout[3..5];
 //   fout must not alias u (read by the second product) -- the host passes
 //   the w and phi slots.
+// XW_SCALAR: fin = (u, w, phi) -> fout[0..2] = r2c(u x w / N^3) and fout[3..5] =
+//   r2c(u phi / N^3), in place on u and w (phi's own field is only read).
 template <typename T, int LOGM, int MODE>
 __global__ void __launch_bounds__(XwCfg<T, LOGM, MODE>::NT, XwCfg<T, LOGM, MODE>::MINB)
 xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __restrict__ twM,
@@ -689,9 +717,9 @@ xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __re
     R.off = row * g.nxp;
     R.lane = lane;
     // the input fields in the order their rows are consumed
-    const C* seq[Cfg::KEPT == 9 ? 12 : (MODE == XW_ADJ ? 9 : 6)];
-    if constexpr (MODE == XW_DNS) {
-      for (int f = 0; f < 6; ++f) seq[f] = fin.f[f];
+    const C* seq[Cfg::KEPT == 9 ? 12 : (MODE == XW_ADJ ? 9 : (MODE == XW_SCALAR ? 7 : 6))];
+    if constexpr (MODE == XW_DNS || MODE == XW_SCALAR) {
+      for (int f = 0; f < (MODE == XW_SCALAR ? 7 : 6); ++f) seq[f] = fin.f[f];
     } else if constexpr (MODE == XW_SMAG) {
       for (int f = 0; f < 3; ++f) seq[f] = fin.f[f];          // u (load_a)
       for (int f = 0; f < 6; ++f) seq[3 + f] = fin.f[6 + f];  // S_ij (load_s)
@@ -710,12 +738,16 @@ xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __re
       R.err = xa.err;
       R.stage_start();
     }
-    if constexpr (MODE == XW_DNS) {
+    if constexpr (MODE == XW_DNS || MODE == XW_SCALAR) {
       const C* a[3] = {fin.f[0], fin.f[1], fin.f[2]};
       const C* b[3] = {fin.f[3], fin.f[4], fin.f[5]};
       C* o[3] = {fout.f[0], fout.f[1], fout.f[2]};
       R.load_a(a);
       R.cross_store(b, o, xa.scale);
+      if constexpr (MODE == XW_SCALAR) {
+        C* of[3] = {fout.f[3], fout.f[4], fout.f[5]};
+        R.flux_store(fin.f[6], of, xa.scale);
+      }
     } else if constexpr (MODE == XW_SMAG) {
       const C* a[3] = {fin.f[0], fin.f[1], fin.f[2]};
       const C* b[3] = {fin.f[3], fin.f[4], fin.f[5]};

@@ -135,3 +135,34 @@ def test_device_state_round_trip(specns_lib, shape, prec, shift):
         assert np.array_equal(b.reshape(-1), a)
         assert np.array_equal(c[shift:shift + n * cs].cpu().numpy().view(DT[prec]), a)
         assert int(c[:shift].sum()) == 0 and int(c[shift + n * cs:].sum()) == 0
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", [(8, 16, 8), (16, 8, 32), (32, 8, 16), (64, 16, 8), (128, 8, 64), (256, 8, 8),
+                                   (512, 8, 16), (1024, 8, 8), (32, 32, 512)])
+def test_scalar_passes_shapes(specns_lib, shape, prec):
+    """The scalar's flux in the velocity's passes at every row length (warp,
+    lane-group and block x-pass), both forced scalar solvers; and with the
+    kx = 0 copy off its symmetric values."""
+    nx, ny, nz = shape
+    f = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 61, ncomp=4, kcut=4.0)]
+    f[3][:, :, 0] *= DT[prec](1 + 0.2j)
+    kw = dict(nu=0.02, dt=1e-3, eps=0.2)
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, **kw))
+    fd = [a.astype(np.complex128) for a in f]
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, **kw)) as h:
+        h.set_state(*f[:3])
+        h.set_scalar(f[3])
+        h.rot_scalar_steps(3, om=2.0, fk1=1.0, fk2=2.5, pr=0.7, scalarforced=True, epsphi=0.05)
+        rot = list(h.get_state()) + [h.get_scalar()]
+        h.set_state(*f[:3])
+        h.set_scalar(f[3])
+        for dt in (1e-3, 8e-4, 1.2e-3):
+            h.ab2v_scalar_pass(dt, 0.7, True, 0.4)
+        var = list(h.get_state()) + [h.get_scalar()]
+    v, phi, _, _ = R.rot_scalar_run(fd[:3], fd[3], g, 3, 2.0, 1.0, 2.5, 0.7, True, 0.05)
+    assert rel_l2(rot[:3], v) < TOL[prec]
+    assert rel_l2(rot[3], phi) < TOL[prec]
+    v, phi, _, _ = R.ab2v_scalar_run(fd[:3], fd[3], g, (1e-3, 8e-4, 1.2e-3), 0.7, True, 0.4)
+    assert rel_l2(var[:3], v) < TOL[prec]
+    assert rel_l2(var[3], phi) < TOL[prec]
