@@ -8,6 +8,7 @@
 #include "sc_xwarp.cuh"
 #include "sc_adjoint.cuh"
 #include "sc_fused.cuh"
+#include "sc_les.cuh"
 
 namespace sc {
 
@@ -114,6 +115,35 @@ cudaError_t launch_zfwd_fields_tma(const CUtensorMap& fmap, const StageArgs<T>& 
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Cfg::P - 1) / Cfg::P, g.ny);
   k<<<grid, Cfg::NT, sm, s>>>(fmap, st, g, tw, err);
+  return cudaGetLastError();
+}
+
+template <typename T, int LOGN>
+cudaError_t launch_les_y(bool inv, const CUtensorMap& map, const TmaPass<T>& tp, const Geom& g, const C2<T>* tw,
+                         int nsm, cudaStream_t s) {
+  using Cfg = TmaCfg<T, LOGN>;
+  auto k = inv ? les_yinv_kernel<T, LOGN> : les_yfwd_kernel<T, LOGN>;
+  constexpr size_t sm = LesYCfg<T, LOGN>::SMEM;
+  static cudaError_t attr_i = smem_attr(les_yinv_kernel<T, LOGN>, sm);
+  static cudaError_t attr_f = smem_attr(les_yfwd_kernel<T, LOGN>, sm);
+  if (attr_i != cudaSuccess) return attr_i;
+  if (attr_f != cudaSuccess) return attr_f;
+  const long long total = (long long)tp.ntx * tp.nouter * (inv ? 6 : 5);
+  long long grid = (long long)nsm * 2;
+  if (grid > total) grid = total;
+  k<<<(unsigned)grid, Cfg::NT, sm, s>>>(map, tp, g, tw);
+  return cudaGetLastError();
+}
+
+template <typename T, int LOGN>
+cudaError_t launch_les_z(const CUtensorMap& fmap, const StageArgs<T>& st, const Geom& g, const C2<T>* tw, int* err,
+                         cudaStream_t s) {
+  using Z = LesZCfg<T, LOGN>;
+  auto k = les_zfwd_kernel<T, LOGN, -1>;
+  static cudaError_t attr = smem_attr(k, Z::SMEM);
+  if (attr != cudaSuccess) return attr;
+  dim3 grid((g.nxh + Z::P - 1) / Z::P, g.ny);
+  k<<<grid, Z::NT, Z::SMEM, s>>>(fmap, st, g, tw, err);
   return cudaGetLastError();
 }
 
@@ -366,6 +396,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
   case L:                                                                                        \
     return mode == sc::XW_ADJ      ? sc::launch_xgroup<T, L, sc::XW_ADJ>(fin, fout, g, twM, twN, xa, s)  \
            : mode == sc::XW_SCALAR ? sc::launch_xgroup<T, L, sc::XW_SCALAR>(fin, fout, g, twM, twN, xa, s) \
+           : mode == sc::XW_GRAD   ? sc::launch_xgroup<T, L, sc::XW_GRAD>(fin, fout, g, twM, twN, xa, s) \
            : mode == sc::XW_SMAG ? sc::launch_xgroup<T, L, sc::XW_SMAG>(fin, fout, g, twM, twN, xa, s) \
                                  : sc::launch_xgroup<T, L, sc::XW_DNS>(fin, fout, g, twM, twN, xa, s);
 
@@ -376,8 +407,34 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
   case L:                                                                                        \
     return mode == sc::XW_ADJ      ? sc::launch_xwarp<T, L, sc::XW_ADJ>(fin, fout, g, twM, twN, xa, s)  \
            : mode == sc::XW_SCALAR ? sc::launch_xwarp<T, L, sc::XW_SCALAR>(fin, fout, g, twM, twN, xa, s) \
+           : mode == sc::XW_GRAD   ? sc::launch_xwarp<T, L, sc::XW_GRAD>(fin, fout, g, twM, twN, xa, s) \
            : mode == sc::XW_SMAG ? sc::launch_xwarp<T, L, sc::XW_SMAG>(fin, fout, g, twM, twN, xa, s) \
                                  : sc::launch_xwarp<T, L, sc::XW_DNS>(fin, fout, g, twM, twN, xa, s);
+
+#define SC_LESY_CASE(L) case L: return sc::launch_les_y<LES_T, L>(inv, map, tp, g, tw, nsm, s);
+#define SC_LESZ_CASE(L) case L: return sc::launch_les_z<LES_T, L>(fmap, st, g, tw, err, s);
+#define SC_LESZT_CASE(L) case L: return sc::LesZCfg<LES_T, L>::P;
+#define SC_DEFINE_LES(T)                                                                         \
+  template <> int sc::Launch<T>::les_ztile(int logn) {                                           \
+    switch (logn) { SC_LOGN_CASES(SC_LESZT_CASE) default: return 0; }                            \
+  }                                                                                              \
+  template <>                                                                                    \
+  cudaError_t sc::Launch<T>::les_y(int logn, bool inv, const CUtensorMap& map,                   \
+                                   const TmaPass<T>& tp, const Geom& g, const C2<T>* tw,         \
+                                   int nsm, cudaStream_t s) {                                    \
+    switch (logn) {                                                                              \
+      SC_LOGN_CASES(SC_LESY_CASE)                                                                \
+      default: return cudaErrorInvalidValue;                                                     \
+    }                                                                                            \
+  }                                                                                              \
+  template <>                                                                                    \
+  cudaError_t sc::Launch<T>::les_z(int logn, const CUtensorMap& fmap, const StageArgs<T>& st,    \
+                                   const Geom& g, const C2<T>* tw, int* err, cudaStream_t s) {   \
+    switch (logn) {                                                                              \
+      SC_LOGN_CASES(SC_LESZ_CASE)                                                                \
+      default: return cudaErrorInvalidValue;                                                     \
+    }                                                                                            \
+  }
 
 #define SC_TMA_TILE_CASE(L) case L: return sc::TmaCfg<TMA_T, L>::P;
 #define SC_TMA_ZTILE_CASE(L) case L: return sc::TmaCfg<TMA_T, L>::PZ;
@@ -623,12 +680,14 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
   case L: return sc::launch_zfwd_zinv<double, L>(lmap, fmap, st, fa, g, tw, err, s);
 #define SC_ZINV5_CASE_float(L)                                                                     \
   case L:                                                                                          \
-    return mode == sc::ZV_SMAG ? sc::launch_zinv5<float, L, sc::ZV_SMAG>(vmap, umap, za, out, g, tw, err, s) \
-                               : sc::launch_zinv5<float, L, sc::ZV_DNS>(vmap, umap, za, out, g, tw, err, s);
+    return mode == sc::ZV_SMAG   ? sc::launch_zinv5<float, L, sc::ZV_SMAG>(vmap, umap, za, out, g, tw, err, s) \
+           : mode == sc::ZV_GRAD ? sc::launch_zinv5<float, L, sc::ZV_GRAD>(vmap, umap, za, out, g, tw, err, s) \
+                                 : sc::launch_zinv5<float, L, sc::ZV_DNS>(vmap, umap, za, out, g, tw, err, s);
 #define SC_ZINV5_CASE_double(L)                                                                    \
   case L:                                                                                          \
-    return mode == sc::ZV_SMAG ? sc::launch_zinv5<double, L, sc::ZV_SMAG>(vmap, umap, za, out, g, tw, err, s) \
-                               : sc::launch_zinv5<double, L, sc::ZV_DNS>(vmap, umap, za, out, g, tw, err, s);
+    return mode == sc::ZV_SMAG   ? sc::launch_zinv5<double, L, sc::ZV_SMAG>(vmap, umap, za, out, g, tw, err, s) \
+           : mode == sc::ZV_GRAD ? sc::launch_zinv5<double, L, sc::ZV_GRAD>(vmap, umap, za, out, g, tw, err, s) \
+                                 : sc::launch_zinv5<double, L, sc::ZV_DNS>(vmap, umap, za, out, g, tw, err, s);
 #define SC_ZPHI_CASE_float(L) case L: return sc::launch_zinv_phi<float, L>(lmap, omap, za, out, g, tw, err, s);
 #define SC_ZPHI_CASE_double(L) case L: return sc::launch_zinv_phi<double, L>(lmap, omap, za, out, g, tw, err, s);
 #define SC_ZI_P_CASE_float(L) case L: return sc::ZiCfg<float, L>::P;

@@ -358,6 +358,41 @@ struct FFTEngine {
     last_stage<INV>(out, sm, tw);
   }
 
+  // The transform of i k(n) x from the tile src (kept), k(n) the signed
+  // wavenumber of point n, through the tile sm; output in registers.  Ends with
+  // a barrier.
+  template <bool INV>
+  __device__ static void run_deriv(C (&out)[JL][RL], const C* src, C* sm, const C* __restrict__ tw) {
+    auto load = [&](C (&v)[R1], int j, int p) {
+#pragma unroll
+      for (int r = 0; r < R1; ++r) {
+        const int n = j + r * (N / R1);
+        v[r] = cmuli(cscale(src[sidx(n) * PS + p], (T)wavenum(n, N)));
+      }
+    };
+#pragma unroll
+    for (int a = 0; a < J1; ++a) {
+      int job = threadIdx.x + a * NT, p, j;
+      decode<R1>(job, p, j);
+      if ((TOT1 % NT == 0) || job < TOT1) {
+        if constexpr (NS == 1) {
+          load(out[a], j, p);
+          dft<R1, INV>(out[a]);
+        } else {
+          C v[R1];
+          load(v, j, p);
+          dft<R1, INV>(v);
+          store_stage0<R1>(v, sm, j, p);
+        }
+      }
+    }
+    __syncthreads();
+    if constexpr (NS > 1) {
+      mid_stages<1, INV>(sm, tw);
+      last_stage<INV>(out, sm, tw);
+    }
+  }
+
   // N = 512 with 32 threads per pencil (NT = 32 P, 16 points each): two
   // passes, 512 = 16 x 32, instead of three radix-8 stages.  Thread (p, j),
   // p = t % P, j = t / P:

@@ -78,6 +78,12 @@ template <> struct ZiFields<ZV_SMAG> {
   __device__ static constexpr int kz_field(int q) { return q < 2 ? 3 + q : (q == 2 ? 8 : (q == 3 ? 10 : 11)); }
   __device__ static constexpr int pw_field(int q) { return q == 0 ? 5 : (q == 1 ? 6 : (q == 2 ? 7 : 9)); }
 };
+// The LES operands' gradient form: u and d/dz u (all three carry kz).
+template <> struct ZiFields<ZV_GRAD> {
+  static constexpr int NKZ = 3, NPW = 0;
+  __device__ static constexpr int kz_field(int q) { return 3 + q; }
+  __device__ static constexpr int pw_field(int) { return 0; }
+};
 // pointwise output f (5: w_z, 6: S11, 7: S12, 9: S22) from u at (kx, ky)
 template <typename C, typename R> __device__ __forceinline__ C zi_pointwise(int f, C ux, C uy, R kx, R ky) {
   switch (f) {
@@ -118,21 +124,25 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
   // tile, u_x and u_y leave; their tiles are then the exchange buffers that
   // finish w_x and w_y, which leave by bulk stores as well.  No half tiles,
   // no work buffer, no element stores (SC_NO_TMEM_W: the half-tile path).
-  if constexpr (MODE == ZV_DNS && EF::TWO_PASS && sizeof(T) == 4) {
+  // ZV_GRAD: the same with the three d/dz u parked; u leaves, d/dz u follows.
+  if constexpr ((MODE == ZV_DNS || MODE == ZV_GRAD) && EF::TWO_PASS && sizeof(T) == 4) {
     if (umap) {
       using Cfg = TmaCfg<T, LOGN>;
+      constexpr int NQ = MODE == ZV_GRAD ? 3 : 2;            // fields parked, 32 columns each
+      constexpr int COLS = MODE == ZV_GRAD ? 256 : 128;      // per CTA: two warps per lane quarter
       __shared__ uint32_t s_tmem;
       const int t = threadIdx.x, warp = t >> 5;
       const int p = t % P, j = t / P;
-      if (warp == 0) tmem_alloc(&s_tmem, 128);
+      if (warp == 0) tmem_alloc(&s_tmem, COLS);
       tmem_fence_before_sync();
       __syncthreads();
       tmem_fence_after_sync();
-      // lanes 32 (warp % 4) .., columns 64 (warp / 4) .. + 63: w_x at +0, w_y at +32
-      const uint32_t tw_addr = s_tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64u * (uint32_t)(warp >> 2);
+      // lanes 32 (warp % 4) .., columns COLS / 2 (warp / 4) ..: field q at + 32 q
+      const uint32_t tw_addr =
+          s_tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(COLS / 2) * (uint32_t)(warp >> 2);
       const T kx = (T)(kx0 + p);
 #pragma unroll 1
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < NQ; ++q) {
         C v[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
@@ -157,30 +167,39 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
       };
       fence_proxy_async();
       __syncthreads();
-      if (t == 0) {
-        store(2, 2);
-        tma_store_commit();
-        store(0, 0);
-        store(1, 1);
-        tma_store_commit();
-        tma_store_wait_read<1>();
+      if constexpr (MODE == ZV_GRAD) {
+        if (t == 0) {
+          for (int c = 0; c < 3; ++c) store(c, c);
+          tma_store_commit();
+          tma_store_wait_read<0>();
+        }
+        __syncthreads();
+      } else {
+        if (t == 0) {
+          store(2, 2);
+          tma_store_commit();
+          store(0, 0);
+          store(1, 1);
+          tma_store_commit();
+          tma_store_wait_read<1>();
+        }
+        __syncthreads();
+        for (int e = t; e < P * N; e += NT) {
+          const int pe = e % P;
+          const C ux = rt[0][e], uy = rt[1][e];
+          rt[2][e] = cmuli(csub(cscale(uy, (T)(kx0 + pe)), cscale(ux, ky)));
+        }
+        fence_proxy_async();
+        __syncthreads();
+        if (t == 0) {
+          store(2, 5);
+          tma_store_commit();
+          tma_store_wait_read<1>();   // u_x and u_y have left their tiles
+        }
+        __syncthreads();
       }
-      __syncthreads();
-      for (int e = t; e < P * N; e += NT) {
-        const int pe = e % P;
-        const C ux = rt[0][e], uy = rt[1][e];
-        rt[2][e] = cmuli(csub(cscale(uy, (T)(kx0 + pe)), cscale(ux, ky)));
-      }
-      fence_proxy_async();
-      __syncthreads();
-      if (t == 0) {
-        store(2, 5);
-        tma_store_commit();
-        tma_store_wait_read<1>();   // u_x and u_y have left their tiles
-      }
-      __syncthreads();
 #pragma unroll 1
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < NQ; ++q) {
         uint32_t r[32];
         tmem_load32(tw_addr + 32u * q, r);
         C v[16];
@@ -193,14 +212,13 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
       __syncthreads();
       tmem_fence_after_sync();
       if (t == 0) {
-        store(0, 3);
-        store(1, 4);
+        for (int q = 0; q < NQ; ++q) store(q, 3 + q);
         tma_store_commit();
         tma_store_wait_read<0>();
       }
       if (warp == 0) {
         __syncwarp();   // the warp-collective release after thread 0's stores
-        tmem_dealloc(s_tmem, 128);
+        tmem_dealloc(s_tmem, COLS);
       }
       __syncthreads();
       return;
@@ -313,7 +331,7 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
   __syncthreads();
 }
 
-// Standalone z-inverse (MODE ZV_DNS, or ZV_SMAG for the LES operands): the
+// Standalone z-inverse (MODE ZV_DNS, or ZV_GRAD / ZV_SMAG for the LES operands): the
 // stage input tile by TMA, K_f partial sums, then zinv_from_tiles.
 // grid = (kx tiles, ny).
 template <typename T, int LOGN, int MODE>

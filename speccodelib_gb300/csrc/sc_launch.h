@@ -108,6 +108,14 @@ template <typename T> struct Launch {
   // forcing, symmetrize and mask, into the field of omap (tiles tma_tile wide)
   static cudaError_t zfwd_div_tma(int logn, const CUtensorMap& fmap, const CUtensorMap& omap, const DivArgs<T>& da,
                                   const Geom& g, const C2<T>* tw, int* err, cudaStream_t s);
+  // LES right-hand side in gradient form (sc_les.cuh): the y passes over the
+  // work fields of `map` (tiles tma_tile wide) and the z-forward of its eight
+  // fields (fmap, tiles les_ztile wide) with the spectral update
+  static int les_ztile(int logn);
+  static cudaError_t les_y(int logn, bool inverse, const CUtensorMap& map, const TmaPass<T>& tp, const Geom& g,
+                           const C2<T>* tw, int nsm, cudaStream_t s);
+  static cudaError_t les_z(int logn, const CUtensorMap& fmap, const StageArgs<T>& st, const Geom& g, const C2<T>* tw,
+                           int* err, cudaStream_t s);
   // z-forward of nin fields (9: the LES Lamb vector and tau_ij) through a
   // TMA ring, fmap tiled tma_tile wide; cudaErrorNotSupported otherwise
   static cudaError_t zfwd_fields_tma(int logn, int nin, const CUtensorMap& fmap, const StageArgs<T>& st,

@@ -123,7 +123,7 @@ pencil_plain_kernel(FieldList<T> fl, PlainArgs<T> pa, Geom g, const C2<T>* __res
 // ---------------------------------------------------------------------------
 // zinv: z-axis inverse pass generating the physical-space operands from v^
 // ---------------------------------------------------------------------------
-enum ZvMode { ZV_DNS = 0, ZV_SMAG = 1, ZV_DYN = 2, ZV_ADJ = 3 };
+enum ZvMode { ZV_DNS = 0, ZV_SMAG = 1, ZV_DYN = 2, ZV_ADJ = 3, ZV_GRAD = 4 };
 template <int MODE> struct ZvOut;
 template <> struct ZvOut<ZV_DNS> { static constexpr int n = 6; };
 template <> struct ZvOut<ZV_SMAG> { static constexpr int n = 12; };
@@ -179,10 +179,15 @@ __device__ __forceinline__ void adj_mu(C* m, int ix, int iy, int iz, const Geom&
 //   ZV_DNS : v (3), w = i k x v (3)                      dns-deform.f90:265-273
 //   ZV_SMAG: + S_ij, order 11 12 13 22 23 33             smag.f90:21-32
 //   ZV_DYN : u (3), g u (3), S_ij (6), g S_ij (6)        dynsmag.f90:29-34,80-93
+//   ZV_GRAD: v (3), d/dz v = i kz v (3)
 template <int MODE, typename C, typename R>
 __device__ __forceinline__ C zv_gen(int f, C v0, C v1, C v2, R kx, R ky, R kz, bool gin) {
   const R half = R(0.5);
   const C v[3] = {v0, v1, v2};
+  if (MODE == ZV_GRAD) {
+    const C x = f % 3 == 0 ? v0 : (f % 3 == 1 ? v1 : v2);
+    return f < 3 ? x : cmuli(cscale(x, kz));
+  }
   int q = f;
   if (MODE == ZV_DYN) {
     // fields: u (0-2), g u (3-5), S (6-11), g S (12-17)
@@ -735,7 +740,7 @@ __global__ void fixup_kx0_kernel(StageArgs<T> st, Geom g) {
 // ---------------------------------------------------------------------------
 enum XpMode { XP_DNS = 0, XP_SMAG = 1, XP_C2R3 = 2, XP_R2C3 = 3, XP_ADJ = 4, XP_SCALAR = 5 };
 // modes of the warp-per-row and lane-group x-passes (sc_xwarp.cuh, sc_xgroup.cuh)
-enum XwMode { XW_DNS = 0, XW_ADJ = 1, XW_SMAG = 2, XW_SCALAR = 3 };
+enum XwMode { XW_DNS = 0, XW_ADJ = 1, XW_SMAG = 2, XW_SCALAR = 3, XW_GRAD = 4 };
 template <int MODE> struct XpIO;
 template <> struct XpIO<XP_DNS> { static constexpr int fin = 6, fout = 3; };
 template <> struct XpIO<XP_SMAG> { static constexpr int fin = 12, fout = 9; };

@@ -309,15 +309,8 @@ template <typename T> struct Impl {
   static double kcut2(sc_handle* h) { return h->p.kcut * h->p.kcut; }
   static int pencil_tile(int logz) { return (sizeof(T) == 4 && logz < 9) ? 16 : 8; }
 
-  // ---- TMA-fed plain strided pass over nf equally spaced fields ----
-  // (src: the fields it reads, when they are not the ones it writes)
-  static int plain_tma(sc_handle* h, const char* name, int axis, bool inv, C* base, int nf, const C* src = nullptr) {
+  static sc::TmaPass<T> tma_pass(sc_handle* h, int axis, C* base, int nf, int P) {
     auto* g = &h->g;
-    const int logn = axis == 1 ? h->logy : h->logz;
-    const int N = axis == 1 ? g->ny : g->nz;
-    const int P = L::tma_tile(logn);
-    CUtensorMap map;
-    SC_TRY(encode_fields(h, src ? src : base, nf, axis, P, N, &map));
     sc::TmaPass<T> tp{};
     tp.base = base;
     tp.field = g->field;
@@ -328,6 +321,19 @@ template <typename T> struct Impl {
     tp.ntx = (g->nxh + P - 1) / P;
     tp.nf = nf;
     tp.err = h->derr;
+    return tp;
+  }
+
+  // ---- TMA-fed plain strided pass over nf equally spaced fields ----
+  // (src: the fields it reads, when they are not the ones it writes)
+  static int plain_tma(sc_handle* h, const char* name, int axis, bool inv, C* base, int nf, const C* src = nullptr) {
+    auto* g = &h->g;
+    const int logn = axis == 1 ? h->logy : h->logz;
+    const int N = axis == 1 ? g->ny : g->nz;
+    const int P = L::tma_tile(logn);
+    CUtensorMap map;
+    SC_TRY(encode_fields(h, src ? src : base, nf, axis, P, N, &map));
+    const sc::TmaPass<T> tp = tma_pass(h, axis, base, nf, P);
     return launch(h, name, [&] { return L::plain_tma(logn, inv, map, tp, *g, tw(h, N), h->nsm, h->stream); });
   }
   // x-pass of the DNS right-hand side: the warp-per-row kernel where it has
@@ -354,6 +360,15 @@ template <typename T> struct Impl {
     return kt * kt;
   }
 
+  // the K_f partial sums come from a z-inverse with tiles pt wide
+  static void set_kf_tiles(sc_handle* h, sc::StageArgs<T>& st, int pt) {
+    int nt = 0;
+    const int ntiles = (h->g.nxh + pt - 1) / pt;
+    while (nt < ntiles && (double)(nt * pt) * (nt * pt) < h->p.fkmax * h->p.fkmax) ++nt;
+    st.kf_tiles = nt;
+    st.kf_ptile = pt;
+  }
+
   static sc::StageArgs<T> stage_args(sc_handle* h) {
     sc::StageArgs<T> st{};
     for (int c = 0; c < 3; ++c) {
@@ -377,11 +392,7 @@ template <typename T> struct Impl {
     const int pt = use_zinv5(h) ? L::zinv5_tile(h->logz)
                    : (h->tma && h->tma_zinv && h->p.sgs == SC_SGS_NONE) ? L::tma_ztile(h->logz)
                                                                         : pencil_tile(h->logz);
-    int nt = 0;
-    const int ntiles = (h->g.nxh + pt - 1) / pt;
-    while (nt < ntiles && (double)(nt * pt) * (nt * pt) < h->p.fkmax * h->p.fkmax) ++nt;
-    st.kf_tiles = nt;
-    st.kf_ptile = pt;
+    set_kf_tiles(h, st, pt);
     st.kcut2 = kcut2(h);
     st.mask_rhs = h->p.mask_mode == SC_MASK_RHS_AND_STEP;
     st.symmetrize = 1;
@@ -621,6 +632,24 @@ template <typename T> struct Impl {
       if (vstore) SC_TRY(encode_fields(h, st.vout[0], 3, 2, P, g->nz, &vmap_out));
       // symmetrize included, its kx = 0 copy exchanged inside the kernel
       return launch(h, "zfwd", [&] { return L::zfwd_tma(h->logz, lmap, vmap_out, vstore ? 1 : 0, st, *g, tw(h, g->nz), h->derr, h->stream); });
+    } else if (les && h->tma && h->zinv5 && h->xwarp && sin_spaced && L::zinv5_supported(h->logz) && h->logx >= 5 &&
+               h->logx <= 9) {
+      // gradient form (sc_les.cuh): the row lengths that the warp and
+      // lane-group x-passes have
+      const int P5 = L::zinv5_tile(h->logz), PY = L::tma_tile(h->logy);
+      CUtensorMap vmap, umap, ymap, fmap;
+      SC_TRY(encode_fields(h, sin[0], 3, 2, P5, g->nz, &vmap));
+      SC_TRY(encode_fields(h, wl.f[0], 6, 2, P5, g->nz, &umap));
+      SC_TRY(encode_fields(h, wl.f[0], 8, 1, PY, g->ny, &ymap));
+      SC_TRY(encode_fields(h, wl.f[0], 8, 2, L::les_ztile(h->logz), g->nz, &fmap));
+      set_kf_tiles(h, st, P5);
+      sc::ZvArgs<T> zu = za;
+      zu.ustore = 1;
+      SC_TRY(launch(h, "zinv", [&] { return L::zinv5_tma(h->logz, vmap, umap, zu, wl, *g, tw(h, g->nz), h->derr, h->stream, sc::ZV_GRAD); }));
+      SC_TRY(launch(h, "ypass_inv", [&] { return L::les_y(h->logy, true, ymap, tma_pass(h, 1, wl.f[0], 6, PY), *g, tw(h, g->ny), h->nsm, h->stream); }));
+      SC_TRY(launch(h, "xpass", [&] { return L::xpass_warp(h->logx - 1, sc::XW_GRAD, wl, wl, *g, tw(h, g->nx / 2), tw(h, g->nx), xargs(h), h->stream); }));
+      SC_TRY(launch(h, "ypass_fwd", [&] { return L::les_y(h->logy, false, ymap, tma_pass(h, 1, wl.f[0], 8, PY), *g, tw(h, g->ny), h->nsm, h->stream); }));
+      return launch(h, "zfwd", [&] { return L::les_z(h->logz, fmap, st, *g, tw(h, g->nz), h->derr, h->stream); });
     } else {
       if (les && h->tma && h->zinv5 && sin_spaced && L::zinv5_supported(h->logz)) {
         // LES operands u, w, S_ij: TMA-fed, eight transforms (not 12), u by bulk stores

@@ -321,6 +321,66 @@ zfwd_fields_tma_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st
   zfwd_finish<E, T>(w, st, g, kx0, iy, nvalid, base, zstride, s_coef);
 }
 
+// The z-forward's spectral update of tile (kx0, iy) from the transformed
+// right-hand side in the tiles w (element (p, n) at n P + p; forcing and
+// symmetrize's copy of the kx = 0 column already in them when `paired`), in
+// batches of EB points per thread: all state loads of a batch are issued
+// before any of them is used.  fblock: the tile meets the forcing band, whose
+// coefficient is coef.  tstore (RK stage 4): the new state goes back into the
+// tiles.
+template <typename T, int P, int N, int NT, int EB, int MODE>
+__device__ __forceinline__ void zfwd_update(C2<T>* const w[3], const StageArgs<T>& st, const Geom& g, int kx0, int iy,
+                                            int nvalid, long long base, long long zstride, bool fblock, double coef,
+                                            int flo_b, int fk_b, bool paired, bool tstore) {
+  using C = C2<T>;
+  const int kyi = wavenum(iy, g.ny), kc_b = k2_lt(st.kcut2);
+  for (int e0 = threadIdx.x; e0 < P * N; e0 += NT * EB) {
+    C wv[EB][3], vv[EB][3], av[EB][3];
+    bool act[EB];
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      const int e = e0 + i * NT;
+      const int p = e % P, iz = e / P;
+      act[i] = e < P * N && p < nvalid;
+      if (!act[i]) continue;
+      const long long idx = base + iz * zstride + p;
+      load_state<T, MODE>(st, idx, vv[i], av[i]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) wv[i][c] = w[c][e];
+    }
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      if (!act[i]) continue;
+      const int e = e0 + i * NT;
+      const int p = e % P, iz = e / P;
+      const int ix = kx0 + p;
+      const long long idx = base + iz * zstride + p;
+      C* wp = wv[i];
+      if (fblock && !(paired && ix == 0)) {
+        const int kz = wavenum(iz, g.nz);
+        const int k2 = ix * ix + kyi * kyi + kz * kz;
+        if (k2 < fk_b && k2 >= flo_b) {
+          const T ac = (T)coef;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) wp[c] = cadd(wp[c], cscale(st.sin[c][idx], ac));
+        }
+      }
+      if (st.symmetrize) {
+        if (iy == g.ny / 2 || iz == g.nz / 2 || ix == g.nxh - 1 || (ix == 0 && iy == 0 && iz == 0))
+          wp[0] = wp[1] = wp[2] = czero<C>();
+      }
+      if (tstore) {
+        C vn[3];
+        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, vv[i], av[i], vn);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) w[c][e] = vn[c];
+      } else {
+        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, vv[i], av[i]);
+      }
+    }
+  }
+}
+
 // z-forward pass of the Lamb vector + the spectral update (DNS).  MODE: the
 // update mode as a compile-time constant (-1: st.mode at run time).  With
 // MODE == SM_RK4 and vstore, the new state goes back into the tiles and
@@ -375,7 +435,7 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
     }
   }
   const bool fblock = st.forced && ((double)kx0 * kx0 + (double)ky * ky < st.fkmax2);
-  const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(st.fkmax2), kc_b = k2_lt(st.kcut2);
+  const int fk_b = k2_lt(st.fkmax2);
   // lower edge of the forcing band (0 for force.f90's k2 < fkmax^2)
   const int flo_b = k2_lt(st.fband_lo2);
   if (fblock && threadIdx.x == 0) {
@@ -397,55 +457,10 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
     hermitian_column<T, P, N, NT>(w, st, g, iy, base, zstride, fblock, fblock ? s_coef : 0.0, flo_b, fk_b);
     if (!ok) return;
   }
-  // Epilogue in batches of EB points per thread: all state loads of a batch
-  // are issued before any of them is used.
   constexpr int EB = NT >= 512 ? 2 : 4;
   const bool tstore = MODE == SM_RK4 && vstore;
-  for (int e0 = threadIdx.x; e0 < P * N; e0 += NT * EB) {
-    C wv[EB][3], vv[EB][3], av[EB][3];
-    bool act[EB];
-#pragma unroll
-    for (int i = 0; i < EB; ++i) {
-      const int e = e0 + i * NT;
-      const int p = e % P, iz = e / P;
-      act[i] = e < P * N && p < nvalid;
-      if (!act[i]) continue;
-      const long long idx = base + iz * zstride + p;
-      load_state<T, MODE>(st, idx, vv[i], av[i]);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) wv[i][c] = w[c][e];
-    }
-#pragma unroll
-    for (int i = 0; i < EB; ++i) {
-      if (!act[i]) continue;
-      const int e = e0 + i * NT;
-      const int p = e % P, iz = e / P;
-      const int ix = kx0 + p;
-      const long long idx = base + iz * zstride + p;
-      C* wp = wv[i];
-      if (fblock && !(paired && ix == 0)) {
-        const int kz = wavenum(iz, g.nz);
-        const int k2 = ix * ix + kyi * kyi + kz * kz;
-        if (k2 < fk_b && k2 >= flo_b) {
-          const T ac = (T)s_coef;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) wp[c] = cadd(wp[c], cscale(st.sin[c][idx], ac));
-        }
-      }
-      if (st.symmetrize) {
-        if (iy == g.ny / 2 || iz == g.nz / 2 || ix == g.nxh - 1 || (ix == 0 && iy == 0 && iz == 0))
-          wp[0] = wp[1] = wp[2] = czero<C>();
-      }
-      if (tstore) {
-        C vn[3];
-        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, vv[i], av[i], vn);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) w[c][e] = vn[c];
-      } else {
-        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, vv[i], av[i]);
-      }
-    }
-  }
+  zfwd_update<T, P, N, NT, EB, MODE>(w, st, g, kx0, iy, nvalid, base, zstride, fblock, fblock ? s_coef : 0.0, flo_b,
+                                     fk_b, paired, tstore);
   if (tstore) {
     fence_proxy_async();
     __syncthreads();

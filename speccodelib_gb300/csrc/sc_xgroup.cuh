@@ -106,13 +106,18 @@ template <typename T, int LOGM> struct XgRow {
   // Z of the half-length c2r in natural order.  A lane forms the pairs
   // (k, M - k) of its first E/2 points; Z_{M-k} belongs to the mate lane's
   // register E-1-r (lane 0: to its own register E-r, and Z_{M/2} = 2 conj X).
-  __device__ __forceinline__ void load_z(const C* f, C (&x)[E]) const {
+  // DX: of the x derivative i k X instead.
+  template <bool DX = false> __device__ __forceinline__ void load_z(const C* f, C (&x)[E]) const {
     const C* rp = f + off;
+    auto at = [&](int k) {
+      const C v = rp[k];
+      return DX ? cmuli(cscale(v, (T)k)) : v;
+    };
     C zp[H];
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       const int k = l + L * r;
-      C xk = rp[k], xm = rp[M - k];
+      C xk = at(k), xm = at(M - k);
       if (r == 0 && l == 0) { xk.y = 0; xm.y = 0; }   // DC and Nyquist are real
       const C e = cadd(xk, cconj(xm));
       const C o = cmulc(csub(xk, cconj(xm)), __ldg(&twN[k]));
@@ -120,7 +125,7 @@ template <typename T, int LOGM> struct XgRow {
       zp[r] = mk<C>(e.x + o.y, o.x - e.y);     // conj(e) + i conj(o)
     }
     if (l == 0) {
-      const C h = rp[M / 2];
+      const C h = at(M / 2);
 #pragma unroll
       for (int r = 0; r < H - 1; ++r) zp[r] = zp[r + 1];
       zp[H - 1] = mk<C>(h.x + h.x, -(h.y + h.y));
@@ -128,31 +133,42 @@ template <typename T, int LOGM> struct XgRow {
 #pragma unroll
     for (int r = 0; r < H; ++r) x[E - 1 - r] = shfl(zp[r], mate);
   }
-  __device__ __forceinline__ void load_phys(const C* f, C (&x)[E]) const {
-    load_z(f, x);
+  template <bool DX = false> __device__ __forceinline__ void load_phys(const C* f, C (&x)[E]) const {
+    load_z<DX>(f, x);
     GF::template nat_to_scr<true>(x, buf, twM, l);
   }
 
-  // half-complex row c (e - i d)/... of natural-order Z: X_k = s/2 (e - i d),
-  // X_{M-k} = s/2 (conj e - i conj d) with e = Z_k + conj Z_{M-k},
-  // d = W_N^k (Z_k - conj Z_{M-k})
-  __device__ __forceinline__ void store_r2c(C (&x)[E], C* f, T s) const {
+  // The row's values from natural-order Z: X_k = s/2 (e - i d) in lo, X_{M-k} =
+  // s/2 (conj e - i conj d) in hi (k = l + L r, r < E/2), X_{M/2} in mid (lane
+  // 0), with e = Z_k + conj Z_{M-k}, d = W_N^k (Z_k - conj Z_{M-k})
+  __device__ __forceinline__ void r2c_vals(C (&x)[E], C (&lo)[H], C (&hi)[H], C& mid, T s) const {
     GF::template scr_to_nat<false>(x, buf, twM, l);
-    C* op = f + off;
     const T c = T(0.5) * s;
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       const C snd = l == 0 ? x[(E - r) % E] : x[E - 1 - r];
       const C zm = shfl(snd, mate), zk = x[r];
-      const int k = l + L * r;
       const C e = cadd(zk, cconj(zm));
-      const C d = cmul(csub(zk, cconj(zm)), cscale(__ldg(&twN[k]), c));
-      if (live) {
-        op[k] = mk<C>(c * e.x + d.y, c * e.y - d.x);
-        op[M - k] = mk<C>(c * e.x - d.y, -(c * e.y) - d.x);
-      }
+      const C d = cmul(csub(zk, cconj(zm)), cscale(__ldg(&twN[l + L * r]), c));
+      lo[r] = mk<C>(c * e.x + d.y, c * e.y - d.x);
+      hi[r] = mk<C>(c * e.x - d.y, -(c * e.y) - d.x);
     }
-    if (l == 0 && live) op[M / 2] = mk<C>(s * x[H].x, -(s * x[H].y));
+    mid = mk<C>(s * x[H].x, -(s * x[H].y));
+  }
+  __device__ __forceinline__ void store_vals(C* f, const C (&lo)[H], const C (&hi)[H], const C& mid) const {
+    if (!live) return;
+    C* op = f + off;
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      op[l + L * r] = lo[r];
+      op[M - l - L * r] = hi[r];
+    }
+    if (l == 0) op[M / 2] = mid;
+  }
+  __device__ __forceinline__ void store_r2c(C (&x)[E], C* f, T s) const {
+    C lo[H], hi[H], mid;
+    r2c_vals(x, lo, hi, mid, s);
+    store_vals(f, lo, hi, mid);
   }
 
   __device__ __forceinline__ void load_a(const C* const f[3]) const {
@@ -193,6 +209,81 @@ template <typename T, int LOGM> struct XgRow {
       x[i] = mk<C>(az.x * bx.x - ax.x * b[i].x, az.y * bx.y - ax.y * b[i].y);
     }
     store_r2c(x, of[1], sc);
+  }
+
+  // XW_GRAD: rows 0-2 = u_c, 3 + 3 j + c = d_j u_c kept, then the products as
+  // XwRow::les_store
+  __device__ __forceinline__ void les_rows(const C* const f[9], C* const of[8], T sc, T tcoef) const {
+    auto put = [&](int q, const C (&x)[E]) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) kept(q, i) = x[i];
+    };
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      C x[E];
+      load_phys(f[c], x);
+      put(c, x);
+      load_phys<true>(f[c], x);
+      put(3 + c, x);
+    }
+#pragma unroll 1
+    for (int q = 3; q < 9; ++q) {
+      C x[E];
+      load_phys(f[q], x);
+      put(3 + q, x);
+    }
+    auto S = [&](int p, int q, int i) {   // S_pq = (d_p u_q + d_q u_p) / 2
+      const C a = kept(3 + 3 * p + q, i), b = kept(3 + 3 * q + p, i);
+      return mk<C>(T(0.5) * (a.x + b.x), T(0.5) * (a.y + b.y));
+    };
+    C s[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const C s11 = kept(3, i), s22 = kept(7, i), s33 = kept(11, i), s12 = S(0, 1, i), s13 = S(0, 2, i), s23 = S(1, 2, i);
+      s[i].x = tcoef * sqrt(T(2) * (s11.x * s11.x + s22.x * s22.x + s33.x * s33.x +
+                                    T(2) * (s12.x * s12.x + s13.x * s13.x + s23.x * s23.x)));
+      s[i].y = tcoef * sqrt(T(2) * (s11.y * s11.y + s22.y * s22.y + s33.y * s33.y +
+                                    T(2) * (s12.y * s12.y + s13.y * s13.y + s23.y * s23.y)));
+    }
+    C lo[H], hi[H], mid;
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+      C x[E], tl[H], th[H], tm;
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const C t = S(0, c, i);
+        x[i] = mk<C>(s[i].x * t.x, s[i].y * t.y);
+      }
+      r2c_vals(x, tl, th, tm, T(1));
+      if (c > 0) store_vals(of[c == 1 ? 3 : 6], tl, th, tm);   // tau_12, tau_13
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const C u1 = kept(c1, i), u2 = kept(c2, i);
+        const C a = kept(3 + 3 * c + c1, i), b = kept(3 + 3 * c1 + c, i);
+        const C d = kept(3 + 3 * c2 + c, i), e = kept(3 + 3 * c + c2, i);
+        x[i] = mk<C>(u1.x * (a.x - b.x) - u2.x * (d.x - e.x), u1.y * (a.y - b.y) - u2.y * (d.y - e.y));
+      }
+      r2c_vals(x, lo, hi, mid, sc);
+#pragma unroll
+      for (int r = 0; r < H; ++r) {
+        const int k = l + L * r;
+        lo[r] = csub(lo[r], cmuli(cscale(tl[r], (T)k)));
+        hi[r] = csub(hi[r], cmuli(cscale(th[r], (T)(M - k))));
+      }
+      mid = csub(mid, cmuli(cscale(tm, (T)(M / 2))));
+      store_vals(of[c], lo, hi, mid);
+    }
+#pragma unroll 1
+    for (int q = 0; q < 3; ++q) {   // tau_22, tau_23, tau_33
+      C x[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const C t = S(q == 2 ? 2 : 1, q == 0 ? 1 : 2, i);
+        x[i] = mk<C>(s[i].x * t.x, s[i].y * t.y);
+      }
+      store_r2c(x, of[q == 2 ? 7 : 4 + q], T(1));
+    }
   }
 
   // of[c] = r2c(sc a_c phi) (convecphi_dns.f90:20-23)
@@ -245,7 +336,7 @@ template <typename T, int LOGM> struct XgRow {
 
 template <typename T, int LOGM, int MODE> struct XgCfg {
   using GF = GroupFFT<T, LOGM>;
-  static constexpr int KEPT = MODE == XW_SMAG ? 6 : 5;
+  static constexpr int KEPT = MODE == XW_GRAD ? 12 : (MODE == XW_SMAG ? 6 : 5);
   static constexpr int PER_WARP = GF::RW * (KEPT * GF::M + GF::BUF);
   // four warps, fewer where their kept rows pass the 227 KB of a CTA
   static constexpr int FIT = (int)(227 * 1024 / (sizeof(C2<T>) * PER_WARP));
@@ -295,6 +386,10 @@ xpass_group_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __r
       C* of[3] = {fout.f[3], fout.f[4], fout.f[5]};
       R.flux_store(fin.f[6], of, xa.scale);
     }
+  } else if constexpr (MODE == XW_GRAD) {
+    const C* f[9] = {u[0], u[1], u[2], fin.f[6], fin.f[7], fin.f[8], w[0], w[1], w[2]};
+    C* of[8] = {o[0], o[1], o[2], fout.f[3], fout.f[4], fout.f[5], fout.f[6], fout.f[7]};
+    R.les_rows(f, of, xa.scale, (T)(-2.0 * (*xa.c1) * xa.delta2) * xa.scale);
   } else if constexpr (MODE == XW_SMAG) {
     const C* s[6] = {fin.f[6], fin.f[7], fin.f[8], fin.f[9], fin.f[10], fin.f[11]};
     C* ot[6] = {fout.f[3], fout.f[4], fout.f[5], fout.f[6], fout.f[7], fout.f[8]};

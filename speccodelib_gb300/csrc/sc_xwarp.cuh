@@ -260,17 +260,18 @@ template <typename T, int LOGM> struct WarpFFT {
 template <typename T, int LOGM, int MODE = XW_DNS> struct XwCfg {
   // per warp: the transpose buffer + the rows kept in scrambled order (u;
   // XW_SMAG also S_ij)
-  static constexpr int KEPT = MODE == XW_SMAG ? 9 : 3;
+  static constexpr int KEPT = MODE == XW_SMAG ? 9 : (MODE == XW_GRAD ? 12 : 3);
   // TM: the kept rows in tensor memory instead (FP32; XW_DNS and XW_ADJ at
   // 4 or 8 points per lane, XW_SMAG at 4; SC_XW_NO_TMEM: shared memory):
   // 2 E KEPT columns per warp, two warps per lane quarter, TM_COLS columns
-  // per CTA (128, or 256 for the nine XW_SMAG rows)
+  // per CTA (128, or 256 for the nine XW_SMAG and twelve XW_GRAD rows; at 8
+  // points per lane the latter take 192 columns, so a CTA has four warps)
 #ifndef SC_XW_NO_TMEM
   static constexpr bool TM = sizeof(T) == 4 && (MODE != XW_SMAG ? (LOGM == 7 || LOGM == 8) : LOGM == 7);
 #else
   static constexpr bool TM = false;
 #endif
-  static constexpr int TM_COLS = MODE == XW_SMAG ? 256 : 128;
+  static constexpr int TM_COLS = MODE == XW_SMAG || MODE == XW_GRAD ? 256 : 128;
   static constexpr int KEPT_SM = TM ? 0 : KEPT;
   // two staging buffers for the warp's next input rows (points 0 .. M,
   // rounded up to 16 bytes)
@@ -286,7 +287,8 @@ template <typename T, int LOGM, int MODE = XW_DNS> struct XwCfg {
                     ((WarpFFT<T, LOGM>::SMEM + KEPT_SM * WarpFFT<T, LOGM>::M) * sizeof(C2<T>)) % 16 == 0,
                 "x-pass staging buffers must start on 16-byte boundaries");
   // 8 warps per CTA unless that passes 110 KB of shared memory
-  static constexpr int WARPS = sizeof(C2<T>) * PER_WARP * 8 <= 110 * 1024 ? 8 : 4;
+  static constexpr int WARPS =
+      sizeof(C2<T>) * PER_WARP * 8 <= 110 * 1024 && !(MODE == XW_GRAD && TM && LOGM == 8) ? 8 : 4;
   static constexpr int NT = 32 * WARPS;
   static_assert(!TM || WARPS == 8 || WARPS == 4, "two lane-quarter blocks of tensor-memory columns at most");
   // CTAs per SM the launch bounds ask for: three (80 registers) where the
@@ -404,6 +406,27 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
 #endif
   }
 
+  // Z of a row and of its x derivative i kx X, in one reading of the staged row
+  __device__ __forceinline__ void load_z2(const C* __restrict__ fp, C (&x)[E], C (&xd)[E]) {
+    const C* __restrict__ rp = stg ? stage_acquire() : fp + off;
+    C wn[E];
+    half_twiddles(wn);
+#pragma unroll
+    for (int r = 0; r < E; ++r) {
+      const int k = lane + 32 * r;
+      C xk = rp[k], xm = rp[M - k];
+      C dk = cmuli(cscale(xk, (T)k)), dm = cmuli(cscale(xm, (T)(M - k)));
+      if (k == 0) { xk.y = 0; xm.y = 0; dk.y = 0; dm.y = 0; }   // DC and Nyquist are real
+      C e = cadd(xk, cconj(xm));
+      C o = cmulc(csub(xk, cconj(xm)), wn[r]);
+      x[r] = cadd(e, cmuli(o));
+      e = cadd(dk, cconj(dm));
+      o = cmulc(csub(dk, cconj(dm)), wn[r]);
+      xd[r] = cadd(e, cmuli(o));
+    }
+    if (stg) stage_release();
+  }
+
   // half-length c2r pre-processing of a row into natural-order Z
   __device__ __forceinline__ void load_z(const C* __restrict__ fp, C (&x)[E]) {
     const C* __restrict__ rp = stg ? stage_acquire() : fp + off;
@@ -421,26 +444,50 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
     if (stg) stage_release();
   }
 
-  // a_c = c2r of rows f[0..2], kept in shared memory
+  // kept row c = c2r of natural-order Z (TM: tmem_wait_store before reading)
+  __device__ __forceinline__ void keep_row(int c, C (&x)[E]) {
+    WF::template nat_to_scr<true, TX>(x, sm, twM, lane, tx);
+    if constexpr (TM) {
+      uint32_t w[2 * E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        w[2 * i] = __float_as_uint(x[i].x);
+        w[2 * i + 1] = __float_as_uint(x[i].y);
+      }
+      if constexpr (E == 8) tmem_store16(ta + 16u * c, w);
+      else tmem_store8(ta + 8u * c, w);
+    } else {
+#pragma unroll
+      for (int i = 0; i < E; ++i) as[(c * E + i) * 32 + lane] = x[i];
+    }
+  }
+
+  // a_c = c2r of rows f[0..2], kept
   __device__ __forceinline__ void load_a(const C* const f[3]) {
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
       C x[E];
       load_z(f[c], x);
-      WF::template nat_to_scr<true, TX>(x, sm, twM, lane, tx);
-      if constexpr (TM) {
-        uint32_t w[2 * E];
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-          w[2 * i] = __float_as_uint(x[i].x);
-          w[2 * i + 1] = __float_as_uint(x[i].y);
-        }
-        if constexpr (E == 8) tmem_store16(ta + 16u * c, w);
-        else tmem_store8(ta + 8u * c, w);
-      } else {
-#pragma unroll
-        for (int i = 0; i < E; ++i) as[(c * E + i) * 32 + lane] = x[i];
-      }
+      keep_row(c, x);
+    }
+    if constexpr (TM) tmem_wait_store();
+  }
+
+  // The LES gradient rows: a_c = u_c (0-2) and d_j u_c (3 + 3 j + c), from the
+  // rows u (0-2), d/dy u (3-5), d/dz u (6-8) of f
+  __device__ __forceinline__ void load_grad(const C* const f[9]) {
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      C x[E], xd[E];
+      load_z2(f[c], x, xd);
+      keep_row(c, x);
+      keep_row(3 + c, xd);
+    }
+#pragma unroll 1
+    for (int q = 3; q < 9; ++q) {
+      C x[E];
+      load_z(f[q], x);
+      keep_row(3 + q, x);
     }
     if constexpr (TM) tmem_wait_store();
   }
@@ -458,12 +505,12 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
     }
   }
 
-  // r2c post-processing of natural-order Z into the half-complex row at op:
-  // needs Z_{M-k}; k = lane + 32 r pairs with lane (32 - lane) % 32,
-  // register E-1-r (lane 0: its own register (E - r) % E)
-  __device__ __forceinline__ void r2c_store(C (&x)[E], C* __restrict__ op) const {
+  // r2c post-processing of natural-order Z, in place (X_k, k = lane + 32 r; X_M
+  // valid in lane 0): needs Z_{M-k}; k = lane + 32 r pairs with lane
+  // (32 - lane) % 32, register E-1-r (lane 0: its own register (E - r) % E)
+  __device__ __forceinline__ void r2c_vals(C (&x)[E], C& xM) const {
     const int src = (32 - lane) & 31;
-    C wn[E];
+    C wn[E], o[E];
     half_twiddles(wn);
 #pragma unroll
     for (int r = 0; r < E; ++r) {
@@ -471,17 +518,26 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
       zm.x = __shfl_sync(0xffffffffu, x[E - 1 - r].x, src);
       zm.y = __shfl_sync(0xffffffffu, x[E - 1 - r].y, src);
       if (lane == 0) zm = x[(E - r) % E];
-      const int k = lane + 32 * r;
       const C zk = x[r];
       const C zmc = cconj(zm);
       const C e = cadd(zk, zmc);
       const C d = cmul(csub(zk, zmc), wn[r]);
-      op[k] = cscale(csub(e, cmuli(d)), T(0.5));
-      if (k == 0) {   // X_M from Z_0
+      o[r] = cscale(csub(e, cmuli(d)), T(0.5));
+      if (r == 0) {   // X_M from Z_0
         const C d0 = cmul(csub(zk, zmc), __ldg(&twN[M]));
-        op[M] = cscale(csub(e, cmuli(d0)), T(0.5));
+        xM = cscale(csub(e, cmuli(d0)), T(0.5));
       }
     }
+#pragma unroll
+    for (int r = 0; r < E; ++r) x[r] = o[r];
+  }
+  // ... and out to the half-complex row at op
+  __device__ __forceinline__ void r2c_store(C (&x)[E], C* __restrict__ op) const {
+    C xM;
+    r2c_vals(x, xM);
+#pragma unroll
+    for (int r = 0; r < E; ++r) op[lane + 32 * r] = x[r];
+    if (lane == 0) op[M] = xM;
   }
 
   // a_c at points i0 .. i0 + G - 1 (G = min(E, 4))
@@ -559,6 +615,99 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
     }
     out(l0, 0);
     out(l1, 1);
+  }
+
+  // The LES products from the kept gradient rows (smag.f90:41-64,
+  // convec_dns.f90:30-38): of[0..2] = (u x w)_i / N^3 - i kx tau_i1, of[3..7] =
+  // tau_12, tau_22, tau_23, tau_13, tau_33, with w = curl u, tau_ij = tcoef |S|
+  // S_ij.  Two real points per complex value, as everywhere in this pass.
+  __device__ __forceinline__ void les_store(C* const of[8], T sc, T tcoef) const {
+    constexpr int G = E < 4 ? E : 4;
+    auto grad = [&](int j, int c, int i0, C (&a)[4]) { a_group(3 + 3 * j + c, i0, a); };
+    C s[E];   // tcoef |S|
+#pragma unroll
+    for (int i0 = 0; i0 < E; i0 += G) {
+      C d[4], o[4];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        C a[4], b[4];
+        grad(j, j, i0, a);
+#pragma unroll
+        for (int i = 0; i < G; ++i)
+          d[i] = j == 0 ? mk<C>(a[i].x * a[i].x, a[i].y * a[i].y)
+                        : mk<C>(a[i].x * a[i].x + d[i].x, a[i].y * a[i].y + d[i].y);
+        const int p = j == 2 ? 1 : 0, q = j == 0 ? 1 : 2;   // (0,1), (0,2), (1,2)
+        grad(p, q, i0, a);
+        grad(q, p, i0, b);
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+          const C t = mk<C>(T(0.5) * (a[i].x + b[i].x), T(0.5) * (a[i].y + b[i].y));
+          o[i] = j == 0 ? mk<C>(t.x * t.x, t.y * t.y) : mk<C>(t.x * t.x + o[i].x, t.y * t.y + o[i].y);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < G; ++i)
+        s[i0 + i] = mk<C>(tcoef * sqrt(T(2) * (d[i].x + T(2) * o[i].x)), tcoef * sqrt(T(2) * (d[i].y + T(2) * o[i].y)));
+    }
+    // spectral row of tau_pq
+    auto tau = [&](int p, int q, C (&x)[E], C& xM) {
+#pragma unroll
+      for (int i0 = 0; i0 < E; i0 += G) {
+        C a[4], b[4];
+        grad(p, q, i0, a);
+        grad(q, p, i0, b);
+#pragma unroll
+        for (int i = 0; i < G; ++i)
+          x[i0 + i] = mk<C>(s[i0 + i].x * (T(0.5) * (a[i].x + b[i].x)), s[i0 + i].y * (T(0.5) * (a[i].y + b[i].y)));
+      }
+      WF::template scr_to_nat<false, TX>(x, sm, twM, lane, tx);
+      r2c_vals(x, xM);
+    };
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+      C l[E], lM, t[E], tM;
+#pragma unroll
+      for (int i0 = 0; i0 < E; i0 += G) {
+        // L_c = u_c1 w_c2 - u_c2 w_c1, w_c2 = d_c u_c1 - d_c1 u_c, w_c1 = d_c2 u_c - d_c u_c2
+        C u[4], a[4], b[4];
+        a_group(c1, i0, u);
+        grad(c, c1, i0, a);
+        grad(c1, c, i0, b);
+#pragma unroll
+        for (int i = 0; i < G; ++i) l[i0 + i] = mk<C>(u[i].x * (a[i].x - b[i].x), u[i].y * (a[i].y - b[i].y));
+        a_group(c2, i0, u);
+        grad(c2, c, i0, a);
+        grad(c, c2, i0, b);
+#pragma unroll
+        for (int i = 0; i < G; ++i)
+          l[i0 + i] = mk<C>((l[i0 + i].x - u[i].x * (a[i].x - b[i].x)) * sc, (l[i0 + i].y - u[i].y * (a[i].y - b[i].y)) * sc);
+      }
+      WF::template scr_to_nat<false, TX>(l, sm, twM, lane, tx);
+      r2c_vals(l, lM);
+      tau(0, c, t, tM);
+      C* op = of[c] + off;
+      C* ot = c == 1 ? of[3] + off : of[6] + off;   // tau_12, tau_13
+#pragma unroll
+      for (int r = 0; r < E; ++r) {
+        const int k = lane + 32 * r;
+        op[k] = csub(l[r], cmuli(cscale(t[r], (T)k)));
+        if (c > 0) ot[k] = t[r];
+      }
+      if (lane == 0) {
+        op[M] = csub(lM, cmuli(cscale(tM, (T)M)));
+        if (c > 0) ot[M] = tM;
+      }
+    }
+#pragma unroll 1
+    for (int q = 0; q < 3; ++q) {   // tau_22, tau_23, tau_33
+      C t[E], tM;
+      tau(q == 2 ? 2 : 1, q == 0 ? 1 : 2, t, tM);
+      C* ot = of[q == 2 ? 7 : 4 + q] + off;
+#pragma unroll
+      for (int r = 0; r < E; ++r) ot[lane + 32 * r] = t[r];
+      if (lane == 0) ot[M] = tM;
+    }
   }
 
   // of[c] = r2c(sc * a_c phi), phi = c2r of row pf (convecphi_dns.f90:20-23)
@@ -677,6 +826,8 @@ template <typename T, int LOGM, bool TM = false> struct XwRow {
 // XW_SMAG: fin = (u, w, S_ij) -> fout[0..2] = r2c(u x w / N^3) and
 //   fout[3..8] = r2c(tau_ij), tau_ij = -2 c1 D^2 |S| S_ij / N^3 (smag.f90:41-64),
 //   in place allowed: u and S are staged and w is read before any output.
+// XW_GRAD: fin = (u, d/dz u, d/dy u) -> the eight fields of les_store
+//   (sc_les.cuh), in place allowed: every row is kept before the first output.
 // XW_ADJ: fin = (u, w, phi) -> adjoint of the Lamb product (no scale):
 //   w x phi = -(phi x w) into fout[0..2], then phi x u into fout[3..5];
 //   fout must not alias u (read by the second product) -- the host passes
@@ -717,9 +868,13 @@ xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __re
     R.off = row * g.nxp;
     R.lane = lane;
     // the input fields in the order their rows are consumed
-    const C* seq[Cfg::KEPT == 9 ? 12 : (MODE == XW_ADJ ? 9 : (MODE == XW_SCALAR ? 7 : 6))];
+    const C* seq[MODE == XW_SMAG ? 12 : (MODE == XW_ADJ || MODE == XW_GRAD ? 9 : (MODE == XW_SCALAR ? 7 : 6))];
     if constexpr (MODE == XW_DNS || MODE == XW_SCALAR) {
       for (int f = 0; f < (MODE == XW_SCALAR ? 7 : 6); ++f) seq[f] = fin.f[f];
+    } else if constexpr (MODE == XW_GRAD) {
+      for (int f = 0; f < 3; ++f) seq[f] = fin.f[f];          // u
+      for (int f = 0; f < 3; ++f) seq[3 + f] = fin.f[6 + f];  // d/dy u
+      for (int f = 0; f < 3; ++f) seq[6 + f] = fin.f[3 + f];  // d/dz u
     } else if constexpr (MODE == XW_SMAG) {
       for (int f = 0; f < 3; ++f) seq[f] = fin.f[f];          // u (load_a)
       for (int f = 0; f < 6; ++f) seq[3 + f] = fin.f[6 + f];  // S_ij (load_s)
@@ -748,6 +903,11 @@ xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __re
         C* of[3] = {fout.f[3], fout.f[4], fout.f[5]};
         R.flux_store(fin.f[6], of, xa.scale);
       }
+    } else if constexpr (MODE == XW_GRAD) {
+      C* of[8] = {fout.f[0], fout.f[1], fout.f[2], fout.f[3], fout.f[4], fout.f[5], fout.f[6], fout.f[7]};
+      const T tcoef = (T)(-2.0 * (*xa.c1) * xa.delta2) * xa.scale;
+      R.load_grad(seq);
+      R.les_store(of, xa.scale, tcoef);
     } else if constexpr (MODE == XW_SMAG) {
       const C* a[3] = {fin.f[0], fin.f[1], fin.f[2]};
       const C* b[3] = {fin.f[3], fin.f[4], fin.f[5]};

@@ -166,3 +166,28 @@ def test_scalar_passes_shapes(specns_lib, shape, prec):
     v, phi, _, _ = R.ab2v_scalar_run(fd[:3], fd[3], g, (1e-3, 8e-4, 1.2e-3), 0.7, True, 0.4)
     assert rel_l2(var[:3], v) < TOL[prec]
     assert rel_l2(var[3], phi) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", [(32, 256, 8), (32, 8, 256), (64, 512, 16), (128, 16, 512), (32, 1024, 8),
+                                   (64, 8, 1024), (256, 64, 32), (512, 8, 64)])
+def test_les_passes(specns_lib, shape, prec):
+    """The y and z passes of the LES right-hand side at every tile shape, with
+    a forcing band several tiles wide, one RK4 step, and a right-hand side
+    without symmetrize (a variable-step pass)."""
+    nx, ny, nz = shape
+    kw = dict(nu=0.01, dt=1e-3, fkmax=6.2, eps=0.3, c1=0.03)
+    v = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 71, kcut=8.0)]
+    vd = [a.astype(np.complex128) for a in v]
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, sgs="smag", **kw))
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, sgs=S.SC_SGS_SMAG, **kw)) as h:
+        h.set_state(*v)
+        w = h.rhs()
+        h.rk4_steps(1)
+        out = h.get_state()
+        h.set_state(*v)
+        h.ab2v_pass(1e-3)
+        var = h.get_state()
+    assert rel_l2(w, R.ratesdudt(vd, g)) < TOL[prec]
+    assert rel_l2(out, R.rk4_run(vd, g, 1)) < TOL[prec]
+    assert rel_l2(var, R.ab2v_run(vd, g, (1e-3,))[0]) < TOL[prec]
