@@ -18,9 +18,15 @@
 // products are conjugates of each other, once instead of twice (12 operations
 // per pair, not 20); the final scale rides on fused multiply-adds.  About 225
 // operations per complex point of a Lamb product instead of 565.  At 128^3
-// FP64 a launch takes 448 us (the warp pass 940), near the pipe's 375.  In FP32
-// it serves the short rows (M = 16, 32) that leave a whole warp per row no
-// points to work on, in place of the block kernel (64^3 step 212 -> 201 us).
+// FP64 a launch takes 448 us (the warp pass 940), near the pipe's 375.
+//
+// In FP32 it serves rows of M = 16 to 64, where a whole warp per row has one
+// or two points per lane (block kernel at 16 and 32): Lamb product at 128^3
+// 34.9 -> 18.0 us, its adjoint 56 -> 29, the LES products 92 -> 58; 64^3 step
+// 212 -> 201.  At M = 128 both forms take the same time (181 us at 256^3; the
+// LES products 458 in the warp pass, 684 here) and at M = 256 the warp pass
+// with its staged rows is faster (1.20 ms at 512^3, 1.33 here): the line lies
+// between 64 and 128.
 #pragma once
 #include "sc_passes.cuh"
 #include "sc_xwarp.cuh"
@@ -83,12 +89,15 @@ template <typename T, int LOGM> struct GroupFFT {
 };
 
 // One lane's view of its group's row at element offset `off` of every field.
-template <typename T, int LOGM> struct XgRow {
+// KT: the first KT kept rows wait in tensor memory (FP32), the others in
+// shared memory; both are lane-private, read four points at a time.
+template <typename T, int LOGM, int KT = 0> struct XgRow {
   using GF = GroupFFT<T, LOGM>;
   using C = C2<T>;
   static constexpr int M = GF::M, E = GF::E, L = GF::L, H = GF::E / 2;
   C* buf;          // the group's transpose buffer
-  C* keep;         // kept rows in scrambled order, lane-private: row c at [(c E + i) 32 + lane]
+  C* keep;         // kept rows in scrambled order: row c >= KT at [((c - KT) E + i) 32 + lane]
+  uint32_t ta = 0; // row c < KT at columns ta + 2 E c .. of the warp's lanes
   const C* twM;
   const C* twN;
   long long off;
@@ -101,7 +110,40 @@ template <typename T, int LOGM> struct XgRow {
     r.y = __shfl_sync(0xffffffffu, v.y, src);
     return r;
   }
-  __device__ __forceinline__ C& kept(int c, int i) const { return keep[(c * E + i) * 32 + lane]; }
+  __device__ __forceinline__ void put(int c, const C (&x)[E]) const {
+    if (c < KT) {
+      if constexpr (KT > 0 && sizeof(T) == 4) {
+#pragma unroll
+        for (int i0 = 0; i0 < E; i0 += 8) {
+          uint32_t w[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            w[2 * i] = __float_as_uint(x[i0 + i].x);
+            w[2 * i + 1] = __float_as_uint(x[i0 + i].y);
+          }
+          tmem_store16(ta + (uint32_t)(2 * E * c + 2 * i0), w);
+        }
+        tmem_wait_store();
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < E; ++i) keep[((c - KT) * E + i) * 32 + lane] = x[i];
+    }
+  }
+  // row c at points i0 .. i0 + 3
+  __device__ __forceinline__ void get(int c, int i0, C (&a)[4]) const {
+    if (c < KT) {
+      if constexpr (KT > 0 && sizeof(T) == 4) {
+        uint32_t w[8];
+        tmem_load8(ta + (uint32_t)(2 * E * c + 2 * i0), w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = mk<C>(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = keep[((c - KT) * E + i0 + i) * 32 + lane];
+    }
+  }
 
   // Z of the half-length c2r in natural order.  A lane forms the pairs
   // (k, M - k) of its first E/2 points; Z_{M-k} belongs to the mate lane's
@@ -156,14 +198,16 @@ template <typename T, int LOGM> struct XgRow {
     mid = mk<C>(s * x[H].x, -(s * x[H].y));
   }
   __device__ __forceinline__ void store_vals(C* f, const C (&lo)[H], const C (&hi)[H], const C& mid) const {
-    if (!live) return;
     C* op = f + off;
+    if (live) {
 #pragma unroll
-    for (int r = 0; r < H; ++r) {
-      op[l + L * r] = lo[r];
-      op[M - l - L * r] = hi[r];
+      for (int r = 0; r < H; ++r) {
+        op[l + L * r] = lo[r];
+        op[M - l - L * r] = hi[r];
+      }
+      if (l == 0) op[M / 2] = mid;
     }
-    if (l == 0) op[M / 2] = mid;
+    __syncwarp();   // tensor-memory accesses are warp-collective
   }
   __device__ __forceinline__ void store_r2c(C (&x)[E], C* f, T s) const {
     C lo[H], hi[H], mid;
@@ -176,8 +220,7 @@ template <typename T, int LOGM> struct XgRow {
     for (int c = 0; c < 3; ++c) {
       C x[E];
       load_phys(f[c], x);
-#pragma unroll
-      for (int i = 0; i < E; ++i) kept(c, i) = x[i];
+      put(c, x);
     }
   }
 
@@ -186,38 +229,59 @@ template <typename T, int LOGM> struct XgRow {
   __device__ __forceinline__ void cross_store(const C* const bf[3], C* const of[3], T sc) const {
     C b[E], x[E];
     load_phys(bf[0], b);
-#pragma unroll
-    for (int i = 0; i < E; ++i) kept(3, i) = b[i];
+    put(3, b);
     load_phys(bf[1], b);
+    put(4, b);
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      kept(4, i) = b[i];
-      const C ax = kept(0, i), ay = kept(1, i), bx = kept(3, i);
-      x[i] = mk<C>(ax.x * b[i].x - ay.x * bx.x, ax.y * b[i].y - ay.y * bx.y);
+    for (int i0 = 0; i0 < E; i0 += 4) {
+      C ax[4], ay[4], bx[4];
+      get(0, i0, ax);
+      get(1, i0, ay);
+      get(3, i0, bx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        x[i0 + i] = mk<C>(ax[i].x * b[i0 + i].x - ay[i].x * bx[i].x, ax[i].y * b[i0 + i].y - ay[i].y * bx[i].y);
     }
     store_r2c(x, of[2], sc);
     load_phys(bf[2], b);
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const C ay = kept(1, i), az = kept(2, i), by = kept(4, i);
-      x[i] = mk<C>(ay.x * b[i].x - az.x * by.x, ay.y * b[i].y - az.y * by.y);
+    for (int i0 = 0; i0 < E; i0 += 4) {
+      C ay[4], az[4], by[4];
+      get(1, i0, ay);
+      get(2, i0, az);
+      get(4, i0, by);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        x[i0 + i] = mk<C>(ay[i].x * b[i0 + i].x - az[i].x * by[i].x, ay[i].y * b[i0 + i].y - az[i].y * by[i].y);
     }
     store_r2c(x, of[0], sc);
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const C ax = kept(0, i), az = kept(2, i), bx = kept(3, i);
-      x[i] = mk<C>(az.x * bx.x - ax.x * b[i].x, az.y * bx.y - ax.y * b[i].y);
+    for (int i0 = 0; i0 < E; i0 += 4) {
+      C ax[4], az[4], bx[4];
+      get(0, i0, ax);
+      get(2, i0, az);
+      get(3, i0, bx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        x[i0 + i] = mk<C>(az[i].x * bx[i].x - ax[i].x * b[i0 + i].x, az[i].y * bx[i].y - ax[i].y * b[i0 + i].y);
     }
     store_r2c(x, of[1], sc);
+  }
+
+  // t[0..3] = S_pq = (d_p u_q + d_q u_p) / 2 at points i0 .. from the kept
+  // gradient rows of les_rows
+  __device__ __forceinline__ void strain(int p, int q, int i0, C (&t)[4]) const {
+    get(3 + 3 * p + q, i0, t);
+    if (p == q) return;
+    C b[4];
+    get(3 + 3 * q + p, i0, b);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = mk<C>(T(0.5) * (t[i].x + b[i].x), T(0.5) * (t[i].y + b[i].y));
   }
 
   // XW_GRAD: rows 0-2 = u_c, 3 + 3 j + c = d_j u_c kept, then the products as
   // XwRow::les_store
   __device__ __forceinline__ void les_rows(const C* const f[9], C* const of[8], T sc, T tcoef) const {
-    auto put = [&](int q, const C (&x)[E]) {
-#pragma unroll
-      for (int i = 0; i < E; ++i) kept(q, i) = x[i];
-    };
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
       C x[E];
@@ -232,37 +296,64 @@ template <typename T, int LOGM> struct XgRow {
       load_phys(f[q], x);
       put(3 + q, x);
     }
-    auto S = [&](int p, int q, int i) {   // S_pq = (d_p u_q + d_q u_p) / 2
-      const C a = kept(3 + 3 * p + q, i), b = kept(3 + 3 * q + p, i);
-      return mk<C>(T(0.5) * (a.x + b.x), T(0.5) * (a.y + b.y));
-    };
     C s[E];
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const C s11 = kept(3, i), s22 = kept(7, i), s33 = kept(11, i), s12 = S(0, 1, i), s13 = S(0, 2, i), s23 = S(1, 2, i);
-      s[i].x = tcoef * sqrt(T(2) * (s11.x * s11.x + s22.x * s22.x + s33.x * s33.x +
-                                    T(2) * (s12.x * s12.x + s13.x * s13.x + s23.x * s23.x)));
-      s[i].y = tcoef * sqrt(T(2) * (s11.y * s11.y + s22.y * s22.y + s33.y * s33.y +
-                                    T(2) * (s12.y * s12.y + s13.y * s13.y + s23.y * s23.y)));
+    for (int i0 = 0; i0 < E; i0 += 4) {
+      C d[4], o[4], t[4];
+      auto add = [&](C (&acc)[4], bool first) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          acc[i] = first ? mk<C>(t[i].x * t[i].x, t[i].y * t[i].y)
+                         : mk<C>(t[i].x * t[i].x + acc[i].x, t[i].y * t[i].y + acc[i].y);
+      };
+      strain(0, 0, i0, t);
+      add(d, true);
+      strain(1, 1, i0, t);
+      add(d, false);
+      strain(2, 2, i0, t);
+      add(d, false);
+      strain(0, 1, i0, t);
+      add(o, true);
+      strain(0, 2, i0, t);
+      add(o, false);
+      strain(1, 2, i0, t);
+      add(o, false);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        s[i0 + i] = mk<C>(tcoef * sqrt(T(2) * (d[i].x + T(2) * o[i].x)), tcoef * sqrt(T(2) * (d[i].y + T(2) * o[i].y)));
     }
+    auto tau = [&](int p, int q, C (&x)[E]) {
+#pragma unroll
+      for (int i0 = 0; i0 < E; i0 += 4) {
+        C t[4];
+        strain(p, q, i0, t);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i0 + i] = mk<C>(s[i0 + i].x * t[i].x, s[i0 + i].y * t[i].y);
+      }
+    };
     C lo[H], hi[H], mid;
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
       const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
       C x[E], tl[H], th[H], tm;
-#pragma unroll
-      for (int i = 0; i < E; ++i) {
-        const C t = S(0, c, i);
-        x[i] = mk<C>(s[i].x * t.x, s[i].y * t.y);
-      }
+      tau(0, c, x);
       r2c_vals(x, tl, th, tm, T(1));
       if (c > 0) store_vals(of[c == 1 ? 3 : 6], tl, th, tm);   // tau_12, tau_13
 #pragma unroll
-      for (int i = 0; i < E; ++i) {
-        const C u1 = kept(c1, i), u2 = kept(c2, i);
-        const C a = kept(3 + 3 * c + c1, i), b = kept(3 + 3 * c1 + c, i);
-        const C d = kept(3 + 3 * c2 + c, i), e = kept(3 + 3 * c + c2, i);
-        x[i] = mk<C>(u1.x * (a.x - b.x) - u2.x * (d.x - e.x), u1.y * (a.y - b.y) - u2.y * (d.y - e.y));
+      for (int i0 = 0; i0 < E; i0 += 4) {
+        // L_c = u_c1 (d_c u_c1 - d_c1 u_c) - u_c2 (d_c2 u_c - d_c u_c2)
+        C u[4], a[4], b[4];
+        get(c1, i0, u);
+        get(3 + 3 * c + c1, i0, a);
+        get(3 + 3 * c1 + c, i0, b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i0 + i] = mk<C>(u[i].x * (a[i].x - b[i].x), u[i].y * (a[i].y - b[i].y));
+        get(c2, i0, u);
+        get(3 + 3 * c2 + c, i0, a);
+        get(3 + 3 * c + c2, i0, b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          x[i0 + i] = mk<C>(x[i0 + i].x - u[i].x * (a[i].x - b[i].x), x[i0 + i].y - u[i].y * (a[i].y - b[i].y));
       }
       r2c_vals(x, lo, hi, mid, sc);
 #pragma unroll
@@ -277,11 +368,7 @@ template <typename T, int LOGM> struct XgRow {
 #pragma unroll 1
     for (int q = 0; q < 3; ++q) {   // tau_22, tau_23, tau_33
       C x[E];
-#pragma unroll
-      for (int i = 0; i < E; ++i) {
-        const C t = S(q == 2 ? 2 : 1, q == 0 ? 1 : 2, i);
-        x[i] = mk<C>(s[i].x * t.x, s[i].y * t.y);
-      }
+      tau(q == 2 ? 2 : 1, q == 0 ? 1 : 2, x);
       store_r2c(x, of[q == 2 ? 7 : 4 + q], T(1));
     }
   }
@@ -294,9 +381,11 @@ template <typename T, int LOGM> struct XgRow {
     for (int c = 0; c < 3; ++c) {
       C x[E];
 #pragma unroll
-      for (int i = 0; i < E; ++i) {
-        const C a = kept(c, i);
-        x[i] = mk<C>(a.x * b[i].x, a.y * b[i].y);
+      for (int i0 = 0; i0 < E; i0 += 4) {
+        C a[4];
+        get(c, i0, a);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i0 + i] = mk<C>(a[i].x * b[i0 + i].x, a[i].y * b[i0 + i].y);
       }
       store_r2c(x, of[c], sc);
     }
@@ -309,25 +398,31 @@ template <typename T, int LOGM> struct XgRow {
     for (int q = 0; q < 6; ++q) {
       C x[E];
       load_phys(sf[q], x);
-#pragma unroll
-      for (int i = 0; i < E; ++i) kept(q, i) = x[i];
+      put(q, x);
     }
     C a[E];
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const C s11 = kept(0, i), s12 = kept(1, i), s13 = kept(2, i), s22 = kept(3, i), s23 = kept(4, i), s33 = kept(5, i);
-      a[i].x = sqrt(T(2) * (s11.x * s11.x + s22.x * s22.x + s33.x * s33.x +
-                            T(2) * (s12.x * s12.x + s13.x * s13.x + s23.x * s23.x)));
-      a[i].y = sqrt(T(2) * (s11.y * s11.y + s22.y * s22.y + s33.y * s33.y +
-                            T(2) * (s12.y * s12.y + s13.y * s13.y + s23.y * s23.y)));
+    for (int i0 = 0; i0 < E; i0 += 4) {
+      C s[6][4];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) get(q, i0, s[q]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[i0 + i].x = sqrt(T(2) * (s[0][i].x * s[0][i].x + s[3][i].x * s[3][i].x + s[5][i].x * s[5][i].x +
+                                   T(2) * (s[1][i].x * s[1][i].x + s[2][i].x * s[2][i].x + s[4][i].x * s[4][i].x)));
+        a[i0 + i].y = sqrt(T(2) * (s[0][i].y * s[0][i].y + s[3][i].y * s[3][i].y + s[5][i].y * s[5][i].y +
+                                   T(2) * (s[1][i].y * s[1][i].y + s[2][i].y * s[2][i].y + s[4][i].y * s[4][i].y)));
+      }
     }
 #pragma unroll 1
     for (int q = 0; q < 6; ++q) {
       C x[E];
 #pragma unroll
-      for (int i = 0; i < E; ++i) {
-        const C s = kept(q, i);
-        x[i] = mk<C>(a[i].x * s.x, a[i].y * s.y);
+      for (int i0 = 0; i0 < E; i0 += 4) {
+        C s[4];
+        get(q, i0, s);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i0 + i] = mk<C>(a[i0 + i].x * s[i].x, a[i0 + i].y * s[i].y);
       }
       store_r2c(x, of[q], tcoef);
     }
@@ -337,25 +432,32 @@ template <typename T, int LOGM> struct XgRow {
 template <typename T, int LOGM, int MODE> struct XgCfg {
   using GF = GroupFFT<T, LOGM>;
   static constexpr int KEPT = MODE == XW_GRAD ? 12 : (MODE == XW_SMAG ? 6 : 5);
-  static constexpr int PER_WARP = GF::RW * (KEPT * GF::M + GF::BUF);
+  // FP32 rows of 64 points: three (XW_GRAD: six) kept rows in tensor memory,
+  // which leaves shared memory for four CTAs per SM (LES products at 128^3 71
+  // -> 58 us); a warp per lane quarter
+  static constexpr int KT = sizeof(T) == 4 && LOGM >= 6 ? (MODE == XW_GRAD ? 6 : 3) : 0;
+  static constexpr int TM_COLS = 2 * GF::E * KT <= 64 ? 64 : 128;
+  static_assert(2 * GF::E * KT <= TM_COLS, "tensor-memory rows");
+  static constexpr int PER_WARP = GF::RW * ((KEPT - KT) * GF::M + GF::BUF);
   // four warps, fewer where their kept rows pass the 227 KB of a CTA
   static constexpr int FIT = (int)(227 * 1024 / (sizeof(C2<T>) * PER_WARP));
   static constexpr int WARPS = FIT < 4 ? FIT : 4, NT = 32 * WARPS;
   static constexpr size_t SMEM = sizeof(C2<T>) * (size_t)PER_WARP * WARPS;
-  static constexpr int MINB = SMEM * 2 <= 220 * 1024 ? 2 : 1;
+  static constexpr int FITB = (int)(220 * 1024 / SMEM), MAXB = sizeof(T) == 4 ? 4 : 2;
+  static constexpr int MINB = FITB < 1 ? 1 : (FITB > MAXB ? MAXB : FITB);
 };
 
-template <typename T, int LOGM>
-__device__ __forceinline__ XgRow<T, LOGM> xg_row(C2<T>* warp_smem, int kept, long long warp, const Geom& g,
-                                                 const C2<T>* twM, const C2<T>* twN, long long rows) {
+template <typename T, int LOGM, int KT = 0>
+__device__ __forceinline__ XgRow<T, LOGM, KT> xg_row(C2<T>* warp_smem, int kept, long long warp, const Geom& g,
+                                                     const C2<T>* twM, const C2<T>* twN, long long rows) {
   using GF = GroupFFT<T, LOGM>;
-  XgRow<T, LOGM> R;
+  XgRow<T, LOGM, KT> R;
   R.lane = threadIdx.x & 31;
   R.l = R.lane % GF::L;
   const int q = R.lane / GF::L;
   R.mate = q * GF::L + (GF::L - R.l) % GF::L;
   R.keep = warp_smem;
-  R.buf = warp_smem + kept * GF::M * GF::RW + q * GF::BUF;
+  R.buf = warp_smem + (kept - KT) * GF::M * GF::RW + q * GF::BUF;
   const long long row = warp * GF::RW + q;
   R.live = row < rows;
   R.off = (R.live ? row : rows - 1) * g.nxp;
@@ -374,8 +476,17 @@ xpass_group_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __r
   using Cfg = XgCfg<T, LOGM, MODE>;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int warp = threadIdx.x >> 5;
-  const XgRow<T, LOGM> R = xg_row<T, LOGM>(reinterpret_cast<C*>(smraw) + warp * Cfg::PER_WARP, Cfg::KEPT,
-                                           (long long)blockIdx.x * Cfg::WARPS + warp, g, twM, twN, xa.rows);
+  auto R = xg_row<T, LOGM, Cfg::KT>(reinterpret_cast<C*>(smraw) + warp * Cfg::PER_WARP, Cfg::KEPT,
+                                    (long long)blockIdx.x * Cfg::WARPS + warp, g, twM, twN, xa.rows);
+  __shared__ uint32_t s_tmem;
+  if constexpr (Cfg::KT > 0) {
+    static_assert(Cfg::KT == 0 || Cfg::WARPS == 4, "a warp per lane quarter of tensor memory");
+    if (warp == 0) tmem_alloc(&s_tmem, Cfg::TM_COLS);
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    R.ta = s_tmem + ((uint32_t)(32 * warp) << 16);
+  }
   const C* u[3] = {fin.f[0], fin.f[1], fin.f[2]};
   const C* w[3] = {fin.f[3], fin.f[4], fin.f[5]};
   C* o[3] = {fout.f[0], fout.f[1], fout.f[2]};
@@ -403,6 +514,15 @@ xpass_group_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __r
     R.cross_store(w, o, T(-1));
     R.cross_store(u, o2, T(1));
   }
+  if constexpr (Cfg::KT > 0) {
+    // every warp's tensor-memory reads are complete before the release
+    tmem_fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+      tmem_fence_after_sync();
+      tmem_dealloc(s_tmem, Cfg::TM_COLS);
+    }
+  }
 }
 
 // max |u|^2 and the non-finite count of three velocity fields, as
@@ -422,8 +542,8 @@ xgroup_umax_kernel(FieldList<T> fin, Geom g, const C2<T>* __restrict__ twM, cons
   constexpr int E = GroupFFT<T, LOGM>::E;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int warp = threadIdx.x >> 5;
-  const XgRow<T, LOGM> R = xg_row<T, LOGM>(reinterpret_cast<C*>(smraw) + warp * Cfg::PER_WARP, 0,
-                                           (long long)blockIdx.x * Cfg::WARPS + warp, g, twM, twN, xa.rows);
+  const auto R = xg_row<T, LOGM>(reinterpret_cast<C*>(smraw) + warp * Cfg::PER_WARP, 0,
+                                 (long long)blockIdx.x * Cfg::WARPS + warp, g, twM, twN, xa.rows);
   C u2[E];
 #pragma unroll
   for (int i = 0; i < E; ++i) u2[i] = czero<C>();
