@@ -11,10 +11,13 @@
 #include <vector>
 
 #include "../../include/specns.h"
-#include "sc_ens.cuh"
+#include "sc_ens_split.cuh"
 
 namespace sc {
 int set_last_error(int code, const char* msg);   // sc_runtime.cu
+// 4D tensor map over 8-byte units (sc_runtime.cu); strides in bytes of dims 1..3
+int encode_map4(const void* base, const unsigned long long dims[4], const unsigned long long strides[3],
+                const unsigned box[4], CUtensorMap* out);
 }
 
 namespace {
@@ -32,6 +35,16 @@ bool pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 int ilog(int n) { int l = 0; while ((1 << l) < n) ++l; return l; }
 
 }  // namespace
+
+// The members of one size, for the launch-per-pass form.
+struct EnsClassHost {
+  int n = 0;
+  std::vector<int> members;     // ensemble indices, in memory order
+  size_t off = 0;               // elements of the first member's first field
+  CUtensorMap map;
+  cudaStream_t stream = nullptr;
+  cudaEvent_t done = nullptr;
+};
 
 struct sc_ensemble {
   int prec = SC_FP32;
@@ -54,6 +67,12 @@ struct sc_ensemble {
   std::vector<long long> field;    // per member: elements per field
   std::vector<int> nxp;
   cudaGraphExec_t graph = nullptr;
+  std::vector<EnsClassHost> classes;
+  std::vector<int> class_of, class_index;   // per member
+  void* dpar = nullptr;                     // EnsParam<T> of the members, class by class
+  std::vector<int> par_off;                 // per class
+  cudaEvent_t fork = nullptr;
+  int nsm = 152;
   // launch shape: the autotuner's choice among the compiled variants
   int variant = 0;
   bool tuned = false;
@@ -100,6 +119,14 @@ template <typename T> int launch_stage(sc_ensemble* e, int stage, const sc::EnsM
 template <typename T> int select_variant(sc_ensemble* e, int vi) {
   using C = sc::C2<T>;
   const sc::EnsVariant v = variant(e, vi);
+  if (v.split) {
+    if (e->graph) {
+      cudaGraphExecDestroy(e->graph);
+      e->graph = nullptr;
+    }
+    e->variant = vi;
+    return SC_OK;
+  }
   if (!v.kernel) return efail(SC_ERR_INVALID, "no such ensemble variant");
   const size_t smem = sizeof(C) * (size_t)v.smem_elems;
   EC(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -165,17 +192,29 @@ template <typename T> int setup(sc_ensemble* e) {
   sc::WarpTw::fill(t.data(), [](double a) { return std::cos(a); }, [](double a) { return std::sin(a); });
   EC(cudaMalloc(&e->tw, sizeof(C) * t.size()));
   EC(cudaMemcpy(e->tw, t.data(), sizeof(C) * t.size(), cudaMemcpyHostToDevice));
-  // fields: 6 per member (w, s, acc, work x3)
+  // fields: 6 per member (w, s, acc, work x3), the members of one size side
+  // by side
   size_t total = 0;
   e->field_off.resize(e->nm);
   e->field.resize(e->nm);
   e->nxp.resize(e->nm);
-  for (int m = 0; m < e->nm; ++m) {
-    const int N = e->n[m];
-    e->nxp[m] = (N / 2 + 1 + 15) / 16 * 16;
-    e->field[m] = (long long)N * e->nxp[m];
-    e->field_off[m] = total;
-    total += 6 * (size_t)e->field[m];
+  e->class_of.resize(e->nm);
+  e->class_index.resize(e->nm);
+  for (int N = 64; N <= 1024; N *= 2) {
+    EnsClassHost c;
+    c.n = N;
+    c.off = total;
+    for (int m = 0; m < e->nm; ++m) {
+      if (e->n[m] != N) continue;
+      e->nxp[m] = (N / 2 + 1 + 15) / 16 * 16;
+      e->field[m] = (long long)N * e->nxp[m];
+      e->field_off[m] = total;
+      e->class_of[m] = (int)e->classes.size();
+      e->class_index[m] = (int)c.members.size();
+      c.members.push_back(m);
+      total += 6 * (size_t)e->field[m];
+    }
+    if (!c.members.empty()) e->classes.push_back(c);
   }
   EC(cudaMalloc(&e->mem, sizeof(C) * total));
   EC(cudaMemsetAsync(e->mem, 0, sizeof(C) * total, e->stream));
@@ -184,6 +223,27 @@ template <typename T> int setup(sc_ensemble* e) {
   EC(cudaMemset(e->bar, 0, 2 * sizeof(unsigned)));
   EC(cudaMalloc(&e->err, sizeof(int)));
   EC(cudaMemset(e->err, 0, sizeof(int)));
+  {
+    int dev = 0;
+    EC(cudaGetDevice(&dev));
+    EC(cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, dev));
+  }
+  std::vector<sc::EnsParam<T>> par;
+  for (auto& c : e->classes) {
+    e->par_off.push_back((int)par.size());
+    for (int m : c.members) par.push_back({(T)e->dt[m], (T)e->alpha, (T)e->nu8[m]});
+    const int N = c.n, U = (int)sizeof(C) / 8, P = sc::ens_split_tile<T>(ilog(N));
+    const unsigned long long f = (unsigned long long)e->field[c.members[0]], nxp = e->nxp[c.members[0]];
+    const unsigned long long dims[4] = {(unsigned long long)(N / 2 + 1) * U, (unsigned long long)N, c.members.size(), 6};
+    const unsigned long long strides[3] = {nxp * sizeof(C), 6 * f * sizeof(C), f * sizeof(C)};
+    const unsigned box[4] = {(unsigned)(P * U), (unsigned)(N < 256 ? N : 256), 1, 1};
+    if (int r = sc::encode_map4(static_cast<C*>(e->mem) + c.off, dims, strides, box, &c.map)) return r;
+    EC(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
+    EC(cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming));
+  }
+  EC(cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming));
+  EC(cudaMalloc(&e->dpar, sizeof(sc::EnsParam<T>) * par.size()));
+  EC(cudaMemcpy(e->dpar, par.data(), sizeof(sc::EnsParam<T>) * par.size(), cudaMemcpyHostToDevice));
   e->tune_ms.assign(nvariants(e), -1.0);
   // a pinned variant (SPECNS_ENS_VARIANT) skips the autotuner
   int v0 = 0;
@@ -252,7 +312,43 @@ template <typename T> int tune(sc_ensemble* e, int trial) {
   return rc;
 }
 
+// `count` members of class c from its member m0 on, one step, on stream s
+template <typename T> int split_steps(sc_ensemble* e, int c, int m0, int count, cudaStream_t s) {
+  const EnsClassHost& h = e->classes[c];
+  const int m = h.members[0];
+  sc::EnsClass<T> ec{};
+  ec.n = h.n;
+  ec.logn = ilog(h.n);
+  ec.nxh = h.n / 2 + 1;
+  ec.nxp = e->nxp[m];
+  ec.field = e->field[m];
+  ec.base = static_cast<sc::C2<T>*>(e->mem) + h.off;
+  ec.par = static_cast<const sc::EnsParam<T>*>(e->dpar) + e->par_off[c];
+  ec.scale = (T)(1.0 / ((double)h.n * h.n));
+  ec.tw = static_cast<const sc::C2<T>*>(e->tw);
+  ec.err = e->err;
+  ec.nsm = e->nsm;
+  ec.m0 = m0;
+  ec.count = count;
+  for (ec.stage = 1; ec.stage <= 4; ++ec.stage) EC(sc::ens_split_stage<T>(h.map, ec, s));
+  return SC_OK;
+}
+
 template <typename T> int step_batched(sc_ensemble* e) {
+  if (variant(e, e->variant).split) {
+    // the classes as branches beside e->stream, the largest members first
+    const int nc = (int)e->classes.size();
+    if (nc > 1) EC(cudaEventRecord(e->fork, e->stream));
+    for (int c = nc - 1; c >= 0; --c) {
+      auto& h = e->classes[c];
+      cudaStream_t s = c == nc - 1 ? e->stream : h.stream;
+      if (s != e->stream) EC(cudaStreamWaitEvent(s, e->fork, 0));
+      if (int r = split_steps<T>(e, c, 0, (int)h.members.size(), s)) return r;
+      if (s != e->stream) EC(cudaEventRecord(h.done, s));
+    }
+    for (int c = nc - 2; c >= 0; --c) EC(cudaStreamWaitEvent(e->stream, e->classes[c].done, 0));
+    return SC_OK;
+  }
   auto* mb = static_cast<const sc::EnsMember<T>*>(e->dmem_members);
   for (int st = 1; st <= 4; ++st)
     if (int r = launch_stage<T>(e, st, mb, e->nm, e->items_y, e->items_x)) return r;
@@ -260,6 +356,12 @@ template <typename T> int step_batched(sc_ensemble* e) {
 }
 
 template <typename T> int steps_one_at_a_time(sc_ensemble* e, int nsteps) {
+  if (variant(e, e->variant).split) {
+    for (int m = 0; m < e->nm; ++m)
+      for (int i = 0; i < nsteps; ++i)
+        if (int r = split_steps<T>(e, e->class_of[m], e->class_index[m], 1, e->stream)) return r;
+    return SC_OK;
+  }
   auto* mb = static_cast<const sc::EnsMember<T>*>(e->dmem_members) + e->nm;
   for (int m = 0; m < e->nm; ++m)
     for (int i = 0; i < nsteps; ++i)
@@ -274,7 +376,7 @@ int check_err(sc_ensemble* e) {
   EC(cudaStreamSynchronize(e->stream));
   if (v) {
     cudaMemsetAsync(e->err, 0, sizeof(int), e->stream);
-    return efail(SC_ERR_TIMEOUT, "a bounded grid barrier gave up");
+    return efail(SC_ERR_TIMEOUT, "a bounded device wait gave up (grid barrier or TMA load)");
   }
   return SC_OK;
 }
@@ -346,6 +448,12 @@ int sc_ens_destroy(sc_ensemble* e) {
   cudaFree(e->tw);
   cudaFree(e->bar);
   cudaFree(e->err);
+  cudaFree(e->dpar);
+  for (auto& c : e->classes) {
+    if (c.stream) cudaStreamDestroy(c.stream);
+    if (c.done) cudaEventDestroy(c.done);
+  }
+  if (e->fork) cudaEventDestroy(e->fork);
   if (e->own) cudaStreamDestroy(e->own);
   delete e;
   return SC_OK;

@@ -400,14 +400,16 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) ens_stage_kernel(EnsArgs<T> 
 // The compiled shapes (sc_ens_k_*.cu, one translation unit each), by variant
 // number, <threads, CTAs per SM, tile points, radix, out of line>.  FP32:
 // 0 <256, 2, 4096, 8, no>, 1 <256, 2, 4096, 8, yes>, 2 <512, 1, 8192, 8, no>,
-// 3 <512, 1, 8192, 8, yes>, 4 <256, 2, 4096, 4, no>, 5 <512, 1, 4096, 8, no>.
-// FP64: 0 <256, 2, 4096, 8, no>, 1 <256, 2, 4096, 8, yes>.
+// 3 <512, 1, 8192, 8, yes>, 4 <256, 2, 4096, 4, no>, 5 a launch per pass
+// (sc_ens_split.cuh).  FP64: 0 <256, 2, 4096, 8, no>, 1 a launch per pass.
 
 // A compiled variant as the host sees it.
 struct EnsVariant {
-  const void* kernel;   // ens_stage_kernel<T, Shape>
+  const void* kernel;   // ens_stage_kernel<T, Shape> (split: none)
   int nt, minb, ypts, rmax, outline, smem_elems;
+  bool split = false;   // a launch per pass
 };
+constexpr EnsVariant kEnsSplit{nullptr, 512, 2, 4096, 8, 0, 0, true};
 
 template <class SH, typename T> EnsVariant ens_variant_of() {
   return EnsVariant{reinterpret_cast<const void*>(&ens_stage_kernel<T, SH>), SH::NT, SH::MINB, SH::YPTS, SH::RMAX,

@@ -6,9 +6,7 @@ EnsVariant ens_variant_f32_v1();
 EnsVariant ens_variant_f32_v2();
 EnsVariant ens_variant_f32_v3();
 EnsVariant ens_variant_f32_v4();
-EnsVariant ens_variant_f32_v5();
 EnsVariant ens_variant_f64_v0();
-EnsVariant ens_variant_f64_v1();
 
 EnsVariant ens_variant_f32(int v) {
   switch (v) {
@@ -17,7 +15,7 @@ EnsVariant ens_variant_f32(int v) {
     case 2: return ens_variant_f32_v2();
     case 3: return ens_variant_f32_v3();
     case 4: return ens_variant_f32_v4();
-    case 5: return ens_variant_f32_v5();
+    case 5: return kEnsSplit;
     default: return EnsVariant{nullptr, 0, 0, 0, 0, 0, 0};
   }
 }
@@ -25,7 +23,7 @@ EnsVariant ens_variant_f32(int v) {
 EnsVariant ens_variant_f64(int v) {
   switch (v) {
     case 0: return ens_variant_f64_v0();
-    case 1: return ens_variant_f64_v1();
+    case 1: return kEnsSplit;
     default: return EnsVariant{nullptr, 0, 0, 0, 0, 0, 0};
   }
 }

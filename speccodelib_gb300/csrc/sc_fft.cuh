@@ -358,16 +358,15 @@ struct FFTEngine {
     last_stage<INV>(out, sm, tw);
   }
 
-  // The transform of i k(n) x from the tile src (kept), k(n) the signed
-  // wavenumber of point n, through the tile sm; output in registers.  Ends with
-  // a barrier.
-  template <bool INV>
-  __device__ static void run_deriv(C (&out)[JL][RL], const C* src, C* sm, const C* __restrict__ tw) {
+  // The transform of f(x, p, n) for the points x of the tile src (kept),
+  // through the tile sm; output in registers.  Ends with a barrier.
+  template <bool INV, class F>
+  __device__ static __forceinline__ void run_map(C (&out)[JL][RL], const C* src, C* sm, const C* __restrict__ tw, F&& f) {
     auto load = [&](C (&v)[R1], int j, int p) {
 #pragma unroll
       for (int r = 0; r < R1; ++r) {
         const int n = j + r * (N / R1);
-        v[r] = cmuli(cscale(src[sidx(n) * PS + p], (T)wavenum(n, N)));
+        v[r] = f(src[sidx(n) * PS + p], p, n);
       }
     };
 #pragma unroll

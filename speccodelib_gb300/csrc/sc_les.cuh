@@ -98,7 +98,8 @@ les_yinv_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, 
         }
     };
     if (f < 3) {
-      E::template run_deriv<true>(out, buf(b), work, tw);
+      E::template run_map<true>(out, buf(b), work, tw,
+                                [](C x, int, int n) { return cmuli(cscale(x, (T)wavenum(n, Cfg::N))); });
       store(fp + 6 * tp.field);
     }
     E::template run_smem<true>(out, buf(b), tw);

@@ -195,24 +195,30 @@ PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
   return fn;
 }
 
+// 4D map over 8-byte units: extents, byte strides of dims 1..3, box.
+int encode4(const void* base, const cuuint64_t dims[4], const cuuint64_t strides[3], const cuuint32_t box[4],
+            CUtensorMap* out) {
+  auto enc = tmap_encoder();
+  if (!enc) return fail(SC_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  cuuint32_t es[4] = {1, 1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void*>(base), dims, strides, box, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(SC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+  return SC_OK;
+}
+
 // 4D map over `nf` fields starting at `base` (fields `field` elements apart):
 // dims (x: nxh complex, y, z, field) in 8-byte units; box (P, BOX, 1, 1) for
 // axis 1 (y) or (P, 1, BOX, 1) for axis 2 (z).
 int encode_fields(sc_handle* h, const void* base, int nf, int axis, int P, int N, CUtensorMap* out) {
-  auto enc = tmap_encoder();
-  if (!enc) return fail(SC_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const int U = (int)(h->csize / 8);
   const int box = N < 256 ? N : 256;
   cuuint64_t dims[4] = {(cuuint64_t)h->g.nxh * U, (cuuint64_t)h->g.ny, (cuuint64_t)h->g.nz, (cuuint64_t)nf};
   cuuint64_t strides[3] = {(cuuint64_t)h->g.nxp * h->csize, (cuuint64_t)h->g.nxp * h->g.ny * h->csize,
                            (cuuint64_t)h->g.field * h->csize};
   cuuint32_t boxd[4] = {(cuuint32_t)(P * U), (cuuint32_t)(axis == 1 ? box : 1), (cuuint32_t)(axis == 2 ? box : 1), 1};
-  cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void*>(base), dims, strides, boxd, es,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(SC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return SC_OK;
+  return encode4(base, dims, strides, boxd, out);
 }
 
 int check_derr(sc_handle* h) {
@@ -1870,9 +1876,17 @@ template <typename T> int impl_dispatch_tile(int logz) {
 
 }  // namespace
 
-// Error channel for entry points defined in other translation units.
+// Error channel and tensor maps for entry points defined in other translation
+// units.
 namespace sc {
 int set_last_error(int code, const char* msg) { return fail(code, "%s", msg); }
+int encode_map4(const void* base, const unsigned long long dims[4], const unsigned long long strides[3],
+                const unsigned box[4], CUtensorMap* out) {
+  cuuint64_t d[4], st[3];
+  for (int i = 0; i < 4; ++i) d[i] = dims[i];
+  for (int i = 0; i < 3; ++i) st[i] = strides[i];
+  return encode4(base, d, st, box, out);
+}
 }  // namespace sc
 
 // ===========================================================================
