@@ -55,6 +55,7 @@ struct sc_ensemble {
   double alpha = 0;
   cudaStream_t own = nullptr, stream = nullptr;
   void* mem = nullptr;          // all member fields
+  void* stage = nullptr;        // one member in the reference layout: host copies go through it
   void* dmem_members = nullptr; // EnsMember<T>[nm] (batched) then [nm] (one at a time)
   void* tw = nullptr;
   unsigned* bar = nullptr;
@@ -444,6 +445,7 @@ int sc_ens_destroy(sc_ensemble* e) {
   if (e->stream) cudaStreamSynchronize(e->stream);
   if (e->graph) cudaGraphExecDestroy(e->graph);
   cudaFree(e->mem);
+  cudaFree(e->stage);
   cudaFree(e->dmem_members);
   cudaFree(e->tw);
   cudaFree(e->bar);
@@ -469,22 +471,48 @@ int sc_ens_set_stream(sc_ensemble* e, void* stream) {
   return SC_OK;
 }
 
-int sc_ens_set_member(sc_ensemble* e, int m, const void* w) {
-  if (!e || !w || m < 0 || m >= e->nm) return efail(SC_ERR_INVALID, "sc_ens_set_member: bad arguments");
-  const size_t row = e->csize * (e->n[m] / 2 + 1);
-  char* dst = static_cast<char*>(e->mem) + e->csize * e->field_off[m];
-  EC(cudaMemcpy2DAsync(dst, e->csize * e->nxp[m], w, row, row, e->n[m], cudaMemcpyDefault, e->stream));
+// A member's rows of N/2+1 to or from user memory.  Host memory moves as one
+// contiguous copy through a device buffer: the row-by-row copies of a strided
+// transfer to pageable memory ran at 2.2 GB/s.
+static int copy_member(sc_ensemble* e, int m, void* user, bool in) {
+  const size_t row = e->csize * (e->n[m] / 2 + 1), rows = e->n[m], pitch = e->csize * e->nxp[m];
+  char* dev = static_cast<char*>(e->mem) + e->csize * e->field_off[m];
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, user) != cudaSuccess) cudaGetLastError();
+  const bool host = a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeUnregistered;
+  if (host && !e->stage) {
+    size_t most = 0;
+    for (int k = 0; k < e->nm; ++k) most = std::max(most, e->csize * (e->n[k] / 2 + 1) * (size_t)e->n[k]);
+    if (cudaMalloc(&e->stage, most) != cudaSuccess) {
+      cudaGetLastError();
+      e->stage = nullptr;
+    }
+  }
+  if (host && e->stage) {
+    if (in) {
+      EC(cudaMemcpyAsync(e->stage, user, row * rows, cudaMemcpyHostToDevice, e->stream));
+      EC(cudaMemcpy2DAsync(dev, pitch, e->stage, row, row, rows, cudaMemcpyDeviceToDevice, e->stream));
+    } else {
+      EC(cudaMemcpy2DAsync(e->stage, row, dev, pitch, row, rows, cudaMemcpyDeviceToDevice, e->stream));
+      EC(cudaMemcpyAsync(user, e->stage, row * rows, cudaMemcpyDeviceToHost, e->stream));
+    }
+  } else if (in) {
+    EC(cudaMemcpy2DAsync(dev, pitch, user, row, row, rows, cudaMemcpyDefault, e->stream));
+  } else {
+    EC(cudaMemcpy2DAsync(user, row, dev, pitch, row, rows, cudaMemcpyDefault, e->stream));
+  }
   EC(cudaStreamSynchronize(e->stream));
   return SC_OK;
 }
 
+int sc_ens_set_member(sc_ensemble* e, int m, const void* w) {
+  if (!e || !w || m < 0 || m >= e->nm) return efail(SC_ERR_INVALID, "sc_ens_set_member: bad arguments");
+  return copy_member(e, m, const_cast<void*>(w), true);
+}
+
 int sc_ens_get_member(sc_ensemble* e, int m, void* w) {
   if (!e || !w || m < 0 || m >= e->nm) return efail(SC_ERR_INVALID, "sc_ens_get_member: bad arguments");
-  const size_t row = e->csize * (e->n[m] / 2 + 1);
-  const char* src = static_cast<const char*>(e->mem) + e->csize * e->field_off[m];
-  EC(cudaMemcpy2DAsync(w, row, src, e->csize * e->nxp[m], row, e->n[m], cudaMemcpyDefault, e->stream));
-  EC(cudaStreamSynchronize(e->stream));
-  return SC_OK;
+  return copy_member(e, m, w, false);
 }
 
 int sc_ens_init(sc_ensemble* e, const int* seeds, double kpeak, double energy) {
