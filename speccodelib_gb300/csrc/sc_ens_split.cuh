@@ -47,9 +47,12 @@ template <typename T> struct EnsClass {
 template <typename T, int LOGN> struct EnsSplitCfg {
   static constexpr int N = 1 << LOGN;
   static constexpr int U = sizeof(T) / 4;
-  // 32 KB tiles at N >= 256: two CTAs of a y pass (three tiles) per SM
-  static constexpr int P4 = LOGN <= 8 ? 16 : (LOGN == 9 ? 8 : 4);
+  // rows of 64 bytes or more: 32 KB tiles and two CTAs per SM up to N = 512,
+  // 64 KB and one at 1024 (16 points per thread; its ens_yfwd 185 us for 16
+  // members, 213 with 32-byte rows and two CTAs)
+  static constexpr int P4 = LOGN <= 8 ? 16 : 8;
   static constexpr int P = sizeof(T) == 4 ? P4 : P4 / 2;
+  static constexpr int MINB = LOGN <= 9 ? 2 : 1;
   static constexpr int NT_RAW = P * N / 8;
   static constexpr int NT = NT_RAW > 512 ? 512 : (NT_RAW < 32 ? 32 : NT_RAW);
   static constexpr int BOX = N < 256 ? N : 256;
@@ -97,7 +100,7 @@ __device__ __forceinline__ void ens_uvw(C2<T>* s, C2<T>* work, const C2<T>* __re
 
 // First stage's operands from the state.  Persistent, two tiles in flight.
 template <typename T, int LOGN>
-__global__ void __launch_bounds__(EnsSplitCfg<T, LOGN>::NT, 2)
+__global__ void __launch_bounds__(EnsSplitCfg<T, LOGN>::NT, EnsSplitCfg<T, LOGN>::MINB)
 ens_yinv_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
   using Cfg = EnsSplitCfg<T, LOGN>;
   using C = C2<T>;
@@ -138,7 +141,7 @@ ens_yinv_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
 
 // End of a stage (see the head of this file).  grid = (kx tiles, members).
 template <typename T, int LOGN>
-__global__ void __launch_bounds__(EnsSplitCfg<T, LOGN>::NT, 2)
+__global__ void __launch_bounds__(EnsSplitCfg<T, LOGN>::NT, EnsSplitCfg<T, LOGN>::MINB)
 ens_yfwd_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
   using Cfg = EnsSplitCfg<T, LOGN>;
   using E = typename Cfg::Engine;
