@@ -86,7 +86,7 @@ cudaError_t launch_plain_tma(const CUtensorMap& map, const TmaPass<T>& tp, const
   static cudaError_t attr = smem_attr(k, sm);
   if (attr != cudaSuccess) return attr;
   const long long total = (long long)tp.ntx * tp.nouter * tp.nf;
-  long long grid = (long long)nsm * 2;
+  long long grid = (long long)nsm * Cfg::PB;
   if (grid > total) grid = total;
   k<<<(unsigned)grid, Cfg::NT, sm, s>>>(map, tp, g, tw);
   return cudaGetLastError();

@@ -32,7 +32,11 @@ template <typename T, int LOGN> struct TmaCfg {
   using Engine = FFTEngine<T, LOGN, P, P, NT, true>;
   static constexpr size_t TILE_BYTES = sizeof(C2<T>) * N * P;
   // pipeline depth of pencil_tma_kernel: tiles in flight per CTA
-  static constexpr int STAGES = TILE_BYTES <= 16384 ? 4 : 3;
+  static constexpr int STAGES = TILE_BYTES <= 8192 ? 3 : (TILE_BYTES <= 16384 ? 4 : 3);
+  // its CTAs per SM: eight for tiles of 8 KB and less (128 threads or fewer; the
+  // 512 x 64 x 256 FP32 step 7.73 -> 7.02 ms per five), else two (four CTAs of
+  // 16 KB tiles took 34 us against 29 for nine fields at 128^3)
+  static constexpr int PB = TILE_BYTES <= 8192 ? 8 : 2;
   // zinv uses a narrower tile: 3 inputs + 1 work buffer
   static constexpr int PZ = P >= 8 ? P / 2 : P;
   static constexpr int NTZ_RAW = PZ * N / 8;
@@ -123,7 +127,7 @@ __device__ __forceinline__ void tma_issue_tile(void* dst, const CUtensorMap* map
 }
 
 template <typename T, int LOGN, bool INV>
-__global__ void __launch_bounds__(TmaCfg<T, LOGN>::NT, 2)
+__global__ void __launch_bounds__(TmaCfg<T, LOGN>::NT, TmaCfg<T, LOGN>::PB)
 pencil_tma_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, const C2<T>* __restrict__ tw) {
   using Cfg = TmaCfg<T, LOGN>;
   // stage-0 writes XOR-rotated (conflict-free 64-byte rows) in the forward
