@@ -276,6 +276,7 @@ template <typename T, int LOGN>
 __global__ void __launch_bounds__(AdjTmaCfg<T, LOGN>::NT, AdjTmaCfg<T, LOGN>::MINB)
 zfwd_adj_tma_kernel(const __grid_constant__ CUtensorMap pmap, int4 fidx_lo, int2 fidx_hi, AdjArgs<T> aa, Geom g,
                     const C2<T>* __restrict__ tw, int* err) {
+  pdl_wait();
   using AC = AdjTmaCfg<T, LOGN>;
   using Cfg = TmaCfg<T, LOGN>;
   using E = typename AC::Engine;
@@ -342,6 +343,7 @@ zfwd_adj_tma_kernel(const __grid_constant__ CUtensorMap pmap, int4 fidx_lo, int2
 // and the map is one-to-one, so the points are independent.
 template <typename T>
 __global__ void adj_copyT_kernel(FieldList<T> lw, Geom g) {
+  pdl_wait();
   using C = C2<T>;
   const long long total = (long long)g.ny * g.nz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;

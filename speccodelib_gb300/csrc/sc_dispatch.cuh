@@ -88,8 +88,7 @@ cudaError_t launch_plain_tma(const CUtensorMap& map, const TmaPass<T>& tp, const
   const long long total = (long long)tp.ntx * tp.nouter * tp.nf;
   long long grid = (long long)nsm * Cfg::PB;
   if (grid > total) grid = total;
-  k<<<(unsigned)grid, Cfg::NT, sm, s>>>(map, tp, g, tw);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3((unsigned)grid), dim3(Cfg::NT), sm, s, map, tp, g, tw);
 }
 
 template <typename T, int LOGN>
@@ -131,8 +130,7 @@ cudaError_t launch_les_y(bool inv, const CUtensorMap& map, const TmaPass<T>& tp,
   const long long total = (long long)tp.ntx * tp.nouter * (inv ? 6 : 5);
   long long grid = (long long)nsm * 2;
   if (grid > total) grid = total;
-  k<<<(unsigned)grid, Cfg::NT, sm, s>>>(map, tp, g, tw);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3((unsigned)grid), dim3(Cfg::NT), sm, s, map, tp, g, tw);
 }
 
 template <typename T, int LOGN>
@@ -143,8 +141,7 @@ cudaError_t launch_les_z(const CUtensorMap& fmap, const StageArgs<T>& st, const 
   static cudaError_t attr = smem_attr(k, Z::SMEM);
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Z::P - 1) / Z::P, g.ny);
-  k<<<grid, Z::NT, Z::SMEM, s>>>(fmap, st, g, tw, err);
-  return cudaGetLastError();
+  return launch_pdl(k, grid, dim3(Z::NT), Z::SMEM, s, fmap, st, g, tw, err);
 }
 
 template <typename T, int LOGN>
@@ -156,8 +153,7 @@ cudaError_t launch_zfwd_div(const CUtensorMap& fmap, const CUtensorMap& omap, co
   static cudaError_t attr = smem_attr(k, sm);
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Cfg::P - 1) / Cfg::P, g.ny);
-  k<<<grid, ZfCfg<T, LOGN>::NT, sm, s>>>(fmap, omap, da, g, tw, err);
-  return cudaGetLastError();
+  return launch_pdl(k, grid, dim3(ZfCfg<T, LOGN>::NT), sm, s, fmap, omap, da, g, tw, err);
 }
 
 template <typename T, int LOGN, int MODE>
@@ -169,8 +165,7 @@ cudaError_t launch_zfwd_tma_mode(const CUtensorMap& lmap, const CUtensorMap& vma
   static cudaError_t attr = smem_attr(k, sm);
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Cfg::P - 1) / Cfg::P, g.ny);
-  k<<<grid, ZfCfg<T, LOGN>::NT, sm, s>>>(lmap, vmap, vstore, st, g, tw, err);
-  return cudaGetLastError();
+  return launch_pdl(k, grid, dim3(ZfCfg<T, LOGN>::NT), sm, s, lmap, vmap, vstore, st, g, tw, err);
 }
 
 // RK stage 4 (the step's last) in its own instance, the state stored from the
@@ -193,8 +188,7 @@ cudaError_t launch_zfwd_zinv_mode(const CUtensorMap& lmap, const CUtensorMap& fm
   static cudaError_t attr = smem_attr(k, Z::SMEM);
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Z::P - 1) / Z::P, g.ny);
-  k<<<grid, Z::NT, Z::SMEM, s>>>(lmap, fmap, st, fa, g, tw, err);
-  return cudaGetLastError();
+  return launch_pdl(k, grid, dim3(Z::NT), Z::SMEM, s, lmap, fmap, st, fa, g, tw, err);
 }
 
 // one instance per RK stage (the update's mode a compile-time constant;
@@ -230,8 +224,7 @@ cudaError_t launch_zinv_phi(const CUtensorMap& lmap, const CUtensorMap& omap, co
     static cudaError_t attr = smem_attr(k, Z::SMEM);
     if (attr != cudaSuccess) return attr;
     dim3 grid((g.nxh + Z::P - 1) / Z::P, g.ny);
-    k<<<grid, Z::NT, Z::SMEM, s>>>(lmap, omap, za, out, g, tw, err);
-    return cudaGetLastError();
+    return launch_pdl(k, grid, dim3(Z::NT), Z::SMEM, s, lmap, omap, za, out, g, tw, err);
   }
 }
 
@@ -246,8 +239,7 @@ cudaError_t launch_zinv5(const CUtensorMap& vmap, const CUtensorMap& umap, const
     static cudaError_t attr = smem_attr(k, Z::SMEM);
     if (attr != cudaSuccess) return attr;
     dim3 grid((g.nxh + Z::P - 1) / Z::P, g.ny);
-      k<<<grid, Z::NT, Z::SMEM, s>>>(vmap, umap, za, out, g, tw, err);
-    return cudaGetLastError();
+      return launch_pdl(k, grid, dim3(Z::NT), Z::SMEM, s, vmap, umap, za, out, g, tw, err);
   }
 }
 
@@ -259,8 +251,7 @@ cudaError_t launch_xwarp(const FieldList<T>& fin, const FieldList<T>& fout, cons
   static cudaError_t attr = smem_attr(k, Cfg::SMEM_LAUNCH);
   if (attr != cudaSuccess) return attr;
   const long long nb = (xa.rows + Cfg::WARPS - 1) / Cfg::WARPS;
-  k<<<(unsigned)nb, Cfg::NT, Cfg::SMEM_LAUNCH, s>>>(fin, fout, g, twM, twN, xa);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3((unsigned)nb), dim3(Cfg::NT), Cfg::SMEM_LAUNCH, s, fin, fout, g, twM, twN, xa);
 }
 
 template <typename T, int LOGM, int MODE>
@@ -271,8 +262,7 @@ cudaError_t launch_xgroup(const FieldList<T>& fin, const FieldList<T>& fout, con
   static cudaError_t attr = smem_attr(k, Cfg::SMEM);
   if (attr != cudaSuccess) return attr;
   const int per = Cfg::WARPS * GroupFFT<T, LOGM>::RW;
-  k<<<(unsigned)((xa.rows + per - 1) / per), Cfg::NT, Cfg::SMEM, s>>>(fin, fout, g, twM, twN, xa);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3((unsigned)((xa.rows + per - 1) / per)), dim3(Cfg::NT), Cfg::SMEM, s, fin, fout, g, twM, twN, xa);
 }
 
 template <typename T, int LOGM>
@@ -321,8 +311,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
   dim3 grid((g.nxh + AC::P - 1) / AC::P, g.ny);
   const int4 lo = make_int4(fidx[0], fidx[1], fidx[2], fidx[3]);
   const int2 hi = make_int2(fidx[4], fidx[5]);
-  k<<<grid, AC::NT, AC::SMEM, s>>>(pmap, lo, hi, aa, g, tw, err);
-  return cudaGetLastError();
+  return launch_pdl(k, grid, dim3(AC::NT), AC::SMEM, s, pmap, lo, hi, aa, g, tw, err);
 }
 
 }  // namespace sc
@@ -356,8 +345,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
     long long n = (long long)g.ny * g.nz;                                                        \
     int nb = (int)((n + 255) / 256);                                                             \
     if (nb > 4096) nb = 4096;                                                                    \
-    sc::adj_copyT_kernel<T><<<nb, 256, 0, s>>>(lw, g);                                           \
-    return cudaGetLastError();                                                                   \
+    return sc::launch_pdl(sc::adj_copyT_kernel<T>, dim3(nb), dim3(256), 0, s, lw, g);        \
   }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::adj_op(const AdjOpArgs<T>& ao, const Geom& g, cudaStream_t s) {     \
@@ -581,21 +569,18 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
     long long n = (long long)g.ny * g.nz * g.nxh;                                                \
     int nb = (int)((n + 255) / 256);                                                             \
     if (nb > 152 * 16) nb = 152 * 16;                                                            \
-    sc::rot_update_kernel<T><<<nb, 256, 0, s>>>(ra, g);                                          \
-    return cudaGetLastError();                                                                   \
+    return sc::launch_pdl(sc::rot_update_kernel<T>, dim3(nb), dim3(256), 0, s, ra, g);        \
   }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::band_coef(const BandArgs<T>& ba, const Geom& g, cudaStream_t s) {   \
-    sc::band_coef_kernel<T><<<1, 256, 0, s>>>(ba, g);                                            \
-    return cudaGetLastError();                                                                   \
+    return sc::launch_pdl(sc::band_coef_kernel<T>, dim3(1), dim3(256), 0, s, ba, g);        \
   }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::ab2v(const Ab2vArgs<T>& aa, const Geom& g, cudaStream_t s) {        \
     long long n = (long long)g.ny * g.nz * g.nxh;                                                \
     int nb = (int)((n + 255) / 256);                                                             \
     if (nb > 152 * 16) nb = 152 * 16;                                                            \
-    sc::ab2v_update_kernel<T><<<nb, 256, 0, s>>>(aa, g);                                         \
-    return cudaGetLastError();                                                                   \
+    return sc::launch_pdl(sc::ab2v_update_kernel<T>, dim3(nb), dim3(256), 0, s, aa, g);        \
   }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::moments(const C2<T>* d, const Geom& g, double* partial, int nblocks, \

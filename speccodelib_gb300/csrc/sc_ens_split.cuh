@@ -102,6 +102,7 @@ __device__ __forceinline__ void ens_uvw(C2<T>* s, C2<T>* work, const C2<T>* __re
 template <typename T, int LOGN>
 __global__ void __launch_bounds__(EnsSplitCfg<T, LOGN>::NT, EnsSplitCfg<T, LOGN>::MINB)
 ens_yinv_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
+  pdl_wait();
   using Cfg = EnsSplitCfg<T, LOGN>;
   using C = C2<T>;
   constexpr int P = Cfg::P;
@@ -143,6 +144,7 @@ ens_yinv_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
 template <typename T, int LOGN>
 __global__ void __launch_bounds__(EnsSplitCfg<T, LOGN>::NT, EnsSplitCfg<T, LOGN>::MINB)
 ens_yfwd_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
+  pdl_wait();
   using Cfg = EnsSplitCfg<T, LOGN>;
   using E = typename Cfg::Engine;
   using C = C2<T>;
@@ -252,6 +254,7 @@ template <typename T, int LOGM> struct EnsXCfg {
 };
 template <typename T, int LOGM>
 __global__ void __launch_bounds__(EnsXCfg<T, LOGM>::NT, sizeof(T) == 4 ? 4 : 2) ens_xgroup_kernel(EnsClass<T> ec) {
+  pdl_wait();
   using C = C2<T>;
   using Cfg = EnsXCfg<T, LOGM>;
   using GF = GroupFFT<T, LOGM>;
@@ -278,6 +281,7 @@ __global__ void __launch_bounds__(EnsXCfg<T, LOGM>::NT, sizeof(T) == 4 ? 4 : 2) 
 }
 // M = 512: a warp per row (ens_xrow)
 template <typename T> __global__ void __launch_bounds__(256, 2) ens_xwarp_kernel(EnsClass<T> ec) {
+  pdl_wait();
   using C = C2<T>;
   using WF = WarpFFT<T, 9>;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -315,18 +319,21 @@ template <typename T, int LOGN> cudaError_t ens_split_stage_n(const CUtensorMap&
   const int ntx = (ec.nxh + Cfg::P - 1) / Cfg::P;
   if (ec.stage == 1) {
     const int total = ntx * ec.count, most = 2 * ec.nsm;
-    ens_yinv_kernel<T, LOGN><<<total < most ? total : most, Cfg::NT, Cfg::SMEM_INV, s>>>(map, ec);
+    const cudaError_t e = launch_pdl(ens_yinv_kernel<T, LOGN>, dim3(total < most ? total : most), dim3(Cfg::NT), Cfg::SMEM_INV, s, map, ec);
+    if (e != cudaSuccess) return e;
   }
   const long long rows = (long long)ec.count * ec.n;
   if constexpr (LOGN == 10) {
-    ens_xwarp_kernel<T><<<(unsigned)((rows + 7) / 8), 256, sx9, s>>>(ec);
+    const cudaError_t e = launch_pdl(ens_xwarp_kernel<T>, dim3((unsigned)((rows + 7) / 8)), dim3(256), sx9, s, ec);
+    if (e != cudaSuccess) return e;
   } else {
     using X = EnsXCfg<T, LOGN - 1>;
     const int per = X::WARPS * GroupFFT<T, LOGN - 1>::RW;
-    ens_xgroup_kernel<T, LOGN - 1><<<(unsigned)((rows + per - 1) / per), X::NT, X::SMEM, s>>>(ec);
+    const cudaError_t e =
+        launch_pdl(ens_xgroup_kernel<T, LOGN - 1>, dim3((unsigned)((rows + per - 1) / per)), dim3(X::NT), X::SMEM, s, ec);
+    if (e != cudaSuccess) return e;
   }
-  ens_yfwd_kernel<T, LOGN><<<dim3(ntx, ec.count), Cfg::NT, Cfg::SMEM_FWD, s>>>(map, ec);
-  return cudaGetLastError();
+  return launch_pdl(ens_yfwd_kernel<T, LOGN>, dim3(ntx, ec.count), dim3(Cfg::NT), Cfg::SMEM_FWD, s, map, ec);
 }
 
 // sc_ens_split_*.cu

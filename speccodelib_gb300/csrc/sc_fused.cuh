@@ -338,6 +338,7 @@ template <typename T, int LOGN, int MODE>
 __global__ void __launch_bounds__(ZiCfg<T, LOGN>::NT, ZiCfg<T, LOGN>::MINB)
 zinv5_tma_kernel(const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap umap, ZvArgs<T> za,
                  FieldList<T> out, Geom g, const C2<T>* __restrict__ tw, int* err) {
+  pdl_wait();
   using Z = ZiCfg<T, LOGN>;
   using Cfg = TmaCfg<T, LOGN>;
   using C = C2<T>;
@@ -398,6 +399,7 @@ template <typename T, int LOGN>
 __global__ void __launch_bounds__(ZiCfg<T, LOGN>::NT, ZiCfg<T, LOGN>::MINB)
 zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap omap, ZvArgs<T> za,
                     FieldList<T> out, Geom g, const C2<T>* __restrict__ tw, int* err) {
+  pdl_wait();
   using Z = ZiCfg<T, LOGN>;
   using Cfg = TmaCfg<T, LOGN>;
   using EF = typename Z::EngF;
@@ -497,6 +499,7 @@ template <typename T, int LOGN, int MODE>
 __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(ZiCfg<T, LOGN>::NT, ZiCfg<T, LOGN>::MINB)
 zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap fmap,
                      StageArgs<T> st, FusedArgs<T> fa, Geom g, const C2<T>* __restrict__ tw, int* err) {
+  pdl_wait();
   using Z = ZiCfg<T, LOGN>;
   using Cfg = TmaCfg<T, LOGN>;
   using EF = typename Z::EngF;

@@ -42,6 +42,7 @@ template <typename T, int LOGN> struct LesYCfg {
 template <typename T, int LOGN>
 __global__ void __launch_bounds__(TmaCfg<T, LOGN>::NT, 2)
 les_yinv_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, const C2<T>* __restrict__ tw) {
+  pdl_wait();
   using Cfg = TmaCfg<T, LOGN>;
   using E = typename Cfg::Engine;
   using C = C2<T>;
@@ -115,6 +116,7 @@ les_yinv_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, 
 template <typename T, int LOGN>
 __global__ void __launch_bounds__(TmaCfg<T, LOGN>::NT, 2)
 les_yfwd_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, const C2<T>* __restrict__ tw) {
+  pdl_wait();
   using Cfg = TmaCfg<T, LOGN>;
   using E = FFTEngine<T, LOGN, Cfg::P, Cfg::P, Cfg::NT, true, 0, true>;
   using C = C2<T>;
@@ -227,6 +229,7 @@ template <typename T, int LOGN, int MODE>
 __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(LesZCfg<T, LOGN>::NT, LesZCfg<T, LOGN>::MINB)
 les_zfwd_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st, Geom g, const C2<T>* __restrict__ tw,
                 int* err) {
+  pdl_wait();
   using Z = LesZCfg<T, LOGN>;
   using Cfg = TmaCfg<T, LOGN>;
   using E = typename Z::Engine;

@@ -8,6 +8,7 @@
 // (specdns-forced-omp-ft.f90:142-176).  All sums are accumulated in double.
 #pragma once
 #include "sc_passes.cuh"
+#include "sc_tma.cuh"
 #include "sc_rot.cuh"
 #include "sc_ab2v.cuh"
 
@@ -384,6 +385,7 @@ template <typename T> struct BandArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) band_coef_kernel(BandArgs<T> ba, Geom g) {
+  pdl_wait();
   __shared__ double red[256 / 32 + 1];
   const int lo_b = k2_lt(ba.lo2), hi_b = k2_lt(ba.hi2);
   int kb = 0;
@@ -437,6 +439,7 @@ template <typename T> struct RotArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) rot_update_kernel(RotArgs<T> ra, Geom g) {
+  pdl_wait();
   using C = C2<T>;
   const long long rows = (long long)g.ny * g.nz;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -520,6 +523,7 @@ template <typename T> struct Ab2vArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) ab2v_update_kernel(Ab2vArgs<T> aa, Geom g) {
+  pdl_wait();
   using C = C2<T>;
   const long long rows = (long long)g.ny * g.nz;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;

@@ -123,6 +123,32 @@ __device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int c0, 
                : "memory");
 }
 
+// Programmatic dependent launch.  A step is a chain of kernels that each need
+// the whole of the one before; on small grids the gaps between them weigh.  A
+// kernel launched by launch_pdl is set up while its predecessor drains and
+// calls pdl_wait first, which returns once the predecessor has completed and
+// its writes are visible (no effect under a plain launch).  Ten 64^3 FP32 steps
+// 1.42 -> 1.37 ms, ten dynamic LES steps at 128^3 9.52 -> 9.08 ms.  Kernels do
+// not trigger their successors early: its CTAs then hold slots while they wait
+// (64^3 1.71 ms, 512^3 46.4 -> 51.7 ms).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Launch of a kernel that calls pdl_wait before any global access.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                              const Args&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+}
+
 // Barrier over the CTAs of a cluster (release / acquire, every thread).
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");

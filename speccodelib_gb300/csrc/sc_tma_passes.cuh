@@ -129,6 +129,7 @@ __device__ __forceinline__ void tma_issue_tile(void* dst, const CUtensorMap* map
 template <typename T, int LOGN, bool INV>
 __global__ void __launch_bounds__(TmaCfg<T, LOGN>::NT, TmaCfg<T, LOGN>::PB)
 pencil_tma_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, const C2<T>* __restrict__ tw) {
+  pdl_wait();
   using Cfg = TmaCfg<T, LOGN>;
   // stage-0 writes XOR-rotated (conflict-free 64-byte rows) in the forward
   // pass only: measured 4% faster there, 3% slower in the inverse pass
@@ -406,6 +407,7 @@ template <typename T, int LOGN, int MODE>
 __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(ZfCfg<T, LOGN>::NT, 2)
 zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap vmap, int vstore,
                 StageArgs<T> st, Geom g, const C2<T>* __restrict__ tw, int* err) {
+  pdl_wait();
   using Cfg = TmaCfg<T, LOGN>;
   using E = typename ZfCfg<T, LOGN>::Engine;
   using C = C2<T>;
@@ -500,6 +502,7 @@ template <typename T, int LOGN>
 __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(ZfCfg<T, LOGN>::NT, 2)
 zfwd_div_tma_kernel(const __grid_constant__ CUtensorMap fmap, const __grid_constant__ CUtensorMap omap, DivArgs<T> da,
                     Geom g, const C2<T>* __restrict__ tw, int* err) {
+  pdl_wait();
   using Cfg = TmaCfg<T, LOGN>;
   using E = typename ZfCfg<T, LOGN>::Engine;
   using C = C2<T>;

@@ -472,6 +472,7 @@ template <typename T, int LOGM, int MODE>
 __global__ void __launch_bounds__(XgCfg<T, LOGM, MODE>::NT, XgCfg<T, LOGM, MODE>::MINB)
 xpass_group_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __restrict__ twM,
                    const C2<T>* __restrict__ twN, XArgs<T> xa) {
+  pdl_wait();
   using C = C2<T>;
   using Cfg = XgCfg<T, LOGM, MODE>;
   extern __shared__ __align__(16) unsigned char smraw[];

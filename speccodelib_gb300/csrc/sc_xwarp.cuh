@@ -838,6 +838,7 @@ template <typename T, int LOGM, int MODE>
 __global__ void __launch_bounds__(XwCfg<T, LOGM, MODE>::NT, XwCfg<T, LOGM, MODE>::MINB)
 xpass_warp_kernel(FieldList<T> fin, FieldList<T> fout, Geom g, const C2<T>* __restrict__ twM,
                   const C2<T>* __restrict__ twN, XArgs<T> xa) {
+  pdl_wait();
   using C = C2<T>;
   using Cfg = XwCfg<T, LOGM, MODE>;
   using Row = XwRow<T, LOGM, Cfg::TM>;
