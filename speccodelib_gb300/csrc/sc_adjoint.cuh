@@ -33,12 +33,13 @@ template <typename T> struct AdjArgs {
   const T* ez;
   T dt;
   int forced;
-  double fkmax2, eps;
+  K2Lt fkmax2;
+  double eps;
   const double* kf_partial;
   const double* c_partial;
   int kf_tiles, kf_ptile;
   int mask_rhs;
-  double kcut2;
+  K2Lt kcut2;
   // stage 1 only: chain = also start the previous step's adjoint (its masked
   // lam into lt_next, dt/6 of it into lw, what a separate init pass would
   // write); write_lam = store lam itself (the last step: the gradient)
@@ -96,7 +97,7 @@ __device__ __forceinline__ void adj_accum(C2<T> (&l)[E::JL][E::RL][3], const C2<
 template <typename E, typename T>
 __device__ __forceinline__ void adj_epilogue(C2<T> (&l)[E::JL][E::RL][3], const AdjArgs<T>& aa, const Geom& g,
                                              int kx0, int iy, int nvalid, long long base, long long zstride,
-                                             bool fblock, double s_a, double s_b) {
+                                             bool fblock, T s_a, T s_b) {
   using C = C2<T>;
   constexpr int NP = E::JL * E::RL;
   constexpr int B = 2;
@@ -106,7 +107,7 @@ __device__ __forceinline__ void adj_epilogue(C2<T> (&l)[E::JL][E::RL][3], const 
   C* __restrict__ lam[3] = {aa.lam[0], aa.lam[1], aa.lam[2]};
   const int stage = aa.stage;
   const T dt = aa.dt;
-  const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(aa.fkmax2), kc_b = k2_lt(aa.kcut2);
+  const int kyi = wavenum(iy, g.ny), fk_b = aa.fkmax2.b, kc_b = aa.kcut2.b;
 #pragma unroll
   for (int q0 = 0; q0 < NP; q0 += B) {
     long long idx[B];
@@ -140,7 +141,7 @@ __device__ __forceinline__ void adj_epilogue(C2<T> (&l)[E::JL][E::RL][3], const 
         if (k2i < fk_b) {
           C m[3] = {lw[0][idx[b]], lw[1][idx[b]], lw[2][idx[b]]};
           adj_mu<C, T>(m, ix, iy, iz, g, aa.mask_rhs, kc_b);
-          const T sa = (T)s_a, sb = (T)(ix == 0 ? 0.5 * s_b : s_b);
+          const T sa = s_a, sb = ix == 0 ? T(0.5) * s_b : s_b;
 #pragma unroll
           for (int c = 0; c < 3; ++c)
             ls[c] = cadd(ls[c], csub(cscale(m[c], sa), cscale(aa.s[c][idx[b]], sb)));
@@ -188,15 +189,17 @@ __device__ __forceinline__ void adj_epilogue(C2<T> (&l)[E::JL][E::RL][3], const 
   }
 }
 
-// Band coefficients of the forcing adjoint (thread 0): a = eps / (2 K_f),
-// b = 2 a c / K_f.
+// Band coefficients of the forcing adjoint (one warp; lane 0 writes): a = eps /
+// (2 K_f), b = 2 a c / K_f.
 template <typename T>
-__device__ __forceinline__ void adj_band_coef(const AdjArgs<T>& aa, const Geom& g, double& s_a, double& s_b) {
-  const double kf = forcing_energy(aa.kf_partial, aa.kf_tiles, aa.kf_ptile, g.ny, aa.fkmax2);
-  const double cc = forcing_energy(aa.c_partial, aa.kf_tiles, aa.kf_ptile, g.ny, aa.fkmax2);
-  const double a = aa.eps / (2.0 * kf);
-  s_a = a;
-  s_b = 2.0 * a * cc / kf;
+__device__ __forceinline__ void adj_band_coef(const AdjArgs<T>& aa, const Geom& g, T& s_a, T& s_b) {
+  const double kf = warp_sum(forcing_energy_lane(aa.kf_partial, aa.kf_tiles, aa.kf_ptile, g.ny, aa.fkmax2.b));
+  const double cc = warp_sum(forcing_energy_lane(aa.c_partial, aa.kf_tiles, aa.kf_ptile, g.ny, aa.fkmax2.b));
+  if ((threadIdx.x & 31) == 0) {
+    const double a = aa.eps / (2.0 * kf);
+    s_a = (T)a;
+    s_b = (T)(2.0 * a * cc / kf);
+  }
 }
 
 template <typename T, int LOGN>
@@ -208,7 +211,7 @@ zfwd_adj_kernel(FieldList<T> fin, AdjArgs<T> aa, Geom g, const C2<T>* __restrict
   constexpr int P = Cfg::P;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
-  __shared__ double s_a, s_b;
+  __shared__ T s_a, s_b;
   const int kx0 = blockIdx.x * P;
   const int iy = blockIdx.y;
   const int nvalid = min(P, g.nxh - kx0);
@@ -235,14 +238,9 @@ zfwd_adj_kernel(FieldList<T> fin, AdjArgs<T> aa, Geom g, const C2<T>* __restrict
     E::template run<false>(in, o, sm, tw);
     adj_accum<E, T>(l, o, f, kx0, ky, g);
   }
-  const bool fblock = aa.forced && ((double)kx0 * kx0 + (double)ky * ky < aa.fkmax2);
+  const bool fblock = aa.forced && kx0 * kx0 + wavenum(iy, g.ny) * wavenum(iy, g.ny) < aa.fkmax2.b;
   if (fblock) {
-    if (threadIdx.x == 0) {
-      double a, b;
-      adj_band_coef<T>(aa, g, a, b);
-      s_a = a;
-      s_b = b;
-    }
+    if (threadIdx.x < 32) adj_band_coef<T>(aa, g, s_a, s_b);
     __syncthreads();
   }
   adj_epilogue<E, T>(l, aa, g, kx0, iy, nvalid, base, zstride, fblock, s_a, s_b);
@@ -286,7 +284,7 @@ zfwd_adj_tma_kernel(const __grid_constant__ CUtensorMap pmap, int4 fidx_lo, int2
   unsigned char* smraw = align128(smdyn);
   C* buf[2] = {reinterpret_cast<C*>(smraw), reinterpret_cast<C*>(smraw + AC::TILE_BYTES)};
   __shared__ __align__(8) uint64_t bars[2];
-  __shared__ double s_a, s_b;
+  __shared__ T s_a, s_b;
   const int kx0 = blockIdx.x * P;
   const int iy = blockIdx.y;
   const int nvalid = min(P, g.nxh - kx0);
@@ -301,7 +299,7 @@ zfwd_adj_tma_kernel(const __grid_constant__ CUtensorMap pmap, int4 fidx_lo, int2
       tma_load_4d(reinterpret_cast<char*>(buf[f & 1]) + (size_t)h * Cfg::BOX * P * sizeof(C), &pmap, &bars[f & 1],
                   kx0 * Cfg::U, iy, h * Cfg::BOX, fidx[f]);
   };
-  const bool fblock = aa.forced && ((double)kx0 * kx0 + (double)ky * ky < aa.fkmax2);
+  const bool fblock = aa.forced && kx0 * kx0 + wavenum(iy, g.ny) * wavenum(iy, g.ny) < aa.fkmax2.b;
   if (threadIdx.x == 0) {
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
@@ -309,13 +307,8 @@ zfwd_adj_tma_kernel(const __grid_constant__ CUtensorMap pmap, int4 fidx_lo, int2
     fence_proxy_async();
     issue(0);
     issue(1);
-    if (fblock) {
-      double a, b;
-      adj_band_coef<T>(aa, g, a, b);
-      s_a = a;
-      s_b = b;
-    }
   }
+  if (fblock && threadIdx.x >= AC::NT - 32) adj_band_coef<T>(aa, g, s_a, s_b);
   __syncthreads();
   C l[E::JL][E::RL][3];
 #pragma unroll
@@ -371,7 +364,7 @@ template <typename T> struct AdjOpArgs {
   C2<T>* out1[3];
   C2<T>* out2[3];
   T dt;
-  double kcut2;
+  K2Lt kcut2;
   int kmin, kmax;
 };
 
@@ -379,7 +372,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) adj_op_kernel(AdjOpArgs<T> ao, Geom g) {
   using C = C2<T>;
   const long long total = (long long)g.ny * g.nz * g.nxh;
-  const int kc_b = k2_lt(ao.kcut2);
+  const int kc_b = ao.kcut2.b;
   for (Walk3 w(blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x, total, g.nxh,
                g.ny);
        w.ok(); w.next()) {

@@ -84,6 +84,14 @@ __host__ __device__ inline int k2_clamp(double b) {
   return b >= 2147483647.0 ? 2147483647 : (b <= -2147483647.0 ? -2147483647 : (int)b);
 }
 __host__ __device__ inline int k2_lt(double t) { return k2_clamp(ceil(t)); }
+// A kernel argument's bound, made an integer where the host assigns it: formed
+// by every thread of a short kernel from a double, the bounds alone took 2 to 3
+// us of a z pass at 64^3.
+struct K2Lt {   // k2 < t  <=>  k2 < b
+  int b;
+  K2Lt() = default;
+  K2Lt(double t) : b(k2_lt(t)) {}
+};
 
 // floor(sqrt(k2) + 1/2) for an integer k2 >= 0, exactly: the n with
 // n^2 - n < k2 <= n^2 + n (a float root is within one of it).

@@ -165,7 +165,7 @@ cudaError_t launch_zfwd_tma_mode(const CUtensorMap& lmap, const CUtensorMap& vma
   static cudaError_t attr = smem_attr(k, sm);
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + Cfg::P - 1) / Cfg::P, g.ny);
-  return launch_pdl(k, grid, dim3(ZfCfg<T, LOGN>::NT), sm, s, lmap, vmap, vstore, st, g, tw, err);
+  return launch_pdl(k, grid, dim3(ZfCfg<T, LOGN>::NTF), sm, s, lmap, vmap, vstore, st, g, tw, err);
 }
 
 // RK stage 4 (the step's last) in its own instance, the state stored from the

@@ -147,7 +147,7 @@ template <int R, bool INV, typename C> __device__ __forceinline__ void dft(C* v)
 }
 
 template <typename T, int LOGN, int P, int PS, int NT, bool PFAST, int PADSHIFT = 0, bool ROTATE = false,
-          int RMAX = 8>
+          int RMAX = 8, bool GROUPED = false>
 struct FFTEngine {
   using C = C2<T>;
   static constexpr int N = 1 << LOGN;
@@ -158,6 +158,14 @@ struct FFTEngine {
   static constexpr int TOTL = P * (N / RL);
   static constexpr int J1 = (TOT1 + NT - 1) / NT;
   static constexpr int JL = (TOTL + NT - 1) / NT;
+  // GROUPED: NT threads are one of several groups of a CTA, each with a
+  // transform of its own and barrier 1 + group for its stages (NT a multiple
+  // of 32 and a power of two).
+  __device__ static __forceinline__ int tid() { return GROUPED ? threadIdx.x % NT : threadIdx.x; }
+  __device__ static __forceinline__ void sync() {
+    if constexpr (GROUPED) asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / NT), "n"(NT) : "memory");
+    else __syncthreads();
+  }
   // Shared-memory slot of point n.  With PADSHIFT = s one slot is skipped
   // every 2^s points, which spreads the stride-R scatter of the first stage
   // over all banks: s = 4 keeps both that scatter and 16-wide contiguous
@@ -180,14 +188,14 @@ struct FFTEngine {
   }
   // Position of in[a][r]; returns false for padding jobs.
   __device__ static __forceinline__ bool in_pos(int a, int r, int& p, int& n) {
-    int job = threadIdx.x + a * NT, j;
+    int job = tid() + a * NT, j;
     decode<R1>(job, p, j);
     n = j + r * (N / R1);
     return (TOT1 % NT == 0) || job < TOT1;
   }
   // Position of out[a][r]; returns false for padding jobs.
   __device__ static __forceinline__ bool out_pos(int a, int r, int& p, int& n) {
-    int job = threadIdx.x + a * NT, j;
+    int job = tid() + a * NT, j;
     decode<RL>(job, p, j);
     n = j + r * (N / RL);
     return (TOTL % NT == 0) || job < TOTL;
@@ -274,7 +282,7 @@ struct FFTEngine {
     C v[J][R], w[TW_EARLY && NSV > 1 ? J : 1][R];
 #pragma unroll
     for (int a = 0; a < J; ++a) {
-      int job = threadIdx.x + a * NT, p, j;
+      int job = tid() + a * NT, p, j;
       decode<R>(job, p, j);
       if ((TOT % NT == 0) || job < TOT) {
 #pragma unroll
@@ -282,10 +290,10 @@ struct FFTEngine {
         if constexpr (TW_EARLY && NSV > 1) twiddle_load<R, NSV>(w[a], j % NSV, tw);
       }
     }
-    __syncthreads();
+    sync();
 #pragma unroll
     for (int a = 0; a < J; ++a) {
-      int job = threadIdx.x + a * NT, p, j;
+      int job = tid() + a * NT, p, j;
       decode<R>(job, p, j);
       if ((TOT % NT == 0) || job < TOT) {
         const int k = j % NSV;
@@ -301,7 +309,7 @@ struct FFTEngine {
         }
       }
     }
-    __syncthreads();
+    sync();
   }
 
   template <int S, bool INV>
@@ -329,7 +337,7 @@ struct FFTEngine {
     C w[TW_EARLY && NSV > 1 ? JL : 1][RL];
 #pragma unroll
     for (int a = 0; a < JL; ++a) {
-      int job = threadIdx.x + a * NT, p, j;
+      int job = tid() + a * NT, p, j;
       decode<RL>(job, p, j);
       if ((TOTL % NT == 0) || job < TOTL) {
 #pragma unroll
@@ -337,10 +345,10 @@ struct FFTEngine {
         if constexpr (TW_EARLY && NSV > 1) twiddle_load<RL, NSV>(w[a], j, tw);
       }
     }
-    __syncthreads();
+    sync();
 #pragma unroll
     for (int a = 0; a < JL; ++a) {
-      int job = threadIdx.x + a * NT, p, j;
+      int job = tid() + a * NT, p, j;
       decode<RL>(job, p, j);
       if ((TOTL % NT == 0) || job < TOTL) {
         if constexpr (TW_EARLY && NSV > 1) twiddle_apply<RL, NSV, INV>(out[a], w[a]);
@@ -371,7 +379,7 @@ struct FFTEngine {
     };
 #pragma unroll
     for (int a = 0; a < J1; ++a) {
-      int job = threadIdx.x + a * NT, p, j;
+      int job = tid() + a * NT, p, j;
       decode<R1>(job, p, j);
       if ((TOT1 % NT == 0) || job < TOT1) {
         if constexpr (NS == 1) {
@@ -385,7 +393,7 @@ struct FFTEngine {
         }
       }
     }
-    __syncthreads();
+    sync();
     if constexpr (NS > 1) {
       mid_stages<1, INV>(sm, tw);
       last_stage<INV>(out, sm, tw);
@@ -420,7 +428,7 @@ struct FFTEngine {
   // return (the names say 512; N = 256 uses them too).
   template <bool INV>
   __device__ static __forceinline__ void phase1_512(C (&v)[16], const C* __restrict__ tw) {
-    const int j = threadIdx.x / P;
+    const int j = tid() / P;
     dft16<INV>(v);
 #pragma unroll
     for (int k1 = 1; k1 < 16; ++k1) {
@@ -434,25 +442,25 @@ struct FFTEngine {
   // transform in sm in natural order.  Ends with a barrier.
   template <bool INV>
   __device__ static __forceinline__ void finish_512(C (&v)[16], C* sm, const C* __restrict__ tw) {
-    const int t = threadIdx.x;
+    const int t = tid();
     const int p = t % P, j = t / P;
     if constexpr (LOGN == 8) {
 #pragma unroll
       for (int k1 = 0; k1 < 16; ++k1) sm[(k1 * 16 + j) * PS + p] = v[k1];
-      __syncthreads();
+      sync();
       // thread (p, k1 = j): the 16-point DFT over the exchange row's j
 #pragma unroll
       for (int m = 0; m < 16; ++m) v[m] = sm[(j * 16 + m) * PS + p];
       dft16<INV>(v);
-      __syncthreads();
+      sync();
 #pragma unroll
       for (int k2 = 0; k2 < 16; ++k2) sm[(j + 16 * k2) * PS + p] = v[k2];
-      __syncthreads();
+      sync();
       return;
     }
 #pragma unroll
     for (int k1 = 0; k1 < 16; ++k1) sm[(k1 * 32 + (j ^ (k1 & 1))) * PS + p] = v[k1];
-    __syncthreads();
+    sync();
     const int k1 = (j & 1) | ((j >> 2) << 1), e = (j >> 1) & 1;
 #pragma unroll
     for (int m = 0; m < 16; ++m) v[m] = sm[(k1 * 32 + ((2 * m + e) ^ (k1 & 1))) * PS + p];
@@ -463,7 +471,7 @@ struct FFTEngine {
       const C w = __ldg(&tw[16 * k * e]);
       v[k] = INV ? cmulc(v[k], w) : cmul(v[k], w);
     }
-    __syncthreads();
+    sync();
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       // e = 0: keeps A_0[i], sends A_0[8 + i], gets W A_1[i];
@@ -478,18 +486,18 @@ struct FFTEngine {
       sm[(k1 + 16 * kp) * PS + p] = cadd(a0, b);
       sm[(k1 + 16 * (kp + 16)) * PS + p] = csub(a0, b);
     }
-    __syncthreads();
+    sync();
   }
 
   template <bool INV>
   __device__ static void inplace_512(C* sm, const C* __restrict__ tw) {
-    const int t = threadIdx.x;
+    const int t = tid();
     const int p = t % P, j = t / P;
     C v[16];
 #pragma unroll
     for (int m = 0; m < 16; ++m) v[m] = sm[(j + S1 * m) * PS + p];
     phase1_512<INV>(v, tw);
-    __syncthreads();
+    sync();
     finish_512<INV>(v, sm, tw);
   }
 
@@ -504,6 +512,24 @@ struct FFTEngine {
     }
 #endif
     all_stages<0, INV>(sm, tw);
+  }
+
+  // Stage 0 of the transform of f(p, n) into the tile sm (no barrier):
+  // all_stages<1> finishes it in place.
+  template <bool INV, class F>
+  __device__ static __forceinline__ void stage0_map(C* sm, F&& f) {
+#pragma unroll
+    for (int a = 0; a < J1; ++a) {
+      int job = tid() + a * NT, p, j;
+      decode<R1>(job, p, j);
+      if ((TOT1 % NT == 0) || job < TOT1) {
+        C v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; ++r) v[r] = f(p, j + r * (N / R1));
+        dft<R1, INV>(v);
+        store_stage0<R1>(v, sm, j, p);
+      }
+    }
   }
 
   // Full transform: registers (first-stage layout) -> registers (last-stage
@@ -521,14 +547,14 @@ struct FFTEngine {
       // stage 0: registers -> shared (Ns = 1, no twiddles)
 #pragma unroll
       for (int a = 0; a < J1; ++a) {
-        int job = threadIdx.x + a * NT, p, j;
+        int job = tid() + a * NT, p, j;
         decode<R1>(job, p, j);
         if ((TOT1 % NT == 0) || job < TOT1) {
           dft<R1, INV>(in[a]);
           store_stage0<R1>(in[a], sm, j, p);
         }
       }
-      __syncthreads();
+      sync();
       mid_stages<1, INV>(sm, tw);
       last_stage<INV>(out, sm, tw);
     }

@@ -44,23 +44,23 @@ template <typename T, int LOGN> struct ZiCfg {
   // measured slower: 32-byte row segments)
   static constexpr int P = Cfg::P;
   static constexpr int N = Cfg::N;
-  // two points per thread and radix-8 job at most 256 threads (ZI_DIV 16,
-  // ZI_MAX 256), or one job per thread up to 512 (ZI_DIV 8, ZI_MAX 512)
+  using ZG = ZgCfg<T, LOGN>;
+  static constexpr bool GROUPED = ZG::ON;   // three groups of threads (ZgCfg), six tiles
+  // else two jobs per thread, at most 256 threads (ZI_DIV 16, ZI_MAX 256), or
+  // one job per thread up to 512 (ZI_DIV 8, ZI_MAX 512)
   static constexpr int NT_RAW = P * N / ZI_DIV;
-  static constexpr int NT = NT_RAW > ZI_MAX ? ZI_MAX : (NT_RAW < 32 ? 32 : NT_RAW);
-#ifndef SC_ZI_EB
-  static constexpr int EB = NT >= 512 ? 2 : 4;   // epilogue batch
-#else
-  static constexpr int EB = SC_ZI_EB;
-#endif
+  static constexpr int NT = GROUPED ? ZG::NT : (NT_RAW > ZI_MAX ? ZI_MAX : (NT_RAW < 32 ? 32 : NT_RAW));
+  static constexpr int EB = GROUPED ? 3 : (NT >= 512 ? 2 : 4);   // epilogue batch
   using EngF = FFTEngine<T, LOGN, P, P, NT, true, 0, true>;           // whole tile, in place
   using EngH = FFTEngine<T, LOGN, P / 2, P / 2, NT, true, 0, true>;   // half tile
   static constexpr size_t TILE = sizeof(C2<T>) * (size_t)N * P;
-  static constexpr size_t SMEM = 3 * TILE + TILE / 2 + kSmemAlignPad;
+  static constexpr size_t SMEM = (GROUPED ? 6 * TILE : 3 * TILE + TILE / 2) + kSmemAlignPad;
   static constexpr bool SUPPORTED = P >= 2 && SMEM <= 113 * 1024;
-  // CTAs per SM that the shared memory allows (228 KB, 1 KB reserved per CTA)
+  // CTAs per SM that the shared memory allows (228 KB, 1 KB reserved per CTA);
+  // two of the grouped form (one: 128^3 FP32 step 396 -> 433 us)
   static constexpr int MINB_RAW = (int)(233472 / (SMEM + 1024));
-  static constexpr int MINB = MINB_RAW > 4 ? 4 : (MINB_RAW < 1 ? 1 : MINB_RAW);
+  static constexpr int MINB_MAX = GROUPED ? 2 : 4;
+  static constexpr int MINB = MINB_RAW > MINB_MAX ? MINB_MAX : (MINB_RAW < 1 ? 1 : MINB_RAW);
 };
 
 // The outputs of the z-inverse that carry kz, transformed half a tile at a
@@ -115,7 +115,49 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
   constexpr int NT = Z::NT;
   constexpr int PH = P / 2;
   using ZF = ZiFields<MODE>;
+  using Cfg = TmaCfg<T, LOGN>;
   const T ky = (T)wavenum(iy, g.ny);
+  // Short pencils: group c forms w_c (or d/dz u_c) into a tile of its own, then
+  // u_c in place; all six leave by bulk stores.
+  if constexpr (Z::GROUPED && (MODE == ZV_DNS || MODE == ZV_GRAD)) {
+    if (umap) {
+      using ZG = typename Z::ZG;
+      using EG = typename ZG::Engine;
+      static_assert(TmaCfg<T, LOGN>::NBOX == 1, "one box per tile");
+      constexpr int TE = P * N;
+      const int c = threadIdx.x / ZG::NTG;   // this group's component
+      const bool first = threadIdx.x % ZG::NTG == 0;
+      C* const ut = rt[0] + (size_t)c * TE;   // the tiles are contiguous
+      C* const dt = work + (size_t)c * TE;
+      auto store = [&](const C* tile, int f) {
+        fence_proxy_async();
+        EG::sync();
+        if (first) {
+          tma_store_4d(umap, tile, kx0 * Cfg::U, iy, 0, f);
+          tma_store_commit();
+        }
+      };
+      if constexpr (MODE == ZV_GRAD) {
+        EG::template stage0_map<true>(dt, [&](int p, int n) { return cmuli(cscale(ut[n * P + p], (T)wavenum(n, g.nz))); });
+      } else {   // w_c = i (k_a s_b - k_b s_a)
+        const C* const sa = rt[0] + (size_t)(c == 2 ? 0 : c + 1) * TE;
+        const C* const sb = rt[0] + (size_t)(c == 0 ? 2 : c - 1) * TE;
+        EG::template stage0_map<true>(dt, [&](int p, int n) {
+          const T kx = (T)(kx0 + p), kz = (T)wavenum(n, g.nz);
+          const T ka = c == 0 ? ky : (c == 1 ? kz : kx), kb = c == 0 ? kz : (c == 1 ? kx : ky);
+          return cmuli(csub(cscale(sb[n * P + p], ka), cscale(sa[n * P + p], kb)));
+        });
+      }
+      __syncthreads();
+      EG::template run_inplace<true>(ut, tw);
+      store(ut, c);
+      EG::template all_stages<1, true>(dt, tw);
+      store(dt, 3 + c);
+      if (first) tma_store_wait_read<0>();
+      __syncthreads();
+      return;
+    }
+  }
 #ifndef SC_NO_TMEM_W
   // FP32 512- and 256-point pencils with bulk stores: w_x and w_y as whole-tile
   // two-pass transforms.  Each thread forms its 16 step-1 points of both
@@ -127,7 +169,6 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
   // ZV_GRAD: the same with the three d/dz u parked; u leaves, d/dz u follows.
   if constexpr ((MODE == ZV_DNS || MODE == ZV_GRAD) && EF::TWO_PASS && sizeof(T) == 4) {
     if (umap) {
-      using Cfg = TmaCfg<T, LOGN>;
       constexpr int NQ = MODE == ZV_GRAD ? 3 : 2;            // fields parked, 32 columns each
       constexpr int COLS = MODE == ZV_GRAD ? 256 : 128;      // per CTA: two warps per lane quarter
       __shared__ uint32_t s_tmem;
@@ -258,7 +299,6 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
 #endif
   if (umap && MODE != ZV_DNS) {
     // u by bulk stores; the pointwise outputs from the tiles while they drain
-    using Cfg = TmaCfg<T, LOGN>;
     fence_proxy_async();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -281,7 +321,6 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
     return;
   }
   if (umap) {
-    using Cfg = TmaCfg<T, LOGN>;
     auto store = [&](int c, int f) {
       for (int h = 0; h < Cfg::NBOX; ++h)
         tma_store_4d(umap, rt[c] + (size_t)h * Cfg::BOX * P, kx0 * Cfg::U, iy, h * Cfg::BOX, f);
@@ -358,7 +397,7 @@ zinv5_tma_kernel(const __grid_constant__ CUtensorMap vmap, const __grid_constant
   const long long zstride = (long long)g.ny * g.nxp;
   const long long base = (long long)iy * g.nxp + kx0;
   const T ky = (T)wavenum(iy, g.ny);
-  if (launch_failed(err)) return;
+  const bool failed = launch_failed(err);
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init();
@@ -370,11 +409,11 @@ zinv5_tma_kernel(const __grid_constant__ CUtensorMap vmap, const __grid_constant
                     kx0 * Cfg::U, iy, h * Cfg::BOX, c);
   }
   __syncthreads();
-  if (!mbar_wait_bounded(&bar, 0, err)) return;
+  if (!__syncthreads_and(mbar_wait_bounded(&bar, 0, err) && !failed)) return;
   // forcing band energy of the stage input (force.f90:16-22), FP64
-  if (za.fs.enabled && ((double)kx0 * kx0 + (double)ky * ky < za.fs.fkmax2)) {
+  const int kyi = wavenum(iy, g.ny), fk_b = za.fs.fkmax2.b;
+  if (za.fs.enabled && kx0 * kx0 + kyi * kyi < fk_b) {
     double q = 0.0;
-    const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(za.fs.fkmax2);
     for (int e = threadIdx.x; e < P * N; e += NT) {
       const int p = e % P, n = e / P;
       const int kx = kx0 + p, kz = wavenum(n, g.nz);
@@ -418,7 +457,6 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
   const int nvalid = min(P, g.nxh - kx0);
   const long long zstride = (long long)g.ny * g.nxp;
   const long long base = (long long)iy * g.nxp + kx0;
-  const double ky = wavenum(iy, g.ny);
   if (launch_failed(err)) return;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -432,8 +470,8 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
   }
   __syncthreads();
   if (!mbar_wait_bounded(&bar, 0, err)) return;
-  const bool fsum = za.fs.enabled && ((double)kx0 * kx0 + ky * ky < za.fs.fkmax2);
-  const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(za.fs.fkmax2), kc_b = k2_lt(za.kcut2);
+  const int kyi = wavenum(iy, g.ny), fk_b = za.fs.fkmax2.b, kc_b = za.kcut2.b;
+  const bool fsum = za.fs.enabled && kx0 * kx0 + kyi * kyi < fk_b;
   double q = 0.0;
   for (int e = threadIdx.x; e < P * N; e += NT) {
     const int p = e % P, n = e / P;
@@ -450,7 +488,7 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
           q += (double)m[c].x * sv.x + (double)m[c].y * sv.y;
         }
     }
-    const T d = (T)((ix == 0 || ix == g.nxh - 1) ? za.inv_n3 : 0.5 * za.inv_n3);
+    const T d = (ix == 0 || ix == g.nxh - 1) ? za.inv_n3 : T(0.5) * za.inv_n3;
 #pragma unroll
     for (int c = 0; c < 3; ++c) rt[c][e] = cscale(m[c], d);
   }
@@ -464,8 +502,12 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
   // outputs as lmap tiles lam; columns past nx/2+1 lie outside it and are
   // not written).  Shorter pencils: element stores from the transform's
   // registers (the bulk form gained nothing at 128^3).
-  if (EF::TWO_PASS && za.ustore) {
-    for (int c = 0; c < 3; ++c) EF::template run_inplace<true>(rt[c], tw);
+  if ((EF::TWO_PASS || Z::GROUPED) && za.ustore) {
+    if constexpr (Z::GROUPED) {
+      Z::ZG::Engine::template run_inplace<true>(rt[0] + (size_t)(threadIdx.x / Z::ZG::NTG) * P * N, tw);
+    } else {
+      for (int c = 0; c < 3; ++c) EF::template run_inplace<true>(rt[c], tw);
+    }
     fence_proxy_async();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -513,7 +555,7 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
   for (int c = 0; c < 3; ++c) rt[c] = reinterpret_cast<C*>(smraw + c * Z::TILE);
   C* work = reinterpret_cast<C*>(smraw + 3 * Z::TILE);
   __shared__ __align__(8) uint64_t bars[3];
-  __shared__ double s_coef;
+  __shared__ T s_coef;
   __shared__ double red[NT / 32 + 1];
   const int kx0 = blockIdx.x * P;
   const int iy = paired_row(blockIdx.y, g.ny);
@@ -522,9 +564,11 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
   const long long base = (long long)iy * g.nxp + kx0;
   const T ky = (T)wavenum(iy, g.ny);
   const bool paired = kx0 == 0;   // meets its partner: both CTAs stay until then
-  const bool band = st.forced && ((double)kx0 * kx0 + (double)ky * ky < st.fkmax2);
-  const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(st.fkmax2), kc_b = k2_lt(st.kcut2);
-  if (!paired && launch_failed(err)) return;
+  const int kyi = wavenum(iy, g.ny), fk_b = st.fkmax2.b, kc_b = st.kcut2.b;
+  const bool band = st.forced && kx0 * kx0 + kyi * kyi < fk_b;
+  if (paired) cluster_arrive();
+  const bool failed = !paired && launch_failed(err);
+  if (!Z::GROUPED && failed) return;
   if (threadIdx.x == 0) {
     for (int c = 0; c < 3; ++c) mbar_init(&bars[c], 1);
     fence_mbar_init();
@@ -535,23 +579,32 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
         tma_load_4d(reinterpret_cast<char*>(rt[c]) + (size_t)h * Cfg::BOX * P * sizeof(C), &lmap, &bars[c],
                     kx0 * Cfg::U, iy, h * Cfg::BOX, c);
     }
-    if (band) {
-      const double kf = forcing_energy(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, st.fkmax2);
-      s_coef = st.eps / (2.0 * kf);
-    }
+  }
+  if (band && threadIdx.x >= NT - 32) {   // one warp finds the forcing coefficient
+    const double kf = warp_sum(forcing_energy_lane(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, fk_b));
+    if (threadIdx.x == NT - 32) s_coef = (T)(st.eps / (2.0 * kf));
   }
   __syncthreads();
-  bool ok = true;
-  for (int c = 0; c < 3; ++c) {
-    ok = mbar_wait_bounded(&bars[c], 0, err) && ok;
-    if (!ok && !paired) return;
-    // the update's operands into L2 once the Lamb tiles are in (issued with
-    // them, the prefetch delays them)
-    if (c == 2 && threadIdx.x == 0) prefetch_update_tile<Cfg>(&fmap, st, kx0, iy);
-    EF::template run_inplace<false>(rt[c], tw);
+  bool ok = !failed;
+  // the update's operands into L2 once the Lamb tiles are in (issued with
+  // them, the prefetch delays them)
+  if constexpr (Z::GROUPED) {
+    const int grp = threadIdx.x / Z::ZG::NTG;
+    ok = mbar_wait_bounded(&bars[grp], 0, err) && ok;
+    if (threadIdx.x == 2 * Z::ZG::NTG) prefetch_update_tile<Cfg>(&fmap, st, kx0, iy);
+    Z::ZG::Engine::template run_inplace<false>(rt[0] + (size_t)grp * P * N, tw);
+  } else {
+    for (int c = 0; c < 3; ++c) {
+      ok = mbar_wait_bounded(&bars[c], 0, err) && ok;
+      if (!ok && !paired) return;
+      if (c == 2 && threadIdx.x == 0) prefetch_update_tile<Cfg>(&fmap, st, kx0, iy);
+      EF::template run_inplace<false>(rt[c], tw);
+    }
   }
+  ok = __syncthreads_and(ok);
+  if (!ok && !paired) return;
   if (paired) {
-    hermitian_column<T, P, N, NT>(rt, st, g, iy, base, zstride, band, band ? s_coef : 0.0, 0, fk_b);
+    hermitian_column<T, P, N, NT>(rt, work, st, g, iy, base, zstride, band, band ? s_coef : T(0), 0, fk_b);
     if (!ok) return;
   }
   // spectral update; the next stage input goes back into the tiles
@@ -582,7 +635,7 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
       const int kz = wavenum(iz, g.nz);
       const int k2 = ix * ix + kyi * kyi + kz * kz;
       if (band && k2 < fk_b && ix > 0) {
-        const T ac = (T)s_coef;
+        const T ac = s_coef;
 #pragma unroll
         for (int c = 0; c < 3; ++c) wp[c] = cadd(wp[c], cscale(st.sin[c][idx], ac));
       }
@@ -604,14 +657,20 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
       }
     }
   }
-  __syncthreads();
-  // forcing band energy of the next stage input (force.f90:16-22), FP64
+  // forcing band energy of the next stage input (force.f90:16-22), FP64: the
+  // warps' sums now, the block's after the z-inverse
   if (band && fa.kf_next) {
-    const double sum = block_sum<NT>(q, red);
-    if (threadIdx.x == 0) fa.kf_next[(long long)blockIdx.x * g.ny + iy] = sum;
+    q = warp_sum(q);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = q;
   }
+  __syncthreads();
   // fa.out[0..2] are the Lamb fields: lmap tiles them as rt
   zinv_from_tiles<T, LOGN>(rt, work, kx0, iy, nvalid, base, zstride, fa.out, g, tw, &lmap);
+  if (band && fa.kf_next && threadIdx.x == 0) {
+    double sum = 0.0;
+    for (int i = 0; i < NT / 32; ++i) sum += red[i];
+    fa.kf_next[(long long)blockIdx.x * g.ny + iy] = sum;
+  }
 }
 
 }  // namespace sc

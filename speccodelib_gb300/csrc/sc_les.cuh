@@ -241,7 +241,7 @@ les_zfwd_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st, Geom 
   for (int c = 0; c < 3; ++c) w[c] = reinterpret_cast<C*>(smraw + c * Z::TILE);
   C* const tau = reinterpret_cast<C*>(smraw + 3 * Z::TILE);
   __shared__ __align__(8) uint64_t bars[4];
-  __shared__ double s_coef;
+  __shared__ T s_coef;
   const int kx0 = blockIdx.x * P;
   const int iy = paired_row(blockIdx.y, g.ny);
   const int nvalid = min(P, g.nxh - kx0);
@@ -250,8 +250,8 @@ les_zfwd_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st, Geom 
   const T ky = (T)wavenum(iy, g.ny);
   const bool paired = st.symmetrize && kx0 == 0;   // meets its partner: both CTAs stay until then
   if (!paired && launch_failed(err)) return;
-  const bool fblock = st.forced && ((double)kx0 * kx0 + (double)ky * ky < st.fkmax2);
-  const int fk_b = k2_lt(st.fkmax2);
+  const int kyi = wavenum(iy, g.ny), fk_b = st.fkmax2.b;
+  const bool fblock = st.forced && kx0 * kx0 + kyi * kyi < fk_b;
   if (threadIdx.x == 0) {
     for (int c = 0; c < 4; ++c) mbar_init(&bars[c], 1);
     fence_mbar_init();
@@ -260,10 +260,11 @@ les_zfwd_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st, Geom 
     tma_issue_tile<Cfg>(tau, &fmap, &bars[3], 2, kx0, iy, les_t3(0), P, Z::TILE);
     tma_issue_tile<Cfg>(w[1], &fmap, &bars[1], 2, kx0, iy, 1, P, Z::TILE);
     tma_issue_tile<Cfg>(w[2], &fmap, &bars[2], 2, kx0, iy, 2, P, Z::TILE);
-    if (fblock) {
-      const double kf = forcing_energy(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, st.fkmax2);
-      s_coef = st.eps / (2.0 * kf);
-    }
+  }
+  // one warp finds the forcing coefficient
+  if (fblock && threadIdx.x >= NT - 32) {
+    const double kf = warp_sum(forcing_energy_lane(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, fk_b));
+    if (threadIdx.x == NT - 32) s_coef = (T)(st.eps / (2.0 * kf));
   }
   __syncthreads();
   bool ok = true;
@@ -292,10 +293,11 @@ les_zfwd_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st, Geom 
   }
   __syncthreads();
   if (paired) {
-    hermitian_column<T, P, N, NT>(w, st, g, iy, base, zstride, fblock, fblock ? s_coef : 0.0, 0, fk_b);
+    cluster_arrive();   // tau is free for the partner's column
+    hermitian_column<T, P, N, NT>(w, tau, st, g, iy, base, zstride, fblock, fblock ? s_coef : T(0), 0, fk_b);
     if (!ok) return;
   }
-  zfwd_update<T, P, N, NT, 2, MODE>(w, st, g, kx0, iy, nvalid, base, zstride, fblock, fblock ? s_coef : 0.0, 0, fk_b,
+  zfwd_update<T, P, N, NT, 2, MODE>(w, st, g, kx0, iy, nvalid, base, zstride, fblock, fblock ? s_coef : T(0), 0, fk_b,
                                     paired, false);
 }
 

@@ -22,7 +22,7 @@ enum DiagQ { DQ_ENERGY = 0, DQ_K2Q = 1, DQ_MAXDIV = 2, DQ_NONFINITE = 3, DQ_MAXU
 template <typename T> struct DiagArgs {
   const C2<T>* v[3];
   int physical;           // 0: spectral fields (energy etc.); 1: packed physical rows (max |u|^2)
-  double kmax2;           // < 0: every mode; else only modes with k2 < kmax2 (forcing band)
+  K2Lt kmax2;             // < 0: every mode; else only modes with k2 < kmax2 (forcing band)
   int rows_per_block;
   int nshell;             // 0: no spectrum; else nx/2 shells
   double* partial;        // [gridDim.x][DQ_N + nshell]
@@ -111,8 +111,8 @@ __global__ void __launch_bounds__(256, 3) diag_spec_kernel(DiagArgs<T> da, Geom 
   double* const mine = shells + (threadIdx.x % kDiagCopies) * (ns + 1);
   double e = 0.0, k2q = 0.0, nf = 0.0;
   T mdiv2 = T(0);
-  const bool kmax_on = da.kmax2 >= 0.0;
-  const int kmax_b = k2_lt(da.kmax2);
+  const bool kmax_on = da.kmax2.b >= 0;
+  const int kmax_b = da.kmax2.b;
   const bool want_shell = da.shell_hi > 0 || ns > 0;
   const int chunks = (g.nxh + 31) / 32, nbat = (g.ny / 2 + kDiagRun) / kDiagRun;
   const int tasks = diag_tasks(g);
@@ -248,7 +248,7 @@ template <typename T> struct SpecOpArgs {
   const C2<T>* gsrc[3];
   double a, b;            // scalars
   const double* dscal;    // device scalar (OP_SCALE: multiply by sqrt(a / *dscal) if set)
-  double kcut2;
+  K2Lt kcut2;
   double akp, u0, kmin, kmax;
   int spectrum_kind;      // 0: akp shape, 1: k^(-11/6) band
 };
@@ -274,7 +274,8 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
     }
     return;
   }
-  const int kc_b = k2_lt(oa.kcut2), b_b = k2_lt(oa.b);
+  const int kc_b = oa.kcut2.b, b_b = oa.op == OP_FORCE_BAND ? k2_lt(oa.b) : 0;
+  const T a = (T)oa.a, b = (T)oa.b;
   for (Walk3 w(t0, tstride, rows * g.nxh, g.nxh, g.ny); w.ok(); w.next()) {
     const int ix = w.ix, iy = w.iy, iz = w.iz;
     const long long idx = w.row() * g.nxp + ix;
@@ -306,7 +307,6 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
       case OP_FORCE_ADD:
         // k2(1,1,1) = tiny < fkmax^2: the mean mode is in the band too
         if (k2i < kc_b) {
-          const T a = (T)oa.a;
           for (int c = 0; c < 3; ++c) oa.f[c][idx] = cadd(oa.f[c][idx], cscale(oa.gsrc[c][idx], a));
         }
         break;
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
         break;
       case OP_AXPBY:
         for (int c = 0; c < oa.nfields; ++c)
-          oa.f[c][idx] = cadd(cscale(oa.f[c][idx], (T)oa.a), cscale(oa.gsrc[c][idx], (T)oa.b));
+          oa.f[c][idx] = cadd(cscale(oa.f[c][idx], a), cscale(oa.gsrc[c][idx], b));
         break;
       case OP_PMUL: {
         const C gp = oa.gsrc[0][idx];
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
       }
       case OP_IDIV: {
         const C d = cadd(cadd(cscale(oa.f[0][idx], kx), cscale(oa.f[1][idx], ky)), cscale(oa.f[2][idx], kz));
-        oa.f[0][idx] = cmuli(cscale(d, (T)oa.a));
+        oa.f[0][idx] = cmuli(cscale(d, a));
         break;
       }
       case OP_DX:
@@ -357,7 +357,6 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
       }
       case OP_FORCE_BAND:
         if (k2i < kc_b && !(k2i < b_b)) {
-          const T a = (T)oa.a;
           for (int c = 0; c < oa.nfields; ++c) oa.f[c][idx] = cadd(oa.f[c][idx], cscale(oa.gsrc[c][idx], a));
         }
         break;
@@ -379,7 +378,8 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
 template <typename T> struct BandArgs {
   const C2<T>* v[3];
   int nf;                 // fields summed (1 or 3)
-  double lo2, hi2, eps, tiny;
+  K2Lt lo2, hi2;
+  double eps, tiny;
   double* out;
 };
 
@@ -387,7 +387,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) band_coef_kernel(BandArgs<T> ba, Geom g) {
   pdl_wait();
   __shared__ double red[256 / 32 + 1];
-  const int lo_b = k2_lt(ba.lo2), hi_b = k2_lt(ba.hi2);
+  const int lo_b = ba.lo2.b, hi_b = ba.hi2.b;
   int kb = 0;
   while ((kb + 1) * (kb + 1) < hi_b) ++kb;   // largest |k_i| with k_i^2 < hi2
   const int nkx = min(kb, g.nxh - 1) + 1;
@@ -425,7 +425,7 @@ template <typename T> struct RotArgs {
   C2<T>* o[3];           // previous right-hand side (written at pass 0 and >= 2)
   C2<T>* a[2];           // helical amplitudes a+, a-
   double nu, dt, om;     // viscosity, time step, rotation rate
-  double kcut2;          // v = 0 where k2 >= kcut2 (when mask_v)
+  K2Lt kcut2;          // v = 0 where k2 >= kcut2 (when mask_v)
   int mask_v;            // truncate the rebuilt velocity
   // passive scalar (when phi is set): phi, its right-hand side, the previous
   // right-hand side (written at pass 0 and >= 2), the initial phi (written at
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(256) rot_update_kernel(RotArgs<T> ra, Geom g) 
   const long long rows = (long long)g.ny * g.nz;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long tstride = (long long)gridDim.x * blockDim.x;
-  const int kc_b = k2_lt(ra.kcut2);
+  const int kc_b = ra.kcut2.b;
   const T nu = (T)ra.nu, dt = (T)ra.dt, om = (T)ra.om;
   const int pass = ra.pass;
   for (Walk3 it(t0, tstride, rows * g.nxh, g.nxh, g.ny); it.ok(); it.next()) {
@@ -509,7 +509,7 @@ template <typename T> struct Ab2vArgs {
   C2<T>* v0[3];          // initial field (written at pass 0, read at pass 1)
   double nu, dt, dto;    // viscosity, this step, the previous step
   double s, ek, dl;      // the pass's weights
-  double kcut2;          // v = 0 where k2 >= kcut2 and at the mean mode (when mask_v)
+  K2Lt kcut2;          // v = 0 where k2 >= kcut2 and at the mean mode (when mask_v)
   int mask_v;
   // passive scalar (when phi is set): phi, its right-hand side, its history,
   // the initial phi; Prandtl number; hist_rhs: history at pass 0 is wphi
@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(256) ab2v_update_kernel(Ab2vArgs<T> aa, Geom g
   const long long rows = (long long)g.ny * g.nz;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long tstride = (long long)gridDim.x * blockDim.x;
-  const int kc_b = k2_lt(aa.kcut2);
+  const int kc_b = aa.kcut2.b;
   const T nu = (T)aa.nu, dt = (T)aa.dt, dto = (T)aa.dto, s = (T)aa.s, ek = (T)aa.ek, dl = (T)aa.dl;
   const int pass = aa.pass;
   for (Walk3 it(t0, tstride, rows * g.nxh, g.nxh, g.ny); it.ok(); it.next()) {

@@ -132,7 +132,7 @@ template <> struct ZvOut<ZV_ADJ> { static constexpr int n = 6; };   // + 3 adjoi
 
 struct ForceSum {
   int enabled;
-  double fkmax2;
+  K2Lt fkmax2;
   double* partial;   // [tile * ny + iy]
 };
 
@@ -146,8 +146,8 @@ template <typename T> struct ZvArgs {
   const C2<T>* lam[3];
   double* cpartial;  // forcing adjoint: sum over the band of Re(conj(mu) v)
   int mask_rhs;
-  double kcut2;
-  double inv_n3;
+  K2Lt kcut2;
+  T inv_n3;
   int ustore;        // TMA z-inverse: u stored from its tiles by bulk tensor stores
 };
 
@@ -234,11 +234,11 @@ zinv_vel_kernel(ZvArgs<T> za, FieldList<T> out, Geom g, const C2<T>* __restrict_
   const long long base = (long long)iy * g.nxp + kx0;
   const T ky = (T)wavenum(iy, g.ny);
   const int kyi = wavenum(iy, g.ny);
-  const int fk_b = k2_lt(za.fs.fkmax2), kt_b = k2_le(za.ktest2), kc_b = k2_lt(za.kcut2);
+  const int fk_b = za.fs.fkmax2.b, kt_b = k2_le(za.ktest2), kc_b = za.kcut2.b;
 
   C vr[E::J1][E::R1][3];
   double q = 0.0;
-  const bool fsum = za.fs.enabled && ((double)kx0 * kx0 + (double)ky * ky < za.fs.fkmax2);
+  const bool fsum = za.fs.enabled && (kx0 * kx0 + kyi * kyi < fk_b);
 #pragma unroll
   for (int a = 0; a < E::J1; ++a)
 #pragma unroll
@@ -310,7 +310,7 @@ zinv_vel_kernel(ZvArgs<T> za, FieldList<T> out, Geom g, const C2<T>* __restrict_
             }
         }
         const int ix = kx0 + p;
-        const T d = (T)((ix == 0 || ix == g.nxh - 1) ? za.inv_n3 : 0.5 * za.inv_n3);
+        const T d = (ix == 0 || ix == g.nxh - 1) ? za.inv_n3 : T(0.5) * za.inv_n3;
 #pragma unroll
         for (int c = 0; c < 3; ++c) vr[a][r][c] = cscale(m[c], d);
       }
@@ -365,11 +365,12 @@ template <typename T> struct StageArgs {
   const T* ez;
   T dt;
   int forced;
-  double fkmax2, eps;
+  K2Lt fkmax2;
+  double eps;
   const double* kf_partial;
   int kf_tiles;
   int kf_ptile;         // tile width of the zinv kernel that wrote kf_partial
-  double kcut2;
+  K2Lt kcut2;
   int mask_rhs;         // also truncate the RHS (mask = rhs_and_step)
   int symmetrize;       // apply symmetrize.f90:32-64 to w
   int project;          // apply projection.f90 to w
@@ -387,7 +388,7 @@ template <typename T> struct StageArgs {
   // forcing with a coefficient computed on the device (force_rot.f90): when
   // fcoef is set, w += (*fcoef) sin on the band fband_lo2 <= k2 < fkmax2
   const double* fcoef;
-  double fband_lo2;
+  K2Lt fband_lo2;
 };
 
 
@@ -404,7 +405,7 @@ __host__ __device__ constexpr bool mode_reads_acc(int m) {
 // state (v, or v0 for the AB2 midpoint pass) and accumulator values already
 // loaded.  w is the right-hand side after forcing and symmetrize.  With
 // `snext` given, RK stages 1-3 return the next stage input there instead of
-// storing it to st.sout.  kcut_b = k2_lt(st.kcut2), computed once per
+// storing it to st.sout.  kcut_b = st.kcut2.b, computed once per
 // kernel.  MODE >= 0: the update mode as a compile-time constant (st.mode
 // otherwise).
 template <typename T, int MODE = -1>
@@ -554,9 +555,8 @@ __device__ __forceinline__ void finish_point(const StageArgs<T>& st, const Geom&
 // the axis instead put ny double-precision compares (5 us at ny = 64) in front
 // of the band's tiles.
 __device__ __forceinline__ double forcing_energy(const double* partial, int tiles, int P, int ny,
-                                                 double fkmax2) {
+                                                 int fk_b) {
   double s = 0.0;
-  const int fk_b = k2_lt(fkmax2);
   for (int t = 0; t < tiles; ++t) {
     const double* row = partial + (long long)t * ny;
     const int kx2 = t * P * t * P;
@@ -567,6 +567,18 @@ __device__ __forceinline__ double forcing_energy(const double* partial, int tile
     }
     for (int iy = max(ny / 2, ny - k + 1); iy < ny; ++iy) s += row[iy];
   }
+  return s;
+}
+
+// The same by one warp: this lane's share of the sum (the lanes' values add up
+// to it).  The loads are independent, where forcing_energy chains them.
+__device__ __forceinline__ double forcing_energy_lane(const double* partial, int tiles, int P, int ny, int fk_b) {
+  double s = 0.0;
+  for (int t = 0; t < tiles && t * P * t * P < fk_b; ++t)
+    for (int iy = threadIdx.x & 31; iy < ny; iy += 32) {
+      const int ky = wavenum(iy, ny);
+      if (t * P * t * P + ky * ky < fk_b) s += partial[(long long)t * ny + iy];
+    }
   return s;
 }
 
@@ -638,11 +650,11 @@ __device__ __forceinline__ void zfwd_finish(C2<T> (&w)[E::JL][E::RL][3], const S
     return;
   }
   // forcing coefficient a = eps / (2 K_f) (force.f90:23)
-  const bool fblock = st.forced && ((double)kx0 * kx0 + (double)ky * ky < st.fkmax2);
-  const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(st.fkmax2), kc_b = k2_lt(st.kcut2);
+  const int kyi = wavenum(iy, g.ny), fk_b = st.fkmax2.b, kc_b = st.kcut2.b;
+  const bool fblock = st.forced && kx0 * kx0 + kyi * kyi < fk_b;
   if (fblock) {
     if (threadIdx.x == 0) {
-      const double kf = forcing_energy(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, st.fkmax2);
+      const double kf = forcing_energy(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, fk_b);
       s_coef = st.eps / (2.0 * kf);
     }
     __syncthreads();
@@ -720,7 +732,7 @@ template <typename T, int MODE = -1>
 __global__ void fixup_kx0_kernel(StageArgs<T> st, Geom g) {
   using C = C2<T>;
   const long long total = (long long)g.ny * g.nz;
-  const int kc_b = k2_lt(st.kcut2);
+  const int kc_b = st.kcut2.b;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const int iy = (int)(t % g.ny), iz = (int)(t / g.ny);

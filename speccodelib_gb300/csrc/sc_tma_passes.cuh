@@ -66,38 +66,51 @@ __device__ __forceinline__ int paired_row(int b, int ny) {
   return !(b & 1) ? m : (m == 0 ? ny / 2 : ny - m);
 }
 // Hermitian copy of symmetrize.f90:52-62 on the kx = 0 column (p = 0) of the
-// tiles w, after the z-forward transform and before the spectral update:
-// forcing is added to the column, then the targets (kz index over nz/2, and
-// ky index over ny/2 at kz = 0) take the conjugates of w(-ky, -kz) from the
-// partner CTA's tiles through distributed shared memory (from the own tiles
-// at ky = 0), so the update treats the column like any other.  This replaces
-// a side buffer, a fix-up launch after every z-forward and, in the fused RK
-// stages, a one-tile z-inverse launch: three dependent launches per stage
-// become one (256^3 FP32 step 3.08 -> 2.97 ms, 64^3 178 -> 145 us, 512^3
-// 24.0 -> 23.5 ms).
-// Sources and targets are disjoint; every thread of both CTAs calls it.
-template <typename T, int P, int N, int NT>
-__device__ __forceinline__ void hermitian_column(C2<T>* const w[3], const StageArgs<T>& st, const Geom& g, int iy,
-                                                 long long base, long long zstride, bool fblock, double coef, int flo_b,
-                                                 int fk_b) {
-  using C = C2<T>;
-  const int kyi = wavenum(iy, g.ny);
-  if (fblock)
-    for (int n = threadIdx.x; n < N; n += NT) {
-      const int kz = wavenum(n, g.nz), k2 = kyi * kyi + kz * kz;
-      if (k2 < fk_b && k2 >= flo_b)
+// NF tiles w: the targets (kz index over nz/2, and ky index over ny/2 at kz = 0)
+// take the conjugates of w(-ky, -kz) from the partner CTA (from the own tiles at
+// ky = 0).  Each CTA pushes its column into the partner's `col` (NF N/2 values)
+// through distributed shared memory, so one cluster barrier is waited for; the
+// caller has arrived once (cluster_arrive) at its start, which tells the partner
+// that this CTA's shared memory may be written.  src(c, n, w) gives the column's
+// value from the tile's (and may change the tile).  This replaces a side buffer, a
+// fix-up launch after every z-forward and, in the fused RK stages, a one-tile
+// z-inverse launch: three dependent launches per stage become one (256^3 FP32
+// step 3.08 -> 2.97 ms, 64^3 178 -> 145 us, 512^3 24.0 -> 23.5 ms).
+// Every thread of both CTAs calls it, after a barrier on the tiles; it ends with
+// a barrier.
+template <int NF, int P, int N, int NT, typename C, class F>
+__device__ __forceinline__ void column_copy(C* const w[], C* col, int iy, int ny, F&& src) {
+  cluster_wait();
+  const uint32_t to = iy == 0 ? cluster_rank() : (cluster_rank() ^ 1u);
+  for (int n = threadIdx.x; n < N / 2; n += NT)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) w[c][n * P] = cadd(w[c][n * P], cscale(st.sin[c][base + n * zstride], (T)coef));
+    for (int c = 0; c < NF; ++c) {
+      const C v = cconj(src(c, n, w[c][n * P]));
+      if (iy != ny / 2 && (iy == 0 || n > 0 || iy < ny / 2)) cluster_store(&col[c * (N / 2) + n], v, to);
     }
   cluster_sync();
-  const uint32_t from = iy == 0 ? cluster_rank() : (cluster_rank() ^ 1u);
-  for (int n = threadIdx.x; n < N; n += NT) {
-    if (!(n > N / 2 || (n == 0 && iy > g.ny / 2))) continue;
+  for (int n = threadIdx.x; n < N / 2; n += NT) {
+    if (n == 0 && iy <= ny / 2) continue;
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      w[c][n * P] = iy == g.ny / 2 ? czero<C>() : cconj(cluster_load(&w[c][((N - n) % N) * P], from));
+    for (int c = 0; c < NF; ++c) w[c][(N - n) % N * P] = iy == ny / 2 ? czero<C>() : col[c * (N / 2) + n];
   }
-  cluster_sync();   // the partner has read this CTA's column
+  __syncthreads();
+}
+
+// The same after the z-forward transform of the right-hand side and before the
+// spectral update, which treats the column like any other: forcing is added to
+// the column first.
+template <typename T, int P, int N, int NT>
+__device__ __forceinline__ void hermitian_column(C2<T>* const w[3], C2<T>* col, const StageArgs<T>& st, const Geom& g,
+                                                 int iy, long long base, long long zstride, bool fblock, T coef,
+                                                 int flo_b, int fk_b) {
+  using C = C2<T>;
+  const int kyi = wavenum(iy, g.ny);
+  column_copy<3, P, N, NT>(w, col, iy, g.ny, [&](int c, int n, C& v) {
+    const int k2 = kyi * kyi + n * n;
+    if (fblock && k2 < fk_b && k2 >= flo_b) v = cadd(v, cscale(st.sin[c][base + n * zstride], coef));
+    return v;
+  });
 }
 
 // Where a pencil lies: element (p, n) of tile (kx0, outer) of field f is
@@ -237,10 +250,10 @@ zinv_tma_kernel(const __grid_constant__ CUtensorMap vmap, ZvArgs<T> za, FieldLis
   __syncthreads();
   if (!mbar_wait_bounded(&bar, 0, err)) return;
   // forcing band energy of the stage input (force.f90:16-22), FP64
-  const bool fsum = za.fs.enabled && ((double)kx0 * kx0 + (double)ky * ky < za.fs.fkmax2);
+  const int kyi = wavenum(iy, g.ny), fk_b = za.fs.fkmax2.b;
+  const bool fsum = za.fs.enabled && kx0 * kx0 + kyi * kyi < fk_b;
   if (fsum) {
     double q = 0.0;
-    const int kyi = wavenum(iy, g.ny), fk_b = k2_lt(za.fs.fkmax2);
     for (int e = threadIdx.x; e < P * N; e += NT) {
       const int p = e % P, n = e / P;
       const int kx = kx0 + p, kz = wavenum(n, g.nz);
@@ -335,10 +348,10 @@ zfwd_fields_tma_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st
 // tiles.
 template <typename T, int P, int N, int NT, int EB, int MODE>
 __device__ __forceinline__ void zfwd_update(C2<T>* const w[3], const StageArgs<T>& st, const Geom& g, int kx0, int iy,
-                                            int nvalid, long long base, long long zstride, bool fblock, double coef,
+                                            int nvalid, long long base, long long zstride, bool fblock, T coef,
                                             int flo_b, int fk_b, bool paired, bool tstore) {
   using C = C2<T>;
-  const int kyi = wavenum(iy, g.ny), kc_b = k2_lt(st.kcut2);
+  const int kyi = wavenum(iy, g.ny), kc_b = st.kcut2.b;
   for (int e0 = threadIdx.x; e0 < P * N; e0 += NT * EB) {
     C wv[EB][3], vv[EB][3], av[EB][3];
     bool act[EB];
@@ -365,7 +378,7 @@ __device__ __forceinline__ void zfwd_update(C2<T>* const w[3], const StageArgs<T
         const int kz = wavenum(iz, g.nz);
         const int k2 = ix * ix + kyi * kyi + kz * kz;
         if (k2 < fk_b && k2 >= flo_b) {
-          const T ac = (T)coef;
+          const T ac = coef;
 #pragma unroll
           for (int c = 0; c < 3; ++c) wp[c] = cadd(wp[c], cscale(st.sin[c][idx], ac));
         }
@@ -390,6 +403,23 @@ __device__ __forceinline__ void zfwd_update(C2<T>* const w[3], const StageArgs<T
 // update mode as a compile-time constant (-1: st.mode at run time).  With
 // MODE == SM_RK4 and vstore, the new state goes back into the tiles and
 // leaves by bulk tensor stores through vmap (st.vout, tiles as lmap).
+// Short pencils: a z kernel at 64^3 is one CTA or two per SM and its time a
+// chain of latencies, so three groups of threads transform the three tiles at
+// once instead of one group in turn.  FP32 pencils to 128 points and FP64 to 64.
+// A group's threads take one radix-8 job each to 64 points, two at 128.  Step
+// times, groups against in turn: FP32 64^3 137 -> 112 us, 128^3 430 -> 396 us;
+// FP64 32^3 417 -> 267 us, 64^3 933 -> 862 us, but 128^3 5.66 -> 5.79 ms (bound by
+// FP64 issue, and fewer CTAs per SM).  Two jobs per thread at 32 points: 68 -> 74
+// us; one at 128: 396 -> 445 us.
+template <typename T, int LOGN> struct ZgCfg {
+  using Cfg = TmaCfg<T, LOGN>;
+  static constexpr bool ON = LOGN <= (sizeof(T) == 4 ? 7 : 6);
+  static constexpr int NTG_RAW = Cfg::P * Cfg::N / (LOGN <= 6 ? 8 : 16);
+  static constexpr int NTG = NTG_RAW < 32 ? 32 : NTG_RAW;
+  static constexpr int NT = 3 * NTG;
+  using Engine = FFTEngine<T, LOGN, Cfg::P, Cfg::P, NTG, true, 0, true, 8, true>;
+};
+
 // Thread count of zfwd_tma_kernel: for 512- and 256-point pencils 16 points
 // per thread, which gives its in-place transforms the two-pass form
 // (SC_ZFWD_NT8: 8 points per thread, the radix-8 stages).
@@ -401,10 +431,13 @@ template <typename T, int LOGN> struct ZfCfg {
   static constexpr int NT = (LOGN == 9 || LOGN == 8) ? Cfg::P * Cfg::N / 16 : Cfg::NT;
 #endif
   using Engine = FFTEngine<T, LOGN, Cfg::P, Cfg::P, NT, true>;
+  using G = ZgCfg<T, LOGN>;
+  static constexpr bool GROUPED = G::ON;
+  static constexpr int NTF = GROUPED ? G::NT : NT;   // threads of zfwd_tma_kernel
 };
 
 template <typename T, int LOGN, int MODE>
-__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(ZfCfg<T, LOGN>::NT, 2)
+__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(ZfCfg<T, LOGN>::NTF, 2)
 zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap vmap, int vstore,
                 StageArgs<T> st, Geom g, const C2<T>* __restrict__ tw, int* err) {
   pdl_wait();
@@ -413,13 +446,15 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
   using C = C2<T>;
   constexpr int P = Cfg::P;
   constexpr int N = Cfg::N;
-  constexpr int NT = ZfCfg<T, LOGN>::NT;
+  constexpr int NT = ZfCfg<T, LOGN>::NTF;
+  using ZG = ZgCfg<T, LOGN>;
+  constexpr bool GROUPED = ZfCfg<T, LOGN>::GROUPED;
   extern __shared__ __align__(128) unsigned char smdyn[];
   unsigned char* smraw = align128(smdyn);
   C* w[3];
   for (int c = 0; c < 3; ++c) w[c] = reinterpret_cast<C*>(smraw + c * Cfg::TILE_BYTES);
   __shared__ __align__(8) uint64_t bars[3];
-  __shared__ double s_coef;
+  __shared__ T s_coef;
   const int kx0 = blockIdx.x * P;
   const int iy = paired_row(blockIdx.y, g.ny);
   const int nvalid = min(P, g.nxh - kx0);
@@ -428,7 +463,10 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
   const T ky = (T)wavenum(iy, g.ny);
   // the kx = 0 tiles meet their partner: both CTAs stay until then
   const bool paired = st.symmetrize && kx0 == 0;
-  if (!paired && launch_failed(err)) return;
+  __shared__ C s_col[3 * N / 2];
+  if (paired) cluster_arrive();
+  const bool failed = !paired && launch_failed(err);
+  if (!GROUPED && failed) return;
   if (threadIdx.x == 0) {
     for (int c = 0; c < 3; ++c) mbar_init(&bars[c], 1);
     fence_mbar_init();
@@ -440,32 +478,38 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
                     kx0 * Cfg::U, iy, h * Cfg::BOX, c);
     }
   }
-  const bool fblock = st.forced && ((double)kx0 * kx0 + (double)ky * ky < st.fkmax2);
-  const int fk_b = k2_lt(st.fkmax2);
+  const int kyi = wavenum(iy, g.ny), fk_b = st.fkmax2.b;
+  const bool fblock = st.forced && kx0 * kx0 + kyi * kyi < fk_b;
   // lower edge of the forcing band (0 for force.f90's k2 < fkmax^2)
-  const int flo_b = k2_lt(st.fband_lo2);
-  if (fblock && threadIdx.x == 0) {
-    if (st.fcoef) {
-      s_coef = *st.fcoef;
-    } else {
-      const double kf = forcing_energy(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, st.fkmax2);
-      s_coef = st.eps / (2.0 * kf);
-    }
+  const int flo_b = st.fband_lo2.b;
+  if (fblock && threadIdx.x >= NT - 32) {   // one warp finds the forcing coefficient
+    double coef = 0.0;
+    if (st.fcoef) coef = *st.fcoef;
+    else coef = st.eps / (2.0 * warp_sum(forcing_energy_lane(st.kf_partial, st.kf_tiles, st.kf_ptile, g.ny, fk_b)));
+    if (threadIdx.x == NT - 32) s_coef = (T)coef;
   }
   __syncthreads();
-  bool ok = true;
-  for (int c = 0; c < 3; ++c) {
-    ok = mbar_wait_bounded(&bars[c], 0, err) && ok;
-    if (!ok && !paired) return;
-    E::template run_inplace<false>(w[c], tw);
+  bool ok = !failed;
+  if constexpr (GROUPED) {
+    const int grp = threadIdx.x / ZG::NTG;
+    ok = mbar_wait_bounded(&bars[grp], 0, err) && ok;
+    ZG::Engine::template run_inplace<false>(w[0] + (size_t)grp * P * N, tw);
+  } else {
+    for (int c = 0; c < 3; ++c) {
+      ok = mbar_wait_bounded(&bars[c], 0, err) && ok;
+      if (!ok && !paired) return;
+      E::template run_inplace<false>(w[c], tw);
+    }
   }
+  ok = __syncthreads_and(ok);
+  if (!ok && !paired) return;
   if (paired) {
-    hermitian_column<T, P, N, NT>(w, st, g, iy, base, zstride, fblock, fblock ? s_coef : 0.0, flo_b, fk_b);
+    hermitian_column<T, P, N, NT>(w, s_col, st, g, iy, base, zstride, fblock, fblock ? s_coef : T(0), flo_b, fk_b);
     if (!ok) return;
   }
-  constexpr int EB = NT >= 512 ? 2 : 4;
+  constexpr int EB = GROUPED ? 3 : (NT >= 512 ? 2 : 4);
   const bool tstore = MODE == SM_RK4 && vstore;
-  zfwd_update<T, P, N, NT, EB, MODE>(w, st, g, kx0, iy, nvalid, base, zstride, fblock, fblock ? s_coef : 0.0, flo_b,
+  zfwd_update<T, P, N, NT, EB, MODE>(w, st, g, kx0, iy, nvalid, base, zstride, fblock, fblock ? s_coef : T(0), flo_b,
                                      fk_b, paired, tstore);
   if (tstore) {
     fence_proxy_async();
@@ -491,11 +535,11 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
 template <typename T> struct DivArgs {
   const C2<T>* phi;       // band forcing: += (*fcoef) phi on flo2 <= k2 < fhi2 (fcoef may be null)
   const double* fcoef;
-  double flo2, fhi2;
+  K2Lt flo2, fhi2;
   const C2<T>* vz;        // mean gradient: -= meangrad vz (vz may be null)
   T meangrad;
   int mask;               // zero k2 >= kcut2 (k2 > 0)
-  double kcut2;
+  K2Lt kcut2;
 };
 
 template <typename T, int LOGN>
@@ -520,7 +564,9 @@ zfwd_div_tma_kernel(const __grid_constant__ CUtensorMap fmap, const __grid_const
   const long long zstride = (long long)g.ny * g.nxp;
   const long long base = (long long)iy * g.nxp + kx0;
   const bool paired = kx0 == 0;   // meets its partner: both CTAs stay until then
-  if (!paired && launch_failed(err)) return;
+  __shared__ C s_col[N / 2];
+  if (paired) cluster_arrive();
+  else if (launch_failed(err)) return;
   if (threadIdx.x == 0) {
     for (int c = 0; c < 3; ++c) mbar_init(&bars[c], 1);
     fence_mbar_init();
@@ -536,7 +582,7 @@ zfwd_div_tma_kernel(const __grid_constant__ CUtensorMap fmap, const __grid_const
     E::template run_inplace<false>(w[c], tw);
   }
   const int kyi = wavenum(iy, g.ny);
-  const int lo_b = k2_lt(da.flo2), hi_b = k2_lt(da.fhi2), kc_b = k2_lt(da.kcut2);
+  const int lo_b = da.flo2.b, hi_b = da.fhi2.b, kc_b = da.kcut2.b;
   const bool fblock = da.fcoef && kx0 * kx0 + kyi * kyi < hi_b;
   const T fc = fblock ? (T)*da.fcoef : T(0);
   constexpr int EB = NT >= 512 ? 2 : 4;
@@ -564,13 +610,9 @@ zfwd_div_tma_kernel(const __grid_constant__ CUtensorMap fmap, const __grid_const
     }
   }
   if (paired) {
-    // the kx = 0 copy, as hermitian_column: zeroing and mask are the same at k and -k
-    cluster_sync();
-    const uint32_t from = iy == 0 ? cluster_rank() : (cluster_rank() ^ 1u);
-    for (int n = threadIdx.x; n < N; n += NT)
-      if (n > N / 2 || (n == 0 && iy > g.ny / 2))
-        w[0][n * P] = iy == g.ny / 2 ? czero<C>() : cconj(cluster_load(&w[0][((N - n) % N) * P], from));
-    cluster_sync();
+    // the kx = 0 copy: zeroing and mask are the same at k and -k
+    __syncthreads();
+    column_copy<1, P, N, NT>(w, s_col, iy, g.ny, [](int, int, const C& v) { return v; });
     if (!ok) return;
   }
   fence_proxy_async();

@@ -113,6 +113,29 @@ def test_kx0_copy(specns_lib, shape, prec):
 
 
 @pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape,fk", [((32, 8, 8), 2.5), ((32, 128, 16), 40.0), ((128, 16, 32), 20.0), ((64, 16, 64), 2.5),
+                                      ((16, 128, 128), 64.5)])
+def test_short_z_pencils(specns_lib, shape, fk, prec):
+    """The z kernels of short pencils (groups of threads, one component each):
+    forced RK4 steps and their adjoint, with bands of fewer and more rows than a
+    warp and of more than one kx tile."""
+    nx, ny, nz = shape
+    v = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 53, kcut=6.0)]
+    lam = [fresh(a, DT[prec]) for a in hermitian_fields(shape, 54)]
+    vd, ld = ([a.astype(np.complex128) for a in x] for x in (v, lam))
+    kw = dict(nu=0.02, dt=1e-3, fkmax=fk, eps=0.2)
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, **kw))
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, **kw)) as h:
+        h.set_state(*v)
+        out = h.adjoint_vjp(1, lam, 1)
+        h.set_state(*v)
+        h.rk4_steps(2)
+        got = h.get_state()
+    assert rel_l2(got, R.rk4_run(vd, g, 2)) < (1e-11 if prec == S.SC_FP64 else 1e-5)   # as the steps' other tests
+    assert rel_l2(out, R.rk4_step_adj(vd, ld, g)) < (1e-11 if prec == S.SC_FP64 else 1e-4)
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
 @pytest.mark.parametrize("shape", [(8, 8, 8), (32, 16, 64), (512, 8, 32)])
 @pytest.mark.parametrize("shift", [0, 4])
 def test_device_state_round_trip(specns_lib, shape, prec, shift):
