@@ -59,29 +59,24 @@ les_yinv_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, 
     fence_proxy_async();
   }
   __syncthreads();
-  const long long per = (long long)tp.ntx * tp.nouter, total = per * 6;
-  auto decode = [&](long long job, int& kx0, int& outer, int& f) {
-    f = (int)(job / per);
-    const long long t = job % per;
-    kx0 = (int)(t % tp.ntx) * P;
-    outer = (int)(t / tp.ntx);
-  };
-  auto issue = [&](long long job, int b) {
+  const int per = tp.ntx * tp.nouter, total = per * 6, step = gridDim.x;
+  auto decode = [&](int job, int& kx0, int& outer, int& f) { tile_of(tp, job, P, kx0, outer, f); };
+  auto issue = [&](int job, int b) {
     int kx0, outer, f;
     decode(job, kx0, outer, f);
     tma_issue_tile<Cfg>(buf(b), &map, &bars[b], 1, kx0, outer, f, P, Cfg::TILE_BYTES);
   };
-  long long job = blockIdx.x;
+  int job = blockIdx.x;
   if (threadIdx.x == 0 && job < total) issue(job, 0);
-  for (int it = 0; job < total; job += gridDim.x, ++it) {
+  for (int it = 0; job < total; job += step, ++it) {
     const int b = it & 1;
-    if (threadIdx.x == 0 && job + gridDim.x < total) {
+    if (threadIdx.x == 0 && job + step < total) {
       fence_proxy_async();
-      issue(job + gridDim.x, b ^ 1);
+      issue(job + step, b ^ 1);
     }
     if (!mbar_wait_bounded(&bars[b], (it >> 1) & 1, tp.err)) {
       // the copy into the other buffer still has to land
-      if (threadIdx.x == 0 && job + gridDim.x < total) mbar_wait_bounded(&bars[b ^ 1], ((it + 1) >> 1) & 1, nullptr);
+      if (threadIdx.x == 0 && job + step < total) mbar_wait_bounded(&bars[b ^ 1], ((it + 1) >> 1) & 1, nullptr);
       return;
     }
     int kx0, outer, f;
@@ -134,19 +129,15 @@ les_yfwd_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g, 
   }
   __syncthreads();
   // units of this CTA: u = blockIdx.x + i gridDim.x over [pairs | singles]
-  const long long per = (long long)tp.ntx * tp.nouter, pairs = 3 * per, units = 5 * per;
-  auto count = [&](long long n) { return n > blockIdx.x ? (int)((n - blockIdx.x - 1) / gridDim.x + 1) : 0; };
+  const int per = tp.ntx * tp.nouter, pairs = 3 * per, units = 5 * per, first = blockIdx.x, step = gridDim.x;
+  auto count = [&](int n) { return n > first ? (n - first - 1) / step + 1 : 0; };
   const int npair = count(pairs), nunit = count(units);
   const int nstream = nunit + npair;   // tiles: two per pair
   auto decode = [&](int s, int& kx0, int& outer, int& type, bool& tau) {
     const bool pr = s < 2 * npair;
     const int i = pr ? s / 2 : s - npair;
     tau = pr && !(s & 1);
-    const long long u = blockIdx.x + (long long)i * gridDim.x;
-    type = (int)(u / per);
-    const long long t = u % per;
-    kx0 = (int)(t % tp.ntx) * P;
-    outer = (int)(t / tp.ntx);
+    tile_of(tp, first + i * step, P, kx0, outer, type);
   };
   // field of a stream tile: tau_i2 (3 + i) or A_i (i) of pair i; singles 6, 7
   auto field_of = [](int type, bool tau) { return type < 3 ? (tau ? 3 + type : type) : 3 + type; };

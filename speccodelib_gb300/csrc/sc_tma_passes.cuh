@@ -127,6 +127,18 @@ template <typename T> struct TmaPass {
   int* err;               // device error word
 };
 
+// Job `job` of a pass (kx tile fastest, field slowest), in 32-bit arithmetic: the
+// jobs of every grid size stay below 2^31, and 64-bit divisions here made a 64^3
+// FP32 step 104 us instead of 102, 128^3 396 instead of 380, 256^3 2.91 ms instead of 2.85.
+template <typename T>
+__device__ __forceinline__ void tile_of(const TmaPass<T>& tp, int job, int P, int& kx0, int& outer, int& f) {
+  const int per = tp.ntx * tp.nouter;
+  f = job / per;
+  const int t = job - f * per;
+  outer = t / tp.ntx;
+  kx0 = (t - outer * tp.ntx) * P;
+}
+
 // Issue the loads of one field tile: box (P, BOX, 1) along y or (P, 1, BOX) along z.
 template <typename Cfg>
 __device__ __forceinline__ void tma_issue_tile(void* dst, const CUtensorMap* map, uint64_t* bar, int axis,
@@ -153,8 +165,8 @@ pencil_tma_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g
   extern __shared__ __align__(128) unsigned char smdyn[];
   unsigned char* smraw = align128(smdyn);
   __shared__ __align__(8) uint64_t bars[NS];
-  const long long total = (long long)tp.ntx * tp.nouter * tp.nf;
-  if (launch_failed(tp.err)) return;
+  const int total = tp.ntx * tp.nouter * tp.nf;
+  const bool failed = launch_failed(tp.err);
   if (threadIdx.x == 0) {
     for (int b = 0; b < NS; ++b) mbar_init(&bars[b], 1);
     fence_mbar_init();
@@ -165,29 +177,24 @@ pencil_tma_kernel(const __grid_constant__ CUtensorMap map, TmaPass<T> tp, Geom g
   // field slowest: the CTAs in flight work on neighbouring tiles of one
   // field (field fastest, six fields at the same offset, measured 12%
   // slower for the six-field inverse y-pass)
-  auto decode = [&](long long job, int& kx0, int& outer, int& f) {
-    const long long per = (long long)tp.ntx * tp.nouter;
-    f = (int)(job / per);
-    const long long t = job % per;
-    kx0 = (int)(t % tp.ntx) * P;
-    outer = (int)(t / tp.ntx);
-  };
-  auto issue = [&](long long job, int b) {
+  auto decode = [&](int job, int& kx0, int& outer, int& f) { tile_of(tp, job, P, kx0, outer, f); };
+  auto issue = [&](int job, int b) {
     int kx0, outer, f;
     decode(job, kx0, outer, f);
     tma_issue_tile<Cfg>(buf(b), &map, &bars[b], tp.axis, kx0, outer, f, P, Cfg::TILE_BYTES);
   };
+  if (failed) return;
   // prologue: the first NS-1 jobs of this CTA in flight
   if (threadIdx.x == 0) {
     for (int k = 0; k < NS - 1; ++k) {
-      const long long jk = blockIdx.x + (long long)k * gridDim.x;
+      const int jk = blockIdx.x + k * gridDim.x;
       if (jk < total) issue(jk, k);
     }
   }
-  long long job = blockIdx.x;
+  int job = blockIdx.x;
   for (int it = 0; job < total; job += gridDim.x, ++it) {
     const int b = it % NS;
-    const long long ahead = job + (long long)(NS - 1) * gridDim.x;
+    const int ahead = job + (NS - 1) * gridDim.x;
     if (threadIdx.x == 0 && ahead < total) {
       fence_proxy_async();
       issue(ahead, (it + NS - 1) % NS);
