@@ -400,18 +400,21 @@ __host__ __device__ constexpr bool mode_reads_v(int m) {
 __host__ __device__ constexpr bool mode_reads_acc(int m) {
   return m == SM_RK2 || m == SM_RK3 || m == SM_RK4 || m == SM_AB2;
 }
+__host__ __device__ constexpr bool mode_reads_factor(int m) {
+  return m == SM_RK1 || m == SM_RK2 || m == SM_RK3 || m == SM_AB2_EULER || m == SM_AB2 || m == SM_AB2_MID;
+}
 
 // Projection, optional RHS mask and the mode's update at one point, with the
 // state (v, or v0 for the AB2 midpoint pass) and accumulator values already
 // loaded.  w is the right-hand side after forcing and symmetrize.  With
 // `snext` given, RK stages 1-3 return the next stage input there instead of
-// storing it to st.sout.  kcut_b = st.kcut2.b, computed once per
-// kernel.  MODE >= 0: the update mode as a compile-time constant (st.mode
+// storing it to st.sout.  kcut_b = st.kcut2.b.  E: the integrating factor
+// ex ey ez where mode_reads_factor.  MODE >= 0: the update mode as a compile-time constant (st.mode
 // otherwise).
 template <typename T, int MODE = -1>
 __device__ __forceinline__ void finish_point_pre(const StageArgs<T>& st, const Geom& g, long long idx,
                                                  int ix, int iy, int iz, int kcut_b, C2<T>* w, const C2<T>* vv,
-                                                 const C2<T>* av, C2<T>* snext = nullptr) {
+                                                 const C2<T>* av, C2<T>* snext, T E) {
   using C = C2<T>;
   const int kyi = wavenum(iy, g.ny), kzi = wavenum(iz, g.nz);
   const int k2i = ix * ix + kyi * kyi + kzi * kzi;
@@ -460,7 +463,6 @@ __device__ __forceinline__ void finish_point_pre(const StageArgs<T>& st, const G
     for (int c = 0; c < 3; ++c) st.w[c][idx] = w[c];
     return;
   }
-  const T E = st.ex[ix] * st.ey[iy] * st.ez[iz];
   const T E2 = E * E;
   const T dt = st.dt, hdt = T(0.5) * st.dt;
   const bool zero_mean_cut = cut || (ix == 0 && iy == 0 && iz == 0);
@@ -546,7 +548,8 @@ __device__ __forceinline__ void finish_point(const StageArgs<T>& st, const Geom&
                                              int ix, int iy, int iz, int kcut_b, C2<T>* w) {
   C2<T> vv[3], av[3];
   load_state<T, MODE>(st, idx, vv, av);
-  finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kcut_b, w, vv, av);
+  const T E = mode_reads_factor(MODE >= 0 ? MODE : st.mode) ? st.ex[ix] * st.ey[iy] * st.ez[iz] : T(1);
+  finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kcut_b, w, vv, av, nullptr, E);
 }
 
 // K_f of force.f90:16-22 from the zinv partial sums, fixed order.

@@ -346,11 +346,30 @@ zfwd_fields_tma_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st
   zfwd_finish<E, T>(w, st, g, kx0, iy, nvalid, base, zstride, s_coef);
 }
 
+// State, accumulator and integrating factor ez of EB points n0 + i RS of a z
+// pencil (those below N); p0 is the pencil's first point.  The factor comes with
+// the state: loaded at its use it waited for the stores of the point before.
+template <typename T, int EB> struct UpdateBatch {
+  C2<T> v[EB][3], a[EB][3];
+  T ez[EB];
+  template <int MODE, int N, int RS>
+  __device__ __forceinline__ void load(const StageArgs<T>& st, int n0, long long p0, long long zstride, bool factor) {
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      const int iz = n0 + i * RS;
+      if (iz >= N) continue;
+      load_state<T, MODE>(st, p0 + iz * zstride, v[i], a[i]);
+      ez[i] = factor ? st.ez[iz] : T(1);
+    }
+  }
+};
+
 // The z-forward's spectral update of tile (kx0, iy) from the transformed
 // right-hand side in the tiles w (element (p, n) at n P + p; forcing and
 // symmetrize's copy of the kx = 0 column already in them when `paired`), in
 // batches of EB points per thread: all state loads of a batch are issued
-// before any of them is used.  fblock: the tile meets the forcing band, whose
+// before any of them is used (the next batch's before this one is worked on, as
+// zfwd_zinv does, gained nothing here).  fblock: the tile meets the forcing band, whose
 // coefficient is coef.  tstore (RK stage 4): the new state goes back into the
 // tiles.
 template <typename T, int P, int N, int NT, int EB, int MODE>
@@ -358,29 +377,23 @@ __device__ __forceinline__ void zfwd_update(C2<T>* const w[3], const StageArgs<T
                                             int nvalid, long long base, long long zstride, bool fblock, T coef,
                                             int flo_b, int fk_b, bool paired, bool tstore) {
   using C = C2<T>;
+  static_assert(NT % P == 0, "a thread keeps its kx");
+  constexpr int RS = NT / P;
   const int kyi = wavenum(iy, g.ny), kc_b = st.kcut2.b;
-  for (int e0 = threadIdx.x; e0 < P * N; e0 += NT * EB) {
-    C wv[EB][3], vv[EB][3], av[EB][3];
-    bool act[EB];
+  const int p = threadIdx.x % P, ix = kx0 + p;
+  if (p >= nvalid) return;
+  const bool factor = mode_reads_factor(MODE >= 0 ? MODE : st.mode);
+  const T exy = factor ? st.ex[ix] * st.ey[iy] : T(1);
+#pragma unroll 1
+  for (int n0 = threadIdx.x / P; n0 < N; n0 += RS * EB) {
+    UpdateBatch<T, EB> cur;
+    cur.template load<MODE, N, RS>(st, n0, base + p, zstride, factor);
 #pragma unroll
     for (int i = 0; i < EB; ++i) {
-      const int e = e0 + i * NT;
-      const int p = e % P, iz = e / P;
-      act[i] = e < P * N && p < nvalid;
-      if (!act[i]) continue;
+      const int iz = n0 + i * RS;
+      if (iz >= N) continue;
       const long long idx = base + iz * zstride + p;
-      load_state<T, MODE>(st, idx, vv[i], av[i]);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) wv[i][c] = w[c][e];
-    }
-#pragma unroll
-    for (int i = 0; i < EB; ++i) {
-      if (!act[i]) continue;
-      const int e = e0 + i * NT;
-      const int p = e % P, iz = e / P;
-      const int ix = kx0 + p;
-      const long long idx = base + iz * zstride + p;
-      C* wp = wv[i];
+      C wp[3] = {w[0][iz * P + p], w[1][iz * P + p], w[2][iz * P + p]};
       if (fblock && !(paired && ix == 0)) {
         const int kz = wavenum(iz, g.nz);
         const int k2 = ix * ix + kyi * kyi + kz * kz;
@@ -396,11 +409,11 @@ __device__ __forceinline__ void zfwd_update(C2<T>* const w[3], const StageArgs<T
       }
       if (tstore) {
         C vn[3];
-        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, vv[i], av[i], vn);
+        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, cur.v[i], cur.a[i], vn, exy * cur.ez[i]);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) w[c][e] = vn[c];
+        for (int c = 0; c < 3; ++c) w[c][iz * P + p] = vn[c];
       } else {
-        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, vv[i], av[i]);
+        finish_point_pre<T, MODE>(st, g, idx, ix, iy, iz, kc_b, wp, cur.v[i], cur.a[i], nullptr, exy * cur.ez[i]);
       }
     }
   }
