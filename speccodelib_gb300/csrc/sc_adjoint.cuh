@@ -246,7 +246,8 @@ zfwd_adj_kernel(FieldList<T> fin, AdjArgs<T> aa, Geom g, const C2<T>* __restrict
   adj_epilogue<E, T>(l, aa, g, kx0, iy, nvalid, base, zstride, fblock, s_a, s_b);
 }
 
-// The same with the six product tiles fetched by TMA, two in flight: field
+// The same with the six product tiles fetched by TMA, two in flight (pencils whose
+// six tiles do not fit in shared memory; the others: zfwd_adj_group_kernel): field
 // f + 2 loads while field f is transformed.  fidx maps the kernel's field
 // order (0-2: w x phi, 3-5: phi x u) to the tensor map's field index.
 template <typename T, int LOGN> struct AdjTmaCfg {
@@ -329,6 +330,157 @@ zfwd_adj_tma_kernel(const __grid_constant__ CUtensorMap pmap, int4 fidx_lo, int2
     adj_accum<E, T>(l, o, f, kx0, ky, g);
   }
   adj_epilogue<E, T>(l, aa, g, kx0, iy, nvalid, base, zstride, fblock, s_a, s_b);
+}
+
+// The z-forward with its six product tiles resident, for pencils whose tiles fit:
+// kx and ky are constant along a z pencil, so only B_x and B_y (B = phi x u, which
+// meet kz) and the combinations
+//   X = A_x + i ky B_z,  Y = A_y - i kx B_z,  Z = A_z + i kx B_y - i ky B_x
+// (A = w x phi) are transformed, five instead of six, by three groups of threads
+// (group c: X, Y or Z in its tile, then B_x, B_y); then per point
+//   lam_s = D' (X - i kz B_y, Y + i kz B_x, Z).
+// Bound by latency and barriers (3.3 TB/s at 128^3).  Against zfwd_adj_tma_kernel,
+// which serves the pencils whose tiles do not fit: 48.5 -> 39.5 us at 128^3 FP32,
+// ten adjoint steps at 32^3 FP32 2.08 -> 1.90 ms, 256^3 90.0 -> 87.8 ms, 128^3 FP64
+// 154.8 -> 150.6 ms.  Two jobs per thread below 256 points: 128^3 11.8 -> 11.9 ms.
+template <typename T, int LOGN> struct AdjGrpCfg {
+  using Cfg = TmaCfg<T, LOGN>;
+  static constexpr int P = AdjTmaCfg<T, LOGN>::P;   // the product map's tiles
+  static constexpr int N = Cfg::N;
+  static constexpr int NTG_RAW = P * N / (LOGN >= 8 ? 16 : 8);   // 16 points: the two-pass transforms
+  static constexpr int NTG = NTG_RAW < 32 ? 32 : NTG_RAW;
+  static constexpr int NT = 3 * NTG;
+  using Engine = FFTEngine<T, LOGN, P, P, NTG, true, 0, true, 8, true>;
+  static constexpr size_t TILE = sizeof(C2<T>) * N * P;
+  static constexpr size_t SMEM = 6 * TILE + kSmemAlignPad;
+  static constexpr bool SUPPORTED = SMEM <= 226 * 1024 && NT <= 1024;
+  static constexpr int MINB_S = (int)(233472 / (SMEM + 1024)), MINB_T = 1024 / NT;
+  static constexpr int MINB_M = MINB_S < MINB_T ? MINB_S : MINB_T;
+  static constexpr int MINB = MINB_M < 1 ? 1 : (MINB_M > 8 ? 8 : MINB_M);
+};
+
+// The transposed Lawson RK4 stage at a point: ls = lam_s with the forcing adjoint,
+// E the integrating factor, lt / lv the loaded state (the stages' expressions).
+template <int STAGE, typename T, typename C>
+__device__ __forceinline__ void adj_stage_point(const AdjArgs<T>& aa, long long idx, bool cut, T E, const C* ls,
+                                                const C* lt, const C* lv) {
+  const T dt = aa.dt;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if constexpr (STAGE == ADJ4) {
+      aa.lv[c][idx] = cscale(cadd(lt[c], ls[c]), E * E);
+      aa.lw[c][idx] = cadd(cscale(lt[c], E * dt / T(3)), cscale(ls[c], E * dt));
+    } else if constexpr (STAGE == ADJ3) {
+      aa.lv[c][idx] = cadd(lv[c], cscale(ls[c], E));
+      aa.lw[c][idx] = cadd(cscale(lt[c], E * dt / T(3)), cscale(ls[c], T(0.5) * dt));
+    } else if constexpr (STAGE == ADJ2) {
+      aa.lv[c][idx] = cadd(lv[c], cscale(ls[c], E));
+      aa.lw[c][idx] = cadd(cscale(lt[c], E * E * dt / T(6)), cscale(ls[c], T(0.5) * E * dt));
+    } else {
+      const C lm = cadd(lv[c], ls[c]);
+      if (aa.write_lam) aa.lam[c][idx] = lm;
+      if (aa.chain) {
+        const C l0 = cut ? czero<C>() : lm;
+        aa.lt_next[c][idx] = l0;
+        aa.lw[c][idx] = cscale(l0, dt / T(6));
+      }
+    }
+  }
+}
+
+template <typename T, int LOGN, int STAGE>
+__global__ void __launch_bounds__(AdjGrpCfg<T, LOGN>::NT, AdjGrpCfg<T, LOGN>::MINB)
+zfwd_adj_group_kernel(const __grid_constant__ CUtensorMap pmap, int4 fidx_lo, int2 fidx_hi, AdjArgs<T> aa, Geom g,
+                      const C2<T>* __restrict__ tw, int* err) {
+  pdl_wait();
+  using AC = AdjGrpCfg<T, LOGN>;
+  using Cfg = TmaCfg<T, LOGN>;
+  using E = typename AC::Engine;
+  using C = C2<T>;
+  constexpr int P = AC::P, N = AC::N, NT = AC::NT, NTG = AC::NTG, TE = P * N;
+  extern __shared__ __align__(128) unsigned char smdyn[];
+  C* const A = reinterpret_cast<C*>(align128(smdyn));   // A_x, A_y, A_z, B_x, B_y, B_z
+  C* const B = A + 3 * TE;
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ T s_a, s_b;
+  const int kx0 = blockIdx.x * P, iy = blockIdx.y, kyi = wavenum(iy, g.ny);
+  const int nvalid = min(P, g.nxh - kx0);
+  const long long zstride = (long long)g.ny * g.nxp;
+  const long long base = (long long)iy * g.nxp + kx0;
+  const bool failed = launch_failed(err);
+  if (threadIdx.x == 0) {
+    const int fidx[6] = {fidx_lo.x, fidx_lo.y, fidx_lo.z, fidx_lo.w, fidx_hi.x, fidx_hi.y};
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+    fence_proxy_async();
+    mbar_arrive_expect_tx(&bar, (uint32_t)(6 * AC::TILE));
+    for (int f = 0; f < 6; ++f)
+      for (int h = 0; h < Cfg::NBOX; ++h)
+        tma_load_4d(A + (size_t)f * TE + (size_t)h * Cfg::BOX * P, &pmap, &bar, kx0 * Cfg::U, iy, h * Cfg::BOX, fidx[f]);
+  }
+  const int fk_b = aa.fkmax2.b, kc_b = aa.kcut2.b;
+  const bool fblock = aa.forced && kx0 * kx0 + kyi * kyi < fk_b;
+  if (fblock && threadIdx.x >= NT - 32) adj_band_coef<T>(aa, g, s_a, s_b);
+  __syncthreads();
+  if (!__syncthreads_and(mbar_wait_bounded(&bar, 0, err) && !failed)) return;
+  const T ky = (T)kyi;
+  const int grp = threadIdx.x / NTG;
+  C* const t = A + (size_t)grp * TE;
+  for (int e = threadIdx.x % NTG; e < TE; e += NTG) {
+    const T kx = (T)(kx0 + e % P);
+    C x = t[e];
+    if (grp == 0) x = cadd(x, cmuli(cscale(B[2 * TE + e], ky)));
+    else if (grp == 1) x = csub(x, cmuli(cscale(B[2 * TE + e], kx)));
+    else x = cadd(x, cmuli(csub(cscale(B[TE + e], kx), cscale(B[e], ky))));
+    t[e] = x;
+  }
+  __syncthreads();   // B_x and B_y are read
+  E::template run_inplace<false>(t, tw);
+  if (grp < 2) E::template run_inplace<false>(B + (size_t)grp * TE, tw);
+  __syncthreads();
+  // in batches of EB points per thread, every load issued before the first store
+  constexpr int EB = 2, RS = NT / P;
+  static_assert(NT % P == 0, "a thread keeps its kx");
+  const int p = threadIdx.x % P, ix = kx0 + p;
+  if (p >= nvalid) return;
+  const T dp = (ix == 0 || ix == g.nxh - 1) ? T(1) : T(2);
+  const T exy = aa.ex[ix] * aa.ey[iy];
+#pragma unroll 1
+  for (int n0 = threadIdx.x / P; n0 < N; n0 += RS * EB) {
+    C lt[EB][3], lv[EB][3];
+    T ez[EB];
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      const int iz = n0 + i * RS;
+      if (iz >= N) continue;
+      const long long idx = base + iz * zstride + p;
+      ez[i] = aa.ez[iz];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (STAGE != ADJ1) lt[i][c] = aa.lt[c][idx];
+        if (STAGE != ADJ4) lv[i][c] = aa.lv[c][idx];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      const int iz = n0 + i * RS, e = iz * P + p;
+      if (iz >= N) continue;
+      const long long idx = base + iz * zstride + p;
+      const int kzi = wavenum(iz, g.nz), k2i = ix * ix + kyi * kyi + kzi * kzi;
+      const T kz = (T)kzi;
+      C ls[3] = {cscale(csub(A[e], cmuli(cscale(B[TE + e], kz))), dp),
+                 cscale(cadd(A[TE + e], cmuli(cscale(B[e], kz))), dp), cscale(A[2 * TE + e], dp)};
+      if (fblock && k2i < fk_b) {
+        C m[3] = {aa.lw[0][idx], aa.lw[1][idx], aa.lw[2][idx]};
+        adj_mu<C, T>(m, ix, iy, iz, g, aa.mask_rhs, kc_b);
+        const T sb = ix == 0 ? T(0.5) * s_b : s_b;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          ls[c] = cadd(ls[c], csub(cscale(m[c], s_a), cscale(aa.s[c][idx], sb)));
+      }
+      adj_stage_point<STAGE, T>(aa, idx, k2i >= kc_b && k2i > 0, exy * ez[i], ls, lt[i], lv[i]);
+    }
+  }
 }
 
 // Transpose of symmetrize's kx = 0 conjugate copies, in place on lw:

@@ -301,17 +301,37 @@ cudaError_t launch_zfwd_adj(const FieldList<T>& fin, const AdjArgs<T>& aa, const
   return cudaGetLastError();
 }
 
-template <typename T, int LOGN>
-cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], const AdjArgs<T>& aa, const Geom& g,
-                                const C2<T>* tw, int* err, cudaStream_t s) {
-  using AC = AdjTmaCfg<T, LOGN>;
-  auto k = zfwd_adj_tma_kernel<T, LOGN>;
+template <typename T, int LOGN, int STAGE>
+cudaError_t launch_zfwd_adj_group(const CUtensorMap& pmap, int4 lo, int2 hi, const AdjArgs<T>& aa, const Geom& g,
+                                  const C2<T>* tw, int* err, cudaStream_t s) {
+  using AC = AdjGrpCfg<T, LOGN>;
+  auto k = zfwd_adj_group_kernel<T, LOGN, STAGE>;
   static cudaError_t attr = smem_attr(k, AC::SMEM);
   if (attr != cudaSuccess) return attr;
   dim3 grid((g.nxh + AC::P - 1) / AC::P, g.ny);
+  return launch_pdl(k, grid, dim3(AC::NT), AC::SMEM, s, pmap, lo, hi, aa, g, tw, err);
+}
+
+template <typename T, int LOGN>
+cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], const AdjArgs<T>& aa, const Geom& g,
+                                const C2<T>* tw, int* err, cudaStream_t s) {
   const int4 lo = make_int4(fidx[0], fidx[1], fidx[2], fidx[3]);
   const int2 hi = make_int2(fidx[4], fidx[5]);
-  return launch_pdl(k, grid, dim3(AC::NT), AC::SMEM, s, pmap, lo, hi, aa, g, tw, err);
+  if constexpr (AdjGrpCfg<T, LOGN>::SUPPORTED) {
+    switch (aa.stage) {
+      case ADJ4: return launch_zfwd_adj_group<T, LOGN, ADJ4>(pmap, lo, hi, aa, g, tw, err, s);
+      case ADJ3: return launch_zfwd_adj_group<T, LOGN, ADJ3>(pmap, lo, hi, aa, g, tw, err, s);
+      case ADJ2: return launch_zfwd_adj_group<T, LOGN, ADJ2>(pmap, lo, hi, aa, g, tw, err, s);
+      default: return launch_zfwd_adj_group<T, LOGN, ADJ1>(pmap, lo, hi, aa, g, tw, err, s);
+    }
+  } else {
+    using AC = AdjTmaCfg<T, LOGN>;
+    auto k = zfwd_adj_tma_kernel<T, LOGN>;
+    static cudaError_t attr = smem_attr(k, AC::SMEM);
+    if (attr != cudaSuccess) return attr;
+    dim3 grid((g.nxh + AC::P - 1) / AC::P, g.ny);
+    return launch_pdl(k, grid, dim3(AC::NT), AC::SMEM, s, pmap, lo, hi, aa, g, tw, err);
+  }
 }
 
 }  // namespace sc

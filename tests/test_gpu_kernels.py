@@ -136,6 +136,23 @@ def test_short_z_pencils(specns_lib, shape, fk, prec):
 
 
 @pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", [(16, 8, 256), (32, 8, 512), (16, 8, 1024)])
+def test_vjp_long_z_pencils(specns_lib, shape, prec):
+    """The adjoint's z-forward on long pencils: resident tiles (groups of threads)
+    to 512 points, two tiles in flight beyond; band of more than one kx tile."""
+    nx, ny, nz = shape
+    v = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 55, kcut=6.0)]
+    lam = [fresh(a, DT[prec]) for a in hermitian_fields(shape, 56)]
+    kw = dict(nu=0.02, dt=1e-3, fkmax=9.0, eps=0.2)
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, **kw))
+    ref = R.rk4_step_adj([a.astype(np.complex128) for a in v], [a.astype(np.complex128) for a in lam], g)
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, **kw)) as h:
+        h.set_state(*v)
+        out = h.adjoint_vjp(1, lam, 1)
+    assert rel_l2(out, ref) < (1e-11 if prec == S.SC_FP64 else 1e-4)   # the bounds of the adjoint's other tests
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
 @pytest.mark.parametrize("shape", [(8, 8, 8), (32, 16, 64), (512, 8, 32)])
 @pytest.mark.parametrize("shift", [0, 4])
 def test_device_state_round_trip(specns_lib, shape, prec, shift):
