@@ -289,8 +289,9 @@ int sc_ens_get_member(sc_ensemble* e, int m, void* w);
  * the 2/3 mask); seeds[m] per member (only seeds <= 0 select distinct ran1
  * streams, initialize.f90:530) */
 int sc_ens_init(sc_ensemble* e, const int* seeds, double kpeak, double energy);
-/* nsteps IF-RK4 steps of every member.  mode 0: one cooperative launch per
- * stage for all members, a whole step replayed as a CUDA graph; mode 1: the
+/* nsteps IF-RK4 steps of every member.  mode 0: all members
+ * together (one cooperative launch per stage, or one launch per pass and member
+ * size, as the tuner finds faster), a whole step replayed as a CUDA graph; mode 1: the
  * same launches without the graph; mode 2: the members one at a time. */
 int sc_ens_rk4_steps(sc_ensemble* e, int nsteps, int mode);
 /* 1 if mode 0 is running from a captured graph */

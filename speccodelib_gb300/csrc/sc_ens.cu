@@ -1,6 +1,6 @@
 // Host side of the batched 2D vorticity ensembles (sc_ens_* in
-// include/specns.h): member storage, the seeded initial vorticity, one
-// cooperative launch per RK stage, and the CUDA graph of a whole step.
+// include/specns.h): member storage, the seeded initial vorticity, the launches of
+// a stage (one cooperative, or one per pass), and the CUDA graph of a whole step.
 #include <cuda_runtime.h>
 
 #include <cmath>

@@ -1,5 +1,6 @@
 // Batched 2D vorticity ensembles: members of mixed size N advance together,
-// one persistent (cooperative) launch per RK stage.
+// one persistent (cooperative) launch per RK stage (sc_ens_split.cuh: a launch per
+// pass).
 //
 // Physics per member (restated from the 2D solvers of the reference:
 // spectral_dns_2d.f90:94,160-188 and turb_2d.f90:288-403):
