@@ -18,7 +18,8 @@
 // w_x = i (ky s_z - kz s_y) and w_y = i (kz s_x - kx s_z) carry kz and are
 // transformed, half a tile (P/2 pencils) at a time through a half-size work
 // buffer.  Shared memory per CTA: the three s tiles + the half work tile,
-// 112 KB for 32 KB tiles, so two CTAs share an SM.
+// 112 KB for 32 KB tiles, so two CTAs share an SM.  Short pencils take six tiles
+// and three groups of threads (ZgCfg).
 #pragma once
 #include "sc_tma_passes.cuh"
 #include "sc_tmem.cuh"
