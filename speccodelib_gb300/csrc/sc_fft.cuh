@@ -160,7 +160,9 @@ struct FFTEngine {
   static constexpr int JL = (TOTL + NT - 1) / NT;
   // GROUPED: NT threads are one of several groups of a CTA, each with a
   // transform of its own and barrier 1 + group for its stages (NT a multiple
-  // of 32 and a power of two).
+  // of 32 and a power of two).  That barrier waits for NT threads whether or not
+  // some have left, so a CTA that uses it exits uniformly: a give-up (a bounded
+  // wait, the error word) is agreed by __syncthreads_and before a thread returns.
   __device__ static __forceinline__ int tid() { return GROUPED ? threadIdx.x % NT : threadIdx.x; }
   __device__ static __forceinline__ void sync() {
     if constexpr (GROUPED) asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / NT), "n"(NT) : "memory");

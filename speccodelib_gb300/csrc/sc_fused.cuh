@@ -464,7 +464,7 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
   const int nvalid = min(P, g.nxh - kx0);
   const long long zstride = (long long)g.ny * g.nxp;
   const long long base = (long long)iy * g.nxp + kx0;
-  if (launch_failed(err)) return;
+  const bool failed = launch_failed(err);
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init();
@@ -476,7 +476,7 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
                     kx0 * Cfg::U, iy, h * Cfg::BOX, c);
   }
   __syncthreads();
-  if (!mbar_wait_bounded(&bar, 0, err)) return;
+  if (!__syncthreads_and(mbar_wait_bounded(&bar, 0, err) && !failed)) return;
   const int kyi = wavenum(iy, g.ny), fk_b = za.fs.fkmax2.b, kc_b = za.kcut2.b;
   const bool fsum = za.fs.enabled && kx0 * kx0 + kyi * kyi < fk_b;
   double q = 0.0;
@@ -504,11 +504,11 @@ zinv_phi_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_const
     const double s2 = block_sum<NT>(q, red);
     if (threadIdx.x == 0) za.cpartial[(long long)blockIdx.x * g.ny + iy] = s2;
   }
-  // 256- and 512-point pencils (two-pass in-place transforms): phi in place
-  // in the tiles, then out by bulk tensor stores (omap tiles the three
-  // outputs as lmap tiles lam; columns past nx/2+1 lie outside it and are
-  // not written).  Shorter pencils: element stores from the transform's
-  // registers (the bulk form gained nothing at 128^3).
+  // 256- and 512-point pencils (two-pass in-place transforms) and the short ones
+  // of ZgCfg (a group of threads per component): phi in place in the tiles, then
+  // out by bulk tensor stores (omap tiles the three outputs as lmap tiles lam;
+  // columns past nx/2+1 lie outside it and are not written).  The others: element
+  // stores from the transform's registers.
   if ((EF::TWO_PASS || Z::GROUPED) && za.ustore) {
     if constexpr (Z::GROUPED) {
       Z::ZG::Engine::template run_inplace<true>(rt[0] + (size_t)(threadIdx.x / Z::ZG::NTG) * P * N, tw);
