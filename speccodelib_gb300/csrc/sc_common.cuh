@@ -93,6 +93,15 @@ struct K2Lt {   // k2 < t  <=>  k2 < b
   K2Lt(double t) : b(k2_lt(t)) {}
 };
 
+// Largest k <= kmax with k^2 < b (0 for b <= 1): the reach of a band along an
+// axis whose wavenumbers end at kmax.  The bound keeps the squares below 2^31
+// where b is clamped there (k2_clamp), so that the search ends.
+__host__ __device__ inline int band_reach(int b, int kmax) {
+  int k = 0;
+  while (k < kmax && (k + 1) * (k + 1) < b) ++k;
+  return k;
+}
+
 // floor(sqrt(k2) + 1/2) for an integer k2 >= 0, exactly: the n with
 // n^2 - n < k2 <= n^2 + n (a float root is within one of it).
 __host__ __device__ __forceinline__ int shell_index(int k2) {

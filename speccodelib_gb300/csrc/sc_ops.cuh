@@ -388,8 +388,7 @@ __global__ void __launch_bounds__(256) band_coef_kernel(BandArgs<T> ba, Geom g) 
   pdl_wait();
   __shared__ double red[256 / 32 + 1];
   const int lo_b = ba.lo2.b, hi_b = ba.hi2.b;
-  int kb = 0;
-  while ((kb + 1) * (kb + 1) < hi_b) ++kb;   // largest |k_i| with k_i^2 < hi2
+  const int kb = band_reach(hi_b, max(g.nxh - 1, max(g.ny, g.nz) / 2));
   const int nkx = min(kb, g.nxh - 1) + 1;
   const int ky0 = max(-kb, -g.ny / 2), ky1 = min(kb, g.ny / 2 - 1);
   const int kz0 = max(-kb, -g.nz / 2), kz1 = min(kb, g.nz / 2 - 1);

@@ -231,3 +231,27 @@ def test_les_passes(specns_lib, shape, prec):
     assert rel_l2(w, R.ratesdudt(vd, g)) < TOL[prec]
     assert rel_l2(out, R.rk4_run(vd, g, 1)) < TOL[prec]
     assert rel_l2(var, R.ab2v_run(vd, g, (1e-3,))[0]) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("fk2", [1e5, 12.0])
+def test_wide_rotating_band(specns_lib, fk2, prec):
+    """Forcing bands as wide as the grid and wider, the squared upper bound past
+    2^31 among them: the rotating solvers with and without a scalar."""
+    nx, ny, nz = shape = (32, 16, 64)
+    f = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 67, ncomp=4, kcut=6.0)]
+    kw = dict(nu=0.02, dt=1e-3, eps=0.2)
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, **kw))
+    fd = [a.astype(np.complex128) for a in f]
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, **kw)) as h:
+        h.set_state(*f[:3])
+        h.set_scalar(f[3])
+        h.rot_scalar_steps(2, om=2.0, fk1=1.0, fk2=fk2, pr=0.7, scalarforced=True, epsphi=0.05)
+        both = list(h.get_state()) + [h.get_scalar()]
+        h.set_state(*f[:3])
+        h.rot_steps(2, om=2.0, fk1=1.0, fk2=fk2)
+        alone = h.get_state()
+    v, phi, _, _ = R.rot_scalar_run(fd[:3], fd[3], g, 2, 2.0, 1.0, fk2, 0.7, True, 0.05)
+    assert rel_l2(both[:3], v) < TOL[prec]
+    assert rel_l2(both[3], phi) < TOL[prec]
+    assert rel_l2(alone, R.rot_run(fd[:3], g, 2, 2.0, 1.0, fk2)[0]) < TOL[prec]

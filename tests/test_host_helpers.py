@@ -379,3 +379,35 @@ def test_variable_step_scalar_update_matches_oracle(tmp_path, history):
         assert rel_l2(out[0, p, 3], pref) < 1e-13, p
         assert rel_l2(list(out[1, p, :3]), list(vref)) < 1e-5, p
         assert rel_l2(out[1, p, 3], pref) < 1e-5, p
+
+
+REACH_PROGRAM = r'''
+#include <cstdio>
+#include "sc_common.cuh"
+int main() {
+  const int kmaxs[] = {4, 5, 64, 512};
+  const double ts[] = {0.0, 0.5, 1.0, 1.5, 6.25, 16.0, 17.0, 262144.0, 262145.0, 2147395600.0, 2147483646.0, 1e10, 1e300};
+  for (int kmax : kmaxs)
+    for (double t : ts) {
+      int k = 0;   // in doubles, which hold every square here
+      while (k < kmax && (double)(k + 1) * (k + 1) < t) ++k;
+      if (sc::band_reach(sc::k2_lt(t), kmax) != k) { std::printf("%d %g\n", kmax, t); return 1; }
+    }
+  return 0;
+}
+'''
+
+
+def test_band_reach(tmp_path):
+    """The reach of a forcing band ends at the axis for bounds of every size,
+    those past 2^31 included."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    src, exe = tmp_path / "reach.cu", tmp_path / "reach"
+    src.write_text(REACH_PROGRAM)
+    r = subprocess.run([nvcc, "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC, str(src), "-o", str(exe)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout[-500:]
