@@ -611,7 +611,7 @@ zfwd_zinv_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_cons
   ok = __syncthreads_and(ok);
   if (!ok && !paired) return;
   if (paired) {
-    hermitian_column<T, P, N, NT>(rt, work, st, g, iy, base, zstride, band, band ? s_coef : T(0), 0, fk_b);
+    hermitian_column<T, P, N, NT, true>(rt, work, st, g, iy, base, zstride, band, band ? s_coef : T(0), 0, fk_b);
     if (!ok) return;
   }
   // spectral update; the next stage input goes back into the tiles

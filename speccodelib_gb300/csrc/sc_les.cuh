@@ -285,7 +285,7 @@ les_zfwd_kernel(const __grid_constant__ CUtensorMap fmap, StageArgs<T> st, Geom 
   __syncthreads();
   if (paired) {
     cluster_arrive();   // tau is free for the partner's column
-    hermitian_column<T, P, N, NT>(w, tau, st, g, iy, base, zstride, fblock, fblock ? s_coef : T(0), 0, fk_b);
+    hermitian_column<T, P, N, NT, true>(w, tau, st, g, iy, base, zstride, fblock, fblock ? s_coef : T(0), 0, fk_b);
     if (!ok) return;
   }
   zfwd_update<T, P, N, NT, 2, MODE>(w, st, g, kx0, iy, nvalid, base, zstride, fblock, fblock ? s_coef : T(0), 0, fk_b,

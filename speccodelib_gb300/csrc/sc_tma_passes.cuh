@@ -68,45 +68,50 @@ __device__ __forceinline__ int paired_row(int b, int ny) {
 // Hermitian copy of symmetrize.f90:52-62 on the kx = 0 column (p = 0) of the
 // NF tiles w: the targets (kz index over nz/2, and ky index over ny/2 at kz = 0)
 // take the conjugates of w(-ky, -kz) from the partner CTA (from the own tiles at
-// ky = 0).  Each CTA pushes its column into the partner's `col` (NF N/2 values)
-// through distributed shared memory, so one cluster barrier is waited for; the
-// caller has arrived once (cluster_arrive) at its start, which tells the partner
-// that this CTA's shared memory may be written.  src(c, n, w) gives the column's
-// value from the tile's (and may change the tile).  This replaces a side buffer, a
-// fix-up launch after every z-forward and, in the fused RK stages, a one-tile
-// z-inverse launch: three dependent launches per stage become one (256^3 FP32
-// step 3.08 -> 2.97 ms, 64^3 178 -> 145 us, 512^3 24.0 -> 23.5 ms).
+// ky = 0), pushed through distributed shared memory.  src(c, n, w) gives the
+// column's value from the tile's (and may change the tile).  This replaces a side
+// buffer, a fix-up launch after every z-forward and, in the fused RK stages, a
+// one-tile z-inverse launch: three dependent launches per stage become one (256^3
+// FP32 step 3.08 -> 2.97 ms, 64^3 178 -> 145 us, 512^3 24.0 -> 23.5 ms).
+// Where the values go: with COL into `col` (NF N/2 values of shared memory), from
+// which the partner fills its tiles, and the caller has arrived (cluster_arrive)
+// once its col is free; without COL straight into the partner's targets, which are
+// no sources, and the caller arrives after its barrier on the tiles.
 // Every thread of both CTAs calls it, after a barrier on the tiles; it ends with
 // a barrier.
-template <int NF, int P, int N, int NT, typename C, class F>
+template <int NF, int P, int N, int NT, bool COL, typename C, class F>
 __device__ __forceinline__ void column_copy(C* const w[], C* col, int iy, int ny, F&& src) {
   cluster_wait();
   const uint32_t to = iy == 0 ? cluster_rank() : (cluster_rank() ^ 1u);
-  for (int n = threadIdx.x; n < N / 2; n += NT)
+  for (int n = threadIdx.x; n < N / 2; n += NT) {
+    if (n == 0 && iy > ny / 2) continue;   // a target
 #pragma unroll
     for (int c = 0; c < NF; ++c) {
       const C v = cconj(src(c, n, w[c][n * P]));
-      if (iy != ny / 2 && (iy == 0 || n > 0 || iy < ny / 2)) cluster_store(&col[c * (N / 2) + n], v, to);
+      if (iy != ny / 2 && (n > 0 || iy > 0)) cluster_store(COL ? &col[c * (N / 2) + n] : &w[c][(N - n) % N * P], v, to);
     }
-  cluster_sync();
-  for (int n = threadIdx.x; n < N / 2; n += NT) {
-    if (n == 0 && iy <= ny / 2) continue;
-#pragma unroll
-    for (int c = 0; c < NF; ++c) w[c][(N - n) % N * P] = iy == ny / 2 ? czero<C>() : col[c * (N / 2) + n];
   }
-  __syncthreads();
+  cluster_sync();
+  if (COL || iy == ny / 2) {
+    for (int n = threadIdx.x; n < N / 2; n += NT) {
+      if (n == 0 && iy <= ny / 2) continue;
+#pragma unroll
+      for (int c = 0; c < NF; ++c) w[c][(N - n) % N * P] = iy == ny / 2 ? czero<C>() : col[c * (N / 2) + n];
+    }
+    __syncthreads();
+  }
 }
 
 // The same after the z-forward transform of the right-hand side and before the
 // spectral update, which treats the column like any other: forcing is added to
 // the column first.
-template <typename T, int P, int N, int NT>
+template <typename T, int P, int N, int NT, bool COL>
 __device__ __forceinline__ void hermitian_column(C2<T>* const w[3], C2<T>* col, const StageArgs<T>& st, const Geom& g,
                                                  int iy, long long base, long long zstride, bool fblock, T coef,
                                                  int flo_b, int fk_b) {
   using C = C2<T>;
   const int kyi = wavenum(iy, g.ny);
-  column_copy<3, P, N, NT>(w, col, iy, g.ny, [&](int c, int n, C& v) {
+  column_copy<3, P, N, NT, COL>(w, col, iy, g.ny, [&](int c, int n, C& v) {
     const int k2 = kyi * kyi + n * n;
     if (fblock && k2 < fk_b && k2 >= flo_b) v = cadd(v, cscale(st.sin[c][base + n * zstride], coef));
     return v;
@@ -483,8 +488,13 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
   const T ky = (T)wavenum(iy, g.ny);
   // the kx = 0 tiles meet their partner: both CTAs stay until then
   const bool paired = st.symmetrize && kx0 == 0;
-  __shared__ C s_col[3 * N / 2];
-  if (paired) cluster_arrive();
+  // The exchanged column: a buffer of its own on short pencils (the pair then
+  // waits once), else straight into the partner's tiles, which leaves the L1 to
+  // the update's loads (6 KB more per CTA of the 512-point tiles: 512^3 FP32
+  // stage 4 1.09 -> 1.24 ms, variable-step pass 2.14 -> 2.29 ms).
+  constexpr bool COL = GROUPED;
+  __shared__ C s_col[COL ? 3 * N / 2 : 1];
+  if (paired && COL) cluster_arrive();
   const bool failed = !paired && launch_failed(err);
   if (!GROUPED && failed) return;
   if (threadIdx.x == 0) {
@@ -524,7 +534,8 @@ zfwd_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant_
   ok = __syncthreads_and(ok);
   if (!ok && !paired) return;
   if (paired) {
-    hermitian_column<T, P, N, NT>(w, s_col, st, g, iy, base, zstride, fblock, fblock ? s_coef : T(0), flo_b, fk_b);
+    if (!COL) cluster_arrive();
+    hermitian_column<T, P, N, NT, COL>(w, s_col, st, g, iy, base, zstride, fblock, fblock ? s_coef : T(0), flo_b, fk_b);
     if (!ok) return;
   }
   constexpr int EB = GROUPED ? 3 : (NT >= 512 ? 2 : 4);
@@ -584,9 +595,10 @@ zfwd_div_tma_kernel(const __grid_constant__ CUtensorMap fmap, const __grid_const
   const long long zstride = (long long)g.ny * g.nxp;
   const long long base = (long long)iy * g.nxp + kx0;
   const bool paired = kx0 == 0;   // meets its partner: both CTAs stay until then
-  __shared__ C s_col[N / 2];
-  if (paired) cluster_arrive();
-  else if (launch_failed(err)) return;
+  constexpr bool COL = ZfCfg<T, LOGN>::GROUPED;   // as zfwd_tma_kernel
+  __shared__ C s_col[COL ? N / 2 : 1];
+  if (paired && COL) cluster_arrive();
+  if (!paired && launch_failed(err)) return;
   if (threadIdx.x == 0) {
     for (int c = 0; c < 3; ++c) mbar_init(&bars[c], 1);
     fence_mbar_init();
@@ -632,7 +644,8 @@ zfwd_div_tma_kernel(const __grid_constant__ CUtensorMap fmap, const __grid_const
   if (paired) {
     // the kx = 0 copy: zeroing and mask are the same at k and -k
     __syncthreads();
-    column_copy<1, P, N, NT>(w, s_col, iy, g.ny, [](int, int, const C& v) { return v; });
+    if (!COL) cluster_arrive();
+    column_copy<1, P, N, NT, COL>(w, s_col, iy, g.ny, [](int, int, const C& v) { return v; });
     if (!ok) return;
   }
   fence_proxy_async();
