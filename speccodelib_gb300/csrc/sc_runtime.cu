@@ -366,7 +366,8 @@ template <typename T> struct Impl {
     return kt * kt;
   }
 
-  // the K_f partial sums come from a z-inverse with tiles pt wide
+  // the K_f partial sums come from a z-inverse with tiles pt wide (rhs_pipeline
+  // calls it where it chooses that kernel)
   static void set_kf_tiles(sc_handle* h, sc::StageArgs<T>& st, int pt) {
     int nt = 0;
     const int ntiles = (h->g.nxh + pt - 1) / pt;
@@ -394,11 +395,6 @@ template <typename T> struct Impl {
     st.fkmax2 = h->p.fkmax * h->p.fkmax;
     st.eps = h->p.eps;
     st.kf_partial = h->kf_partial;
-    // tiles of the zinv kernel that writes the K_f partial sums
-    const int pt = use_zinv5(h) ? L::zinv5_tile(h->logz)
-                   : (h->tma && h->tma_zinv && h->p.sgs == SC_SGS_NONE) ? L::tma_ztile(h->logz)
-                                                                        : pencil_tile(h->logz);
-    set_kf_tiles(h, st, pt);
     st.kcut2 = kcut2(h);
     st.mask_rhs = h->p.mask_mode == SC_MASK_RHS_AND_STEP;
     st.symmetrize = 1;
@@ -592,8 +588,9 @@ template <typename T> struct Impl {
       // the fused and five-transform kernels tile them
       CUtensorMap lmap5;
       SC_TRY(encode_fields(h, wl.f[0], 6, 2, P5, g->nz, &lmap5));
+      set_kf_tiles(h, st, z5 ? P5 : (h->tma_zinv ? PZ : pencil_tile(h->logz)));
       if (fuse & FUSE_IN) {
-        // produced by the previous stage
+        // produced by the previous stage, tiled as zinv5
       } else if (z5) {
         sc::ZvArgs<T> zu = za;
         zu.ustore = 1;   // lmap5 tiles the output fields wl[0..5] as zinv5 does
@@ -665,8 +662,10 @@ template <typename T> struct Impl {
         SC_TRY(encode_fields(h, wl.f[0], 3, 2, P5, g->nz, &umap));
         sc::ZvArgs<T> zu = za;
         zu.ustore = 1;
+        set_kf_tiles(h, st, P5);
         SC_TRY(launch(h, "zinv", [&] { return L::zinv5_tma(h->logz, vmap, umap, zu, wl, *g, tw(h, g->nz), h->derr, h->stream, sc::ZV_SMAG); }));
       } else {
+        set_kf_tiles(h, st, pencil_tile(h->logz));
         SC_TRY(launch(h, "zinv", [&] { return L::zinv_vel(h->logz, les ? sc::ZV_SMAG : sc::ZV_DNS, za, wl, *g, tw(h, g->nz), h->stream); }));
       }
       if (h->tma) SC_TRY(plain_tma(h, "ypass_inv", 1, true, wl.f[0], nw));

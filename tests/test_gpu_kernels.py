@@ -255,3 +255,19 @@ def test_wide_rotating_band(specns_lib, fk2, prec):
     assert rel_l2(both[:3], v) < TOL[prec]
     assert rel_l2(both[3], phi) < TOL[prec]
     assert rel_l2(alone, R.rot_run(fd[:3], g, 2, 2.0, 1.0, fk2)[0]) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("shape", [(16, 8, 512), (256, 8, 512), (1024, 8, 512), (16, 16, 1024)])
+def test_les_forcing_tiles(specns_lib, shape, prec):
+    """The forcing coefficient of an LES right-hand side where the z-inverse sums
+    the band in tiles of another width than the register kernel's, band wider
+    than either: with and without the gradient form's row lengths."""
+    nx, ny, nz = shape
+    kw = dict(nu=0.01, dt=1e-3, fkmax=6.2, eps=0.3, c1=0.03)
+    v = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 73, kcut=8.0)]
+    ref = R.ratesdudt([a.astype(np.complex128) for a in v], R.Grid(R.Params(nx=nx, ny=ny, nz=nz, sgs="smag", **kw)))
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, sgs=S.SC_SGS_SMAG, **kw)) as h:
+        h.set_state(*v)
+        w = h.rhs()
+    assert rel_l2(w, ref) < TOL[prec]
