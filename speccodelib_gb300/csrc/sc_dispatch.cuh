@@ -231,7 +231,7 @@ cudaError_t launch_zinv_phi(const CUtensorMap& lmap, const CUtensorMap& omap, co
 template <typename T, int LOGN, int MODE>
 cudaError_t launch_zinv5(const CUtensorMap& vmap, const CUtensorMap& umap, const ZvArgs<T>& za,
                          const FieldList<T>& out, const Geom& g, const C2<T>* tw, int* err, cudaStream_t s) {
-  using Z = ZiCfg<T, LOGN>;
+  using Z = ZiCfg<T, LOGN, MODE>;
   if constexpr (!Z::SUPPORTED) {
     return cudaErrorNotSupported;
   } else {
@@ -239,7 +239,7 @@ cudaError_t launch_zinv5(const CUtensorMap& vmap, const CUtensorMap& umap, const
     static cudaError_t attr = smem_attr(k, Z::SMEM);
     if (attr != cudaSuccess) return attr;
     dim3 grid((g.nxh + Z::P - 1) / Z::P, g.ny);
-      return launch_pdl(k, grid, dim3(Z::NT), Z::SMEM, s, vmap, umap, za, out, g, tw, err);
+    return launch_pdl(k, grid, dim3(Z::NT), Z::SMEM, s, vmap, umap, za, out, g, tw, err);
   }
 }
 

@@ -39,14 +39,16 @@ template <typename T> struct FusedArgs {
   int store_all;      // also store every tile of the next stage input (adjoint)
 };
 
-template <typename T, int LOGN> struct ZiCfg {
+template <typename T, int LOGN, int MODE = ZV_DNS> struct ZiCfg {
   using Cfg = TmaCfg<T, LOGN>;
   // tile width: the strided passes' width (halving it, for more CTAs per SM,
   // measured slower: 32-byte row segments)
   static constexpr int P = Cfg::P;
   static constexpr int N = Cfg::N;
   using ZG = ZgCfg<T, LOGN>;
-  static constexpr bool GROUPED = ZG::ON;   // three groups of threads (ZgCfg), six tiles
+  // three groups of threads (ZgCfg), six tiles; not for ZV_SMAG, whose eight
+  // transforms run in turn (grouped, at 64 points of 1024 x 64 x 64 FP32, 60 -> 128 us)
+  static constexpr bool GROUPED = ZG::ON && MODE != ZV_SMAG;
   // else two jobs per thread, at most 256 threads (ZI_DIV 16, ZI_MAX 256), or
   // one job per thread up to 512 (ZI_DIV 8, ZI_MAX 512)
   static constexpr int NT_RAW = P * N / ZI_DIV;
@@ -113,7 +115,7 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
                                                 long long base, long long zstride, const FieldList<T>& out,
                                                 const Geom& g, const C2<T>* __restrict__ tw,
                                                 const CUtensorMap* umap) {
-  using Z = ZiCfg<T, LOGN>;
+  using Z = ZiCfg<T, LOGN, MODE>;
   using EH = typename Z::EngH;
   using EF = typename Z::EngF;
   using C = C2<T>;
@@ -381,11 +383,11 @@ __device__ __forceinline__ void zinv_from_tiles(C2<T>* const rt[3], C2<T>* work,
 // stage input tile by TMA, K_f partial sums, then zinv_from_tiles.
 // grid = (kx tiles, ny).
 template <typename T, int LOGN, int MODE>
-__global__ void __launch_bounds__(ZiCfg<T, LOGN>::NT, ZiCfg<T, LOGN>::MINB)
+__global__ void __launch_bounds__(ZiCfg<T, LOGN, MODE>::NT, ZiCfg<T, LOGN, MODE>::MINB)
 zinv5_tma_kernel(const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap umap, ZvArgs<T> za,
                  FieldList<T> out, Geom g, const C2<T>* __restrict__ tw, int* err) {
   pdl_wait();
-  using Z = ZiCfg<T, LOGN>;
+  using Z = ZiCfg<T, LOGN, MODE>;
   using Cfg = TmaCfg<T, LOGN>;
   using C = C2<T>;
   constexpr int P = Z::P;
