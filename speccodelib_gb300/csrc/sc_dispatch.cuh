@@ -257,12 +257,17 @@ cudaError_t launch_xwarp(const FieldList<T>& fin, const FieldList<T>& fout, cons
 template <typename T, int LOGM, int MODE>
 cudaError_t launch_xgroup(const FieldList<T>& fin, const FieldList<T>& fout, const Geom& g, const C2<T>* twM,
                           const C2<T>* twN, const XArgs<T>& xa, cudaStream_t s) {
-  using Cfg = XgCfg<T, LOGM, MODE>;
-  auto k = xpass_group_kernel<T, LOGM, MODE>;
-  static cudaError_t attr = smem_attr(k, Cfg::SMEM);
-  if (attr != cudaSuccess) return attr;
-  const int per = Cfg::WARPS * GroupFFT<T, LOGM>::RW;
-  return launch_pdl(k, dim3((unsigned)((xa.rows + per - 1) / per)), dim3(Cfg::NT), Cfg::SMEM, s, fin, fout, g, twM, twN, xa);
+  if constexpr (MODE == XW_GRAD && sizeof(T) == 8 && LOGM > 6) {
+    return cudaErrorNotSupported;   // les_gradient_rows
+  } else {
+    if (xg_few_rows<T, LOGM, MODE>(xa.rows, xa.nsm)) return cudaErrorNotSupported;
+    using Cfg = XgCfg<T, LOGM, MODE>;
+    auto k = xpass_group_kernel<T, LOGM, MODE>;
+    static cudaError_t attr = smem_attr(k, Cfg::SMEM);
+    if (attr != cudaSuccess) return attr;
+    const int per = Cfg::WARPS * GroupFFT<T, LOGM>::RW;
+    return launch_pdl(k, dim3((unsigned)((xa.rows + per - 1) / per)), dim3(Cfg::NT), Cfg::SMEM, s, fin, fout, g, twM, twN, xa);
+  }
 }
 
 template <typename T, int LOGM>
@@ -377,6 +382,9 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
   }
 
 #define SC_DEFINE_XWARP(T, CASES, UCASES)                                                        \
+  template <> bool sc::Launch<T>::les_gradient(int logm, long long rows, int nsm) {              \
+    return sc::les_gradient_rows<T>(logm, rows, nsm);                                            \
+  }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::xpass_umax(int logm, const FieldList<T>& fin, const Geom& g,        \
                                         const C2<T>* twM, const C2<T>* twN, const XArgs<T>& xa,  \

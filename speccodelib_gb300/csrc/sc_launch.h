@@ -161,6 +161,9 @@ template <typename T> struct Launch {
   static cudaError_t xpass_warp(int logm, int mode, const FieldList<T>& fin, const FieldList<T>& fout,
                                 const Geom& g, const C2<T>* twM, const C2<T>* twN, const XArgs<T>& xa,
                                 cudaStream_t s);
+  // whether XW_GRAD, and with it the gradient form of the LES right-hand side
+  // (sc_les.cuh), serves `rows` rows of that length
+  static bool les_gradient(int logm, long long rows, int nsm);
   // c2r of three velocity rows at a time, kept in registers: max |u|^2 over the
   // grid and the count of non-finite points, added to out[0] (the bits of a
   // non-negative double) and out[1]; lengths as xpass_warp

@@ -772,6 +772,7 @@ template <typename T> struct XArgs {
   const double* c1;        // device scalar: Smagorinsky c1 (or dynamic cs2)
   double delta2;           // filter width squared
   long long rows;          // ny*nz
+  int nsm;                 // SMs of the device (which kernel serves few rows)
 };
 
 template <typename T, int LOGM, int MODE> struct XpCfg {

@@ -426,6 +426,7 @@ template <typename T> struct Impl {
     xa.c1 = h->dscal;
     xa.delta2 = h->p.delta * h->p.delta;
     xa.rows = (long long)h->g.ny * h->g.nz;
+    xa.nsm = h->nsm;
     return xa;
   }
 
@@ -635,13 +636,9 @@ template <typename T> struct Impl {
       if (vstore) SC_TRY(encode_fields(h, st.vout[0], 3, 2, P, g->nz, &vmap_out));
       // symmetrize included, its kx = 0 copy exchanged inside the kernel
       return launch(h, "zfwd", [&] { return L::zfwd_tma(h->logz, lmap, vmap_out, vstore ? 1 : 0, st, *g, tw(h, g->nz), h->derr, h->stream); });
-    } else if (les && h->tma && h->zinv5 && h->xwarp && sin_spaced && L::zinv5_supported(h->logz) && h->logx >= 5 &&
-               h->logx <= (sizeof(T) == 4 ? 9 : 7)) {
-      // gradient form (sc_les.cuh): the row lengths that the warp and
-      // lane-group x-passes have, but FP64 rows of 256 and 512 points, whose twelve
-      // kept rows leave two warps per SM (Smagorinsky step, gradient form against
-      // S_ij: 128^3 11.3 / 13.0 ms, 256 x 128 x 128 32.0 / 27.8, 512 x 64 x 64
-      // 16.1 / 13.1)
+    } else if (les && h->tma && h->zinv5 && h->xwarp && sin_spaced && L::zinv5_supported(h->logz) &&
+               L::les_gradient(h->logx - 1, (long long)g->ny * g->nz, h->nsm)) {
+      // gradient form (sc_les.cuh)
       const int P5 = L::zinv5_tile(h->logz), PY = L::tma_tile(h->logy);
       CUtensorMap vmap, umap, ymap, fmap;
       SC_TRY(encode_fields(h, sin[0], 3, 2, P5, g->nz, &vmap));

@@ -439,11 +439,16 @@ template <typename T, int LOGM, int MODE> struct XgCfg {
   static constexpr int TM_COLS = 2 * GF::E * KT <= 64 ? 64 : 128;
   static_assert(2 * GF::E * KT <= TM_COLS, "tensor-memory rows");
   static constexpr int PER_WARP = GF::RW * ((KEPT - KT) * GF::M + GF::BUF);
-  // four warps, fewer where their kept rows pass the 227 KB of a CTA
+  // Warps per CTA: four (fewer where their kept rows pass the 227 KB of a CTA).
+  // FP64 rows of up to 128 points one: the warps need nothing of each other, and
+  // few rows then reach more SMs (four steps, FP64: LES at 64 x 32 x 32 4.30 -> 4.06
+  // ms, DNS at 256 x 32 x 32 4.06 -> 3.80; 128^3 unchanged).  At 256 points it is slower
+  // (512 x 32 x 32 LES 12.8 -> 18.0 ms).
   static constexpr int FIT = (int)(227 * 1024 / (sizeof(C2<T>) * PER_WARP));
-  static constexpr int WARPS = FIT < 4 ? FIT : 4, NT = 32 * WARPS;
+  static constexpr int WMAX = sizeof(T) == 8 && LOGM < 8 ? 1 : 4;
+  static constexpr int WARPS = FIT < WMAX ? FIT : WMAX, NT = 32 * WARPS;
   static constexpr size_t SMEM = sizeof(C2<T>) * (size_t)PER_WARP * WARPS;
-  static constexpr int FITB = (int)(220 * 1024 / SMEM), MAXB = sizeof(T) == 4 ? 4 : 2;
+  static constexpr int FITB = (int)(220 * 1024 / SMEM), MAXB = sizeof(T) == 4 ? 4 : 8 / WARPS;
   static constexpr int MINB = FITB < 1 ? 1 : (FITB > MAXB ? MAXB : FITB);
 };
 
@@ -464,6 +469,34 @@ __device__ __forceinline__ XgRow<T, LOGM, KT> xg_row(C2<T>* warp_smem, int kept,
   R.twM = twM;
   R.twN = twN;
   return R;
+}
+
+// Few rows.  A warp here works on its 32 / L rows for as long with one warp per SM
+// as with a full one (FP64, Lamb product: 57 us at M = 32, 63 at 64, 137 at 128, 171
+// at 256), so FP64 grids of few rows leave most of the chip idle, and the block
+// kernel, a CTA per row, is faster: at 512 rows 39, 45, 48 and 101 us, the S_ij
+// products 61, 70, 136 and 292 (here 138, 151, 329, 411).  At 1024 rows it is 39,
+// 45, 91 and 198 us, and from 2048 on slower; the S_ij products at M = 128 stay
+// faster there to 4096 rows (922 us, here 1019; 8192: 1769, 1707), three warps per
+// SM filling this kernel's rounds badly.  The line: 6 rows per SM, 27 for the latter.
+// FP32 rows (a Lamb product of 64 rows in 5 to 6 us) have no such case; M = 16
+// neither (27 us, block 33).
+template <typename T, int LOGM, int MODE> inline bool xg_few_rows(long long rows, int nsm) {
+  if (sizeof(T) == 4 || LOGM < 5 || MODE == XW_SCALAR) return false;   // XW_SCALAR: no block kernel
+  return rows <= (MODE == XW_SMAG && LOGM == 7 ? 27LL : 6LL) * nsm;
+}
+
+// The gradient form of the LES right-hand side: where XW_GRAD has the row length,
+// except in FP64 where few rows would go to the block kernel (Smagorinsky step at 256
+// rows, M = 32 / 64: 786 / 869 us, with the block kernel's S_ij products 573 / 629;
+// at 1024: 1004 / 1173 and 900 / 1225) and at M = 128 and 256, where twelve kept rows
+// leave two warps per SM (256 x 128 x 128 32.0 ms, with S_ij 27.8; 512 x 64 x 64 16.1
+// and 13.1; 128^3 11.3 and 13.0).
+template <typename T> inline bool les_gradient_rows(int logm, long long rows, int nsm) {
+  if (logm < 4 || logm > (sizeof(T) == 4 ? 8 : 6)) return false;
+  return logm == 5   ? !xg_few_rows<T, 5, XW_GRAD>(rows, nsm)
+         : logm == 6 ? !xg_few_rows<T, 6, XW_GRAD>(rows, nsm)
+                     : true;
 }
 
 // Modes, operands and aliasing as xpass_warp_kernel (sc_xwarp.cuh); XW_SMAG

@@ -271,3 +271,37 @@ def test_les_forcing_tiles(specns_lib, shape, prec):
         h.set_state(*v)
         w = h.rhs()
     assert rel_l2(w, ref) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", [S.SC_FP64, S.SC_FP32])
+@pytest.mark.parametrize("sgs", ["none", "smag"])
+@pytest.mark.parametrize("shape", [(64, 16, 32), (64, 32, 64), (128, 16, 32), (128, 32, 64), (256, 16, 32), (256, 32, 64),
+                                   (256, 64, 128), (512, 16, 32), (512, 32, 64)])
+def test_x_row_counts(specns_lib, shape, sgs, prec):
+    """The x-pass on either side of the row counts at which FP64 rows change
+    from the block kernel to lane groups, and the LES from S_ij to gradients."""
+    nx, ny, nz = shape
+    kw = dict(nu=0.01, dt=1e-3, fkmax=3.1, eps=0.3)
+    les = {} if sgs == "none" else dict(sgs=S.SC_SGS_SMAG, c1=0.03)
+    v = [fresh(0.05 * a, DT[prec]) for a in hermitian_fields(shape, 79, kcut=8.0)]
+    g = R.Grid(R.Params(nx=nx, ny=ny, nz=nz, sgs=sgs, c1=0.03, **kw))
+    ref = R.ratesdudt([a.astype(np.complex128) for a in v], g)
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz, **kw, **les)) as h:
+        h.set_state(*v)
+        w = h.rhs()
+    assert rel_l2(w, ref) < TOL[prec]
+
+
+@pytest.mark.parametrize("shape", [(64, 16, 32), (64, 32, 64), (128, 32, 64), (256, 16, 32), (256, 32, 64), (512, 16, 32),
+                                   (512, 32, 64)])
+def test_vjp_row_counts(specns_lib, shape):
+    """The adjoint's x-pass in FP64 on either side of its row count."""
+    nx, ny, nz = shape
+    v = [fresh(0.05 * a, np.complex128) for a in hermitian_fields(shape, 83, kcut=6.0)]
+    lam = [fresh(a, np.complex128) for a in hermitian_fields(shape, 84)]
+    kw = dict(nu=0.02, dt=1e-3)
+    ref = R.rk4_step_adj(v, lam, R.Grid(R.Params(nx=nx, ny=ny, nz=nz, **kw)))
+    with S.SpectralNS(S.default_params(nx, S.SC_FP64, ny=ny, nz=nz, **kw)) as h:
+        h.set_state(*v)
+        out = h.adjoint_vjp(1, lam, 1)
+    assert rel_l2(out, ref) < 1e-11   # the bound of the adjoint's other tests
