@@ -140,7 +140,8 @@ ens_yinv_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
   }
 }
 
-// End of a stage (see the head of this file).  grid = (kx tiles, members).
+// End of a stage (see the head of this file).  A block per kx tile and member, in
+// one dimension: a class may have more members than the other two admit.
 template <typename T, int LOGN>
 __global__ void __launch_bounds__(EnsSplitCfg<T, LOGN>::NT, EnsSplitCfg<T, LOGN>::MINB)
 ens_yfwd_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
@@ -154,7 +155,8 @@ ens_yfwd_kernel(const __grid_constant__ CUtensorMap map, EnsClass<T> ec) {
   C* const t0 = reinterpret_cast<C*>(smraw);
   C* const t1 = reinterpret_cast<C*>(smraw + Cfg::TILE);
   __shared__ __align__(8) uint64_t bars[2];
-  const int kx0 = blockIdx.x * P, m = ec.m0 + blockIdx.y;
+  const int ntx = (ec.nxh + P - 1) / P;
+  const int kx0 = blockIdx.x % ntx * P, m = ec.m0 + blockIdx.x / ntx;
   const int nvalid = min(P, ec.nxh - kx0);
   const C* __restrict__ tw = ec.tw + N;
   if (launch_failed(ec.err)) return;
@@ -333,7 +335,7 @@ template <typename T, int LOGN> cudaError_t ens_split_stage_n(const CUtensorMap&
         launch_pdl(ens_xgroup_kernel<T, LOGN - 1>, dim3((unsigned)((rows + per - 1) / per)), dim3(X::NT), X::SMEM, s, ec);
     if (e != cudaSuccess) return e;
   }
-  return launch_pdl(ens_yfwd_kernel<T, LOGN>, dim3(ntx, ec.count), dim3(Cfg::NT), Cfg::SMEM_FWD, s, map, ec);
+  return launch_pdl(ens_yfwd_kernel<T, LOGN>, dim3(ntx * ec.count), dim3(Cfg::NT), Cfg::SMEM_FWD, s, map, ec);
 }
 
 // sc_ens_split_*.cu

@@ -110,3 +110,49 @@ def test_ensemble_energy_decays_without_forcing(specns_lib):
         e1 = [R.energy2d(e.get_member(m)) for m in range(2)]
     assert all(abs(a - 0.5) < 1e-12 for a in e0)
     assert all(b < a for a, b in zip(e0, e1))
+
+
+def test_many_members_of_one_size(specns_lib):
+    """More members of one size than a grid's second dimension admits, in the
+    launch-per-pass form: members at both ends equal to an ensemble of their own."""
+    nm, n, var = 65540, 64, 5
+    dt, nu = params(n)
+    seeds = [-3, -5, -9]
+    at = [0, 65535, nm - 1]
+    with S.Ensemble2D([n] * 3, [dt] * 3, [nu] * 3, 0.01, S.SC_FP32) as e:
+        e.set_variant(var)
+        e.init(seeds)
+        init = [e.get_member(m) for m in range(3)]
+        e.rk4_steps(2)
+        ref = [e.get_member(m) for m in range(3)]
+    with S.Ensemble2D([n] * nm, [dt] * nm, [nu] * nm, 0.01, S.SC_FP32) as e:
+        e.set_variant(var)
+        for m, w in zip(at, init):
+            e.set_member(m, w)
+        e.rk4_steps(2, 1)
+        for m, w in zip(at, ref):
+            assert np.array_equal(e.get_member(m), w)
+        assert not np.any(e.get_member(1)) and not np.any(e.get_member(nm - 2))
+
+
+@pytest.mark.parametrize("prec,var,sizes", [(S.SC_FP32, 5, [64] * 128), (S.SC_FP32, 5, [1024] * 6),
+                                            (S.SC_FP64, 1, [128] * 40), (S.SC_FP64, 1, [1024] * 4)])
+def test_classes_of_many_tiles(specns_lib, prec, var, sizes):
+    """Classes whose first pass takes each CTA through several tiles (its two
+    buffers refilled, their barriers' phases turned): every member as when it
+    runs alone, the first and the last as the oracle's."""
+    n, nm = sizes[0], len(sizes)
+    dt, nu = params(n)
+    seeds = [-(m + 1) for m in range(nm)]
+    outs = []
+    for mode in (1, 2):
+        with S.Ensemble2D(sizes, [dt] * nm, [nu] * nm, 0.01, prec) as e:
+            e.set_variant(var)
+            e.init(seeds)
+            e.rk4_steps(1, mode)
+            outs.append([e.get_member(m) for m in range(nm)])
+    for a, b in zip(*outs):
+        assert np.array_equal(a, b)
+    for m in (0, nm - 1):
+        ref = oracle_steps(n, R.initialize2d(n, seeds[m]), dt, nu, 1)
+        assert rel_l2(outs[0][m], ref) < (1e-12 if prec == S.SC_FP64 else 1e-5)
