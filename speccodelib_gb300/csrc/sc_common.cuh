@@ -96,7 +96,7 @@ struct K2Lt {   // k2 < t  <=>  k2 < b
 // Largest k <= kmax with k^2 < b (0 for b <= 1): the reach of a band along an
 // axis whose wavenumbers end at kmax.  The bound keeps the squares below 2^31
 // where b is clamped there (k2_clamp), so that the search ends.
-__host__ __device__ inline int band_reach(int b, int kmax) {
+inline int band_reach(int b, int kmax) {
   int k = 0;
   while (k < kmax && (k + 1) * (k + 1) < b) ++k;
   return k;

@@ -601,7 +601,7 @@ cudaError_t launch_zfwd_adj_tma(const CUtensorMap& pmap, const int fidx[6], cons
   }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::band_coef(const BandArgs<T>& ba, const Geom& g, cudaStream_t s) {   \
-    return sc::launch_pdl(sc::band_coef_kernel<T>, dim3(1), dim3(256), 0, s, ba, g);        \
+    return sc::band_launch<T>(ba, g, s);                                                         \
   }                                                                                              \
   template <>                                                                                    \
   cudaError_t sc::Launch<T>::ab2v(const Ab2vArgs<T>& aa, const Geom& g, cudaStream_t s) {        \

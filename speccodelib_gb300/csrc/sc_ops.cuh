@@ -370,10 +370,12 @@ __global__ void __launch_bounds__(256) specop_kernel(SpecOpArgs<T> oa, Geom g) {
 // ---------------------------------------------------------------------------
 // force_rot.f90's coefficient on the device: a = eps / (2 kinet + tiny), kinet
 // the 1/2-weighted (kx = 0) energy of v on lo2 <= k2 < hi2 (force_rot.f90:
-// 16-27); with nf = 1 and tiny = 0 forcephi_rot.f90's, of one field.  One block walks the band's bounding box |k_i| <= floor(sqrt(hi2))
-// in a fixed order and sums in FP64, so the result is deterministic and no
-// host synchronisation is needed (the rotating pass reads *out in its
-// z-forward epilogue).
+// 16-27); with nf = 1 and tiny = 0 forcephi_rot.f90's, of one field.  The band's
+// bounding box |k_i| <= floor(sqrt(hi2)) is walked in a fixed order and summed in
+// FP64, so the result is deterministic and no host synchronisation is needed (the
+// rotating pass reads *out in its z-forward epilogue).  A block takes up to 2048
+// modes of the box alone; wider bands 1024 modes per block and a second launch over
+// their sums: one block over fk2 = 40 at 256^3 took 1.2 ms of a pass, fk2 = 85 12 ms.
 // ---------------------------------------------------------------------------
 template <typename T> struct BandArgs {
   const C2<T>* v[3];
@@ -381,37 +383,68 @@ template <typename T> struct BandArgs {
   K2Lt lo2, hi2;
   double eps, tiny;
   double* out;
+  double* partial;        // kBandBlocks values
+};
+constexpr int kBandBlocks = 1024;
+
+struct BandBox {   // formed on the host
+  int nkx, ky0, nky, kz0, nkz;
+  long long total;
+  BandBox(int hi_b, const Geom& g) {
+    const int hy = g.ny / 2, hz = g.nz / 2;
+    const int kx = band_reach(hi_b, g.nxh - 1), ky = band_reach(hi_b, hy), kz = band_reach(hi_b, hz);
+    nkx = kx + 1;
+    ky0 = -ky;
+    nky = (ky < hy ? ky : hy - 1) - ky0 + 1;
+    kz0 = -kz;
+    nkz = (kz < hz ? kz : hz - 1) - kz0 + 1;
+    total = (long long)nkx * nky * nkz;
+  }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256) band_coef_kernel(BandArgs<T> ba, Geom g) {
+template <typename T, int NF>
+__global__ void __launch_bounds__(256) band_sum_kernel(BandArgs<T> ba, BandBox b, Geom g) {
   pdl_wait();
   __shared__ double red[256 / 32 + 1];
   const int lo_b = ba.lo2.b, hi_b = ba.hi2.b;
-  const int kb = band_reach(hi_b, max(g.nxh - 1, max(g.ny, g.nz) / 2));
-  const int nkx = min(kb, g.nxh - 1) + 1;
-  const int ky0 = max(-kb, -g.ny / 2), ky1 = min(kb, g.ny / 2 - 1);
-  const int kz0 = max(-kb, -g.nz / 2), kz1 = min(kb, g.nz / 2 - 1);
-  const int nky = ky1 - ky0 + 1, nkz = kz1 - kz0 + 1;
-  const long long total = (long long)nkx * nky * nkz;
   double q = 0.0;
-  for (long long t = threadIdx.x; t < total; t += blockDim.x) {
-    const int ix = (int)(t % nkx);
-    const int ky = ky0 + (int)((t / nkx) % nky);
-    const int kz = kz0 + (int)(t / ((long long)nkx * nky));
+  for (long long t = blockIdx.x * 256LL + threadIdx.x; t < b.total; t += gridDim.x * 256LL) {
+    const int ix = (int)(t % b.nkx);
+    const int ky = b.ky0 + (int)((t / b.nkx) % b.nky);
+    const int kz = b.kz0 + (int)(t / ((long long)b.nkx * b.nky));
     const int k2 = ix * ix + ky * ky + kz * kz;
     if (k2 < lo_b || k2 >= hi_b) continue;
     const int iy = ky < 0 ? ky + g.ny : ky, iz = kz < 0 ? kz + g.nz : kz;
     const long long idx = ((long long)iz * g.ny + iy) * g.nxp + ix;
     double e = 0.0;
-    for (int c = 0; c < ba.nf; ++c) {
+#pragma unroll
+    for (int c = 0; c < NF; ++c) {
       const C2<T> a = ba.v[c][idx];
       e += (double)a.x * a.x + (double)a.y * a.y;
     }
     q += ix == 0 ? 0.5 * e : e;
   }
+  const double sum = block_sum<256>(q, red);
+  if (threadIdx.x != 0) return;
+  if (gridDim.x == 1) *ba.out = ba.eps / (2.0 * sum + ba.tiny);
+  else ba.partial[blockIdx.x] = sum;
+}
+template <typename T> __global__ void __launch_bounds__(256) band_coef_kernel(BandArgs<T> ba, int nblocks) {
+  pdl_wait();
+  __shared__ double red[256 / 32 + 1];
+  double q = 0.0;
+  for (int b = threadIdx.x; b < nblocks; b += 256) q += ba.partial[b];
   const double kinet = block_sum<256>(q, red);
   if (threadIdx.x == 0) *ba.out = ba.eps / (2.0 * kinet + ba.tiny);
+}
+template <typename T> inline cudaError_t band_launch(const BandArgs<T>& ba, const Geom& g, cudaStream_t s) {
+  const BandBox box(ba.hi2.b, g);
+  const long long want = box.total <= 2048 ? 1 : (box.total + 1023) / 1024;
+  const int nb = (int)(want < kBandBlocks ? want : kBandBlocks);
+  const cudaError_t e =
+      launch_pdl(ba.nf == 1 ? band_sum_kernel<T, 1> : band_sum_kernel<T, 3>, dim3(nb), dim3(256), 0, s, ba, box, g);
+  if (e != cudaSuccess || nb == 1) return e;
+  return launch_pdl(band_coef_kernel<T>, dim3(1), dim3(256), 0, s, ba, nb);
 }
 
 // ---------------------------------------------------------------------------

@@ -1024,6 +1024,7 @@ template <typename T> struct Impl {
         ba.eps = h->p.eps;
         ba.tiny = sizeof(T) == 4 ? 1.1754943508222875e-38 : 2.2250738585072014e-308;
         ba.out = h->dscal + 4;
+        ba.partial = h->dpart;
         SC_TRY(launch(h, "band_coef", [&] { return L::band_coef(ba, *g, h->stream); }));
         st.fcoef = h->dscal + 4;
         st.fband_lo2 = fk1 * fk1;
@@ -1052,6 +1053,7 @@ template <typename T> struct Impl {
         ba.eps = h->p.eps;
         ba.tiny = sizeof(T) == 4 ? 1.1754943508222875e-38 : 2.2250738585072014e-308;
         ba.out = h->dscal + 4;
+        ba.partial = h->dpart;
         SC_TRY(launch(h, "band_coef", [&] { return L::band_coef(ba, *g, h->stream); }));
         st.fcoef = h->dscal + 4;
         st.fband_lo2 = fk1;
@@ -1070,6 +1072,7 @@ template <typename T> struct Impl {
         ba.hi2 = fk2 * fk2;
         ba.eps = sc->epsphi;
         ba.out = h->dscal + 5;
+        ba.partial = h->dpart;
         SC_TRY(launch(h, "band_coef", [&] { return L::band_coef(ba, *g, h->stream); }));
         sr.da.phi = AX(h, RA_PHI);
         sr.da.fcoef = h->dscal + 5;
