@@ -1743,9 +1743,17 @@ int copy_in(sc_handle* h, void* const* dst, const void* const* src, int n) {
 }
 int copy_in(sc_handle* h, void* dst, const void* src) { return copy_in(h, &dst, &src, 1); }
 
-// n padded device fields -> user memory
+// n padded device fields -> user memory.  Buffers that overlap (one buffer given
+// for all components, say) are written in turn, the last one last.
 int copy_out(sc_handle* h, void* const* dst, const void* const* src, int n) {
   const size_t w = h->csize * h->g.nxh, rows = (size_t)h->g.ny * h->g.nz;
+  for (int i = 0; i < n && n > 1; ++i)
+    for (int j = 0; j < i; ++j) {
+      const uintptr_t a = reinterpret_cast<uintptr_t>(dst[i]), b = reinterpret_cast<uintptr_t>(dst[j]);
+      if ((a > b ? a - b : b - a) >= w * rows) continue;
+      for (int k = 0; k < n; ++k) SC_TRY(copy_out(h, dst + k, src + k, 1));
+      return SC_OK;
+    }
   void* kd[kRepackMax];
   const void* ks[kRepackMax];
   int nk = 0;

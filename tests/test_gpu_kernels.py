@@ -305,3 +305,28 @@ def test_vjp_row_counts(specns_lib, shape):
         h.set_state(*v)
         out = h.adjoint_vjp(1, lam, 1)
     assert rel_l2(out, ref) < 1e-11   # the bound of the adjoint's other tests
+
+
+@pytest.mark.parametrize("where", ["device", "pinned"])
+@pytest.mark.parametrize("lap", [0, 1])
+def test_overlapping_state_buffers(specns_lib, where, lap):
+    """A state read into buffers that overlap holds what copies in turn leave:
+    one buffer for all three components (lap 0), or neighbours half over each
+    other, from the last to the first in memory (lap 1)."""
+    torch = pytest.importorskip("torch")
+    nx, ny, nz = 128, 64, 64
+    n = nz * ny * (nx // 2 + 1)
+    rng = np.random.default_rng(4)
+    v = [(rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64) for _ in range(3)]
+    at = [0, 0, 0] if lap == 0 else [n, n // 2, 0]
+    buf = torch.zeros(2 * n, dtype=torch.complex64, device="cuda") if where == "device" else \
+        torch.zeros(2 * n, dtype=torch.complex64).pin_memory()
+    torch.cuda.synchronize()
+    with S.SpectralNS(S.default_params(nx, S.SC_FP32, ny=ny, nz=nz)) as h:
+        h.set_state(*[a.reshape(nz, ny, nx // 2 + 1) for a in v])
+        for _ in range(5):
+            h.get_state_device(*(buf.data_ptr() + 8 * o for o in at))
+            ref = np.zeros(2 * n, np.complex64)
+            for o, a in zip(at, v):
+                ref[o:o + n] = a
+            assert np.array_equal(buf.cpu().numpy(), ref)
