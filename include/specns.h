@@ -307,8 +307,9 @@ int sc_ens_uses_graph(sc_ensemble* e);
  * bit-reproducible runs.  sc_ens_variant reports the current variant, the
  * number of variants, the last tuning's ms per step per variant
  * (tune_ms[count], -1 = not timed) and the shape {threads, CTAs per SM,
- * tile points, radix, phases out of line} (shape[5]); any pointer may be
- * NULL.
+ * tile points, radix, phases out of line} (shape[5]; of the variant with a
+ * launch per pass, whose shape follows N, that of its FP32 y passes at N = 256
+ * and 512); any pointer may be NULL.
  * No reference counterpart. */
 int sc_ens_tune(sc_ensemble* e, int trial_steps, int* chosen);
 int sc_ens_set_variant(sc_ensemble* e, int variant);

@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) ens_stage_kernel(EnsArgs<T> 
 struct EnsVariant {
   const void* kernel;   // ens_stage_kernel<T, Shape> (split: none)
   int nt, minb, ypts, rmax, outline, smem_elems;
-  bool split = false;   // a launch per pass
+  bool split = false;   // a launch per pass (the shape reported: its FP32 y passes at N = 256 and 512)
 };
 constexpr EnsVariant kEnsSplit{nullptr, 512, 2, 4096, 8, 0, 0, true};
 

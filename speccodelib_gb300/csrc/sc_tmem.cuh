@@ -10,9 +10,9 @@
 // transforms first there (sc_xwarp.cuh).
 //
 // The allocation does not poll: it completes when the columns are free.
-// The kernels that allocate hold at most 512 columns per SM between them: 128 per
-// CTA at two or three CTAs, 256 at two, or 64 in the lane-group x-pass; a CTA waits
-// for columns only of CTAs that finish without it.
+// A kernel's CTAs hold at most 512 columns of an SM between them: 128 per CTA at two
+// or three CTAs, 256 at two, or in the lane-group x-pass 64 (128 for the LES gradient
+// rows) at four; a CTA waits for columns only of CTAs that finish without it.
 #pragma once
 #include <stdint.h>
 

@@ -330,3 +330,21 @@ def test_overlapping_state_buffers(specns_lib, where, lap):
             for o, a in zip(at, v):
                 ref[o:o + n] = a
             assert np.array_equal(buf.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("prec,amp", [(S.SC_FP32, 1e18), (S.SC_FP64, 1e153)])
+@pytest.mark.parametrize("nx", [16, 32, 64, 128, 256, 512, 1024])
+def test_diagnostics_nonfinite_in_space(specns_lib, nx, prec, amp):
+    """A field whose modes all have finite squares but whose velocity, all modes
+    in phase at the origin, has not: only the count behind max |u| sees it."""
+    ny = nz = 16
+    v = [np.zeros((nz, ny, nx // 2 + 1), DT[prec]) for _ in range(3)]
+    with S.SpectralNS(S.default_params(nx, prec, ny=ny, nz=nz)) as h:
+        v[0][:4, :4, 1:5] = amp / 64           # 64 modes, |u| = 2 amp
+        h.set_state(*v)
+        assert h.diagnostics()[0]["nonfinite"] == 0
+        v[0][:4, :4, 1:5] = amp                # |u| = 128 amp, its square beyond the type
+        h.set_state(*v)
+        with pytest.raises(S.SpecNSError) as e:
+            h.diagnostics()
+    assert e.value.code == 3
