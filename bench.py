@@ -340,7 +340,9 @@ def run_ours(a):
                 "frac": achieved / hbm, "peak_source": peak_kind,
                 "traffic": traffic_from_profiles(dom),
                 "algorithmic_bytes_per_launch": alg, "avg_launch_ms": avg_ms}
-    step_bytes = h.step_bytes()
+    # what the step's passes read and write, by their launches
+    step_fields = sum(prof[k][0] * KERNEL_FIELDS[k] for k in prof) / a.steps
+    step_bytes = step_fields * F
     tot_all = max(sum(x[1] for x in prof.values()), 1e-9)
     kernels = {k: {"launches": c, "ms_total": t, "avg_ms": t / max(c, 1), "share": t / tot_all,
                    "achieved_gbs": (KERNEL_FIELDS[k] * F / (t / c / 1e3) / 1e9)
@@ -404,10 +406,10 @@ def run_ours(a):
                             "frac": ach64 / peak64,
                             "peak_source": "measured: sc_fp64_peak_probe (FP64 FMA loop, 8 chains per thread)",
                             "flop_model": "4 RHS x 9 real 3D FFTs x 2.5 N^3 log2 N^3 per step (%.3g flop)" % flops}
-        b64 = 4 * 51 * 2.0 * F
+        b64 = step_fields * 2.0 * F
         fp64["hbm_roofline"] = {"bound": "hbm", "achieved": b64 / (ms64 / k64 / 1e3) / 1e9, "peak": hbm,
                                 "unit": "GB/s", "frac": b64 / (ms64 / k64 / 1e3) / 1e9 / hbm,
-                                "bytes_model": "4 x 51 F per step, F = %.3g B (FP64)" % (2.0 * F)}
+                                "bytes_model": "%g F per step, F = %.3g B (FP64)" % (step_fields, 2.0 * F)}
         # shells holding energy above the FP32 round-off floor of the total
         m = e64 > 1e-10 * float(np.sum(e64))
         fp64["fp32_vs_fp64_after_2_steps"] = {
@@ -500,15 +502,16 @@ def run_ours(a):
             del hl
             les[name] = {"steps_per_s": kl / (ms_l / 1e3), "ms_per_step": ms_l / kl,
                          "energy_after": d_l["energy"], "cs2": d_l["cs2"]}
-            # field-pass model: P = 3 + 4 n_i + 4 n_f + 12 with 12 inverse and 9 forward
-            # transforms (P = 99); the dynamic procedure adds 42 transforms (168 F) on one
-            # step in ten
+            # fields read and written by the passes of the gradient form: z-inverse 9,
+            # y-inverse 15, x-pass 17, y-forward 14, and z-forward with the stage's
+            # update 15, 18, 18, 12; the dynamic procedure adds 42 transforms (168 F) on
+            # one step in ten
             Fl = 129 * 256 * 256 * 8.0
-            bl = 4 * 99 * Fl + (168 * Fl / 10 if sgs == S.SC_SGS_DYNSMAG else 0.0)
+            bl = 283 * Fl + (168 * Fl / 10 if sgs == S.SC_SGS_DYNSMAG else 0.0)
             gbs = bl / (ms_l / kl / 1e3) / 1e9
             les[name]["roofline"] = {"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s",
                                      "frac": gbs / hbm, "bytes_per_step": bl,
-                                     "bytes_model": "4 x 99 F per step%s, F = %.3g B" %
+                                     "bytes_model": "283 F per step%s, F = %.3g B" %
                                      (" + 168 F / 10" if sgs == S.SC_SGS_DYNSMAG else "", Fl)}
         torch.cuda.empty_cache()
 
@@ -549,15 +552,18 @@ def run_ours(a):
                     "ensemble_steps_per_s": ke / t_b,
                     "one_at_a_time_steps_per_s": k1 / t_1,
                     "speedup_vs_one_at_a_time": (ke / t_b) / (k1 / t_1)}
-        # field-pass model of the 2D step: per RHS P = 1 + 2 n_i + 2 n_f + 4 with the
-        # inverse transforms of u, v, w (n_i = 3) and the forward ones of (u w, v w) (n_f = 2)
+        # fields read and written per step: with a launch per pass (the last variant) the
+        # first y-inverse 4, the x-passes 4 x 5, the passes that end a stage 7, 8, 8, 4;
+        # in the cooperative form 15 a stage (inverse transforms of u, v, w, forward ones
+        # of u w and v w, 5 of state)
         F2 = sum((m // 2 + 1) * m * 8.0 for m in sizes)
-        b2 = 4 * 15 * F2
+        f2 = 51 if var == len(tune_ms) - 1 else 60
+        b2 = f2 * F2
         gb2 = b2 * ke / t_b / 1e9
         ensemble["roofline"] = {"bound": "hbm", "achieved": gb2, "peak": hbm, "unit": "GB/s",
                                 "frac": gb2 / hbm, "bytes_per_step": b2,
-                                "bytes_model": "4 x 15 F per step summed over the members, sum F = %.3g B "
-                                               "(the whole ensemble's fields fit in the 129 MB L2)" % F2}
+                                "bytes_model": "%d F per step summed over the members, sum F = %.3g B "
+                                               "(one field of every member; the 129 MB L2 holds that)" % (f2, F2)}
         ens.close()
         del ens
 

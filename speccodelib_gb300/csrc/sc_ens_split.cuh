@@ -16,7 +16,7 @@
 //             stage; then the next stage's u, v, w from the new stage input
 //             still in the tile, which never goes to memory
 //
-// 52 field passes per step instead of 60.  Classes are independent within a
+// 51 field passes per step instead of 60.  Classes are independent within a
 // step and run on streams of their own (branches of the captured graph), so
 // that one fills the tail of another.  Values do not depend on what is
 // batched together.

@@ -9,11 +9,11 @@
 // taken axis by axis the same way: the x-pass returns L_i - i kx tau_i1 and
 // the five stresses still needed (8 fields), the y-forward leaves
 // L_i - i kx tau_i1 - i ky tau_i2 and tau_i3 (6), which the z-forward
-// combines.  70 field passes per right-hand side instead of 96, and 29
+// combines.  71 field passes per right-hand side instead of 97, and 29
 // strided-axis transforms instead of 38: the Smagorinsky step at 256^3 FP32
-// 7.01 -> 5.22 ms, at 128^3 (dynamic) 1.51 -> 1.09 ms.  The form needs a row
-// length that the warp or lane-group x-pass has (nx = 32 .. 512); others keep
-// the twelve fields.
+// 7.01 -> 5.22 ms, at 128^3 (dynamic) 1.51 -> 1.09 ms, at 128^3 FP64 17.7 -> 11.3 ms.
+// The rows that it serves: les_gradient_rows (sc_xgroup.cuh); others keep the
+// twelve fields.
 #pragma once
 #include "sc_tma_passes.cuh"
 
