@@ -27,8 +27,10 @@ int efail(int code, const char* msg) { return sc::set_last_error(code, msg); }
 #define EC(call)                                                             \
   do {                                                                       \
     cudaError_t e_ = (call);                                                 \
-    if (e_ != cudaSuccess) return efail(e_ == cudaErrorMemoryAllocation ? SC_ERR_NOMEM : SC_ERR_CUDA, \
-                                        cudaGetErrorString(e_));             \
+    if (e_ != cudaSuccess) {                                                 \
+      cudaGetLastError();   /* or a later launch check would find it again */ \
+      return efail(e_ == cudaErrorMemoryAllocation ? SC_ERR_NOMEM : SC_ERR_CUDA, cudaGetErrorString(e_)); \
+    }                                                                        \
   } while (0)
 
 bool pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }

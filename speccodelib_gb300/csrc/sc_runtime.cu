@@ -45,12 +45,16 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
+// An error that is reported is also taken from the thread's last error, where a
+// later launch check would find it again.
 #define SC_CUDA(call)                                                                    \
   do {                                                                                   \
     cudaError_t e_ = (call);                                                             \
-    if (e_ != cudaSuccess)                                                               \
+    if (e_ != cudaSuccess) {                                                             \
+      cudaGetLastError();                                                                \
       return fail(e_ == cudaErrorMemoryAllocation ? SC_ERR_NOMEM : SC_ERR_CUDA,          \
                   "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                    \
   } while (0)
 
 #define SC_TRY(call)              \
@@ -158,7 +162,10 @@ template <class F> int launch(sc_handle* h, const char* name, F&& f) {
     cudaEventRecord(b, h->stream);
     h->pending.push_back({name, a, b});
   }
-  if (e != cudaSuccess) return fail(SC_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(SC_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
+  }
   return SC_OK;
 }
 

@@ -348,3 +348,18 @@ def test_diagnostics_nonfinite_in_space(specns_lib, nx, prec, amp):
         with pytest.raises(S.SpecNSError) as e:
             h.diagnostics()
     assert e.value.code == 3
+
+
+def test_calls_after_a_failed_allocation(specns_lib):
+    """An error that one call has reported is not reported again by the next."""
+    torch = pytest.importorskip("torch")
+    n = 32
+    v = [torch.zeros((n, n, n // 2 + 1), dtype=torch.complex64, device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    nm = 20000   # a terabyte of members
+    with S.SpectralNS(S.default_params(n, S.SC_FP32)) as h:
+        for use in (lambda: h.set_state_device(*(a.data_ptr() for a in v)), lambda: h.rk4_steps(1), h.get_state):
+            with pytest.raises(S.SpecNSError) as e:
+                S.Ensemble2D([1024] * nm, [1e-4] * nm, [0.0] * nm, 0.0, S.SC_FP64)
+            assert e.value.code == 5
+            use()
