@@ -2,7 +2,10 @@
 // include/specns.h): member storage, the seeded initial vorticity, the launches of
 // a stage (one cooperative, or one per pass), and the CUDA graph of a whole step.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
@@ -57,7 +60,6 @@ struct sc_ensemble {
   double alpha = 0;
   cudaStream_t own = nullptr, stream = nullptr;
   void* mem = nullptr;          // all member fields
-  void* stage = nullptr;        // one member in the reference layout: host copies go through it
   void* dmem_members = nullptr; // EnsMember<T>[nm] (batched) then [nm] (one at a time)
   void* tw = nullptr;
   unsigned* bar = nullptr;
@@ -447,7 +449,6 @@ int sc_ens_destroy(sc_ensemble* e) {
   if (e->stream) cudaStreamSynchronize(e->stream);
   if (e->graph) cudaGraphExecDestroy(e->graph);
   cudaFree(e->mem);
-  cudaFree(e->stage);
   cudaFree(e->dmem_members);
   cudaFree(e->tw);
   cudaFree(e->bar);
@@ -473,34 +474,37 @@ int sc_ens_set_stream(sc_ensemble* e, void* stream) {
   return SC_OK;
 }
 
-// A member's rows of N/2+1 to or from user memory.  Host memory moves as one
-// contiguous copy through a device buffer: the row-by-row copies of a strided
-// transfer to pageable memory ran at 2.2 GB/s.
+// Pageable memory that a copy from the device is about to fill: the pages that are
+// not there yet (a fresh allocation) are touched here, since each one that the copy
+// meets first costs a fault over the link.  Eleven members of 4.2 MB into fresh heap
+// memory: 33 to 50 ms, with a contiguous copy through a device buffer 3.6 to 50,
+// touched first 17 (by eight threads 22: the faults serialise); into present pages
+// 1.7 (1.9 through the buffer).
+static void fault_in(void* p, size_t bytes) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) cudaGetLastError();
+  if (a.type != cudaMemoryTypeUnregistered || bytes == 0) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), first = reinterpret_cast<uintptr_t>(p), end = first + bytes;
+  unsigned char there[1024];
+  for (uintptr_t at = first / page * page; at < end; at += sizeof there * page) {
+    const uintptr_t n = std::min<uintptr_t>((end - at + page - 1) / page, sizeof there);
+    if (mincore(reinterpret_cast<void*>(at), n * page, there) != 0) return;   // not all mapped: the copy reports it
+    for (uintptr_t i = 0; i < n; ++i) {
+      if (there[i] & 1) continue;
+      volatile char* c = reinterpret_cast<volatile char*>(std::max(first, at + i * page));
+      *c = *c;
+    }
+  }
+}
+
+// A member's rows of N/2+1 to or from user memory, as one strided copy.
 static int copy_member(sc_ensemble* e, int m, void* user, bool in) {
   const size_t row = e->csize * (e->n[m] / 2 + 1), rows = e->n[m], pitch = e->csize * e->nxp[m];
   char* dev = static_cast<char*>(e->mem) + e->csize * e->field_off[m];
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, user) != cudaSuccess) cudaGetLastError();
-  const bool host = a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeUnregistered;
-  if (host && !e->stage) {
-    size_t most = 0;
-    for (int k = 0; k < e->nm; ++k) most = std::max(most, e->csize * (e->n[k] / 2 + 1) * (size_t)e->n[k]);
-    if (cudaMalloc(&e->stage, most) != cudaSuccess) {
-      cudaGetLastError();
-      e->stage = nullptr;
-    }
-  }
-  if (host && e->stage) {
-    if (in) {
-      EC(cudaMemcpyAsync(e->stage, user, row * rows, cudaMemcpyHostToDevice, e->stream));
-      EC(cudaMemcpy2DAsync(dev, pitch, e->stage, row, row, rows, cudaMemcpyDeviceToDevice, e->stream));
-    } else {
-      EC(cudaMemcpy2DAsync(e->stage, row, dev, pitch, row, rows, cudaMemcpyDeviceToDevice, e->stream));
-      EC(cudaMemcpyAsync(user, e->stage, row * rows, cudaMemcpyDeviceToHost, e->stream));
-    }
-  } else if (in) {
+  if (in) {
     EC(cudaMemcpy2DAsync(dev, pitch, user, row, row, rows, cudaMemcpyDefault, e->stream));
   } else {
+    fault_in(user, row * rows);
     EC(cudaMemcpy2DAsync(user, row, dev, pitch, row, rows, cudaMemcpyDefault, e->stream));
   }
   EC(cudaStreamSynchronize(e->stream));

@@ -156,3 +156,30 @@ def test_classes_of_many_tiles(specns_lib, prec, var, sizes):
     for m in (0, nm - 1):
         ref = oracle_steps(n, R.initialize2d(n, seeds[m]), dt, nu, 1)
         assert rel_l2(outs[0][m], ref) < (1e-12 if prec == S.SC_FP64 else 1e-5)
+
+
+def test_member_read_into_fresh_and_odd_memory(specns_lib):
+    """A member read into memory that was never touched, that starts and ends
+    inside pages, and into pinned and device memory: the same values, and nothing
+    beside them."""
+    import ctypes as C
+    import mmap
+    torch = pytest.importorskip("torch")
+    n = 512
+    dt, nu = params(n)
+    size = n * (n // 2 + 1) * 8
+    with S.Ensemble2D([n], [dt], [nu], 0.01, S.SC_FP32) as e:
+        e.init([-3])
+        ref = e.get_member(0).tobytes()
+        for shift in (0, 8, 4096 - 24):
+            m = mmap.mmap(-1, size + 2 * 65536)
+            p = C.addressof(C.c_char.from_buffer(m))
+            assert specns_lib.sc_ens_get_member(e.h, 0, C.c_void_p(p + shift)) == 0
+            assert m[shift:shift + size] == ref
+            assert not any(m[:shift]) and not any(m[shift + size:])
+        for b in (torch.zeros(size + 16, dtype=torch.uint8).pin_memory(), torch.zeros(size + 16, dtype=torch.uint8, device="cuda")):
+            assert specns_lib.sc_ens_get_member(e.h, 0, C.c_void_p(b.data_ptr() + 8)) == 0
+            got = b.cpu().numpy()
+            assert got[8:8 + size].tobytes() == ref and not got[:8].any() and not got[8 + size:].any()
+            assert specns_lib.sc_ens_set_member(e.h, 0, C.c_void_p(b.data_ptr() + 8)) == 0
+            assert e.get_member(0).tobytes() == ref
